@@ -246,7 +246,7 @@ class Context:
 
     def plan(self) -> dict:
         """Launch shape of the construction (ants per block, table layout,
-        register bitmap words per lane, shared memory bytes)."""
+        0, shared memory bytes)."""
         out = np.zeros(4, np.int32)
         _check(self._lib.aco_b200_get_plan(self._h, _p(out)), "aco_b200_get_plan")
         return {"wpb": int(out[0]), "layout": int(out[1]), "vreg": int(out[2]),

@@ -96,11 +96,11 @@ __device__ __forceinline__ uint8_t *cur_tau(uint8_t *tau, uint8_t *tau_alt, cons
 
 // Byte offsets of the construct kernel's dynamic shared memory.
 struct SmemPlan {
-  uint32_t off_cand, off_w, off_coords, off_dem, off_lut, off_draw, off_vis;
-  uint32_t bytes_cand, bytes_w, bytes_coords, bytes_dem;
+  uint32_t off_cand, off_w, off_coords, off_lut, off_draw, off_vis;
+  uint32_t bytes_cand, bytes_w, bytes_coords;
   uint32_t total;
-  int vis_words;           // 32-bit words per ant bitmap
-  int vreg;                // bitmap words per lane held in registers (0: smem)
+  uint32_t vis_bytes;      // one ant's elements (see Unserved)
+  int elem;                // bytes per element; 0: one bit, demands in global memory
   int wpb;                 // warps (ants) per block
   int layout;
   uint32_t off_route;      // route_smem: each ant's route (route_stride ints) in shared memory
@@ -119,6 +119,10 @@ struct InstanceView {
   int stage_extra_tx;      // test hook: bytes the staging wait expects beyond the copies
   const float2 *coords;    // [n+1]
   const int *demand;       // [n+1]
+  // An ant's elements before its first step: demand_bytes(max_demand) bytes
+  // per node, the demand of a customer, the type's largest value for the
+  // depot and for the padding up to unserved_bytes().
+  const uint8_t *elems;
   const uint16_t *cand;    // [(n+1) k]
   const uint16_t *lvl;     // [(n+1) k]
   // Neighbours of ranks k+1 .. k+64 of every node in the candidates' order
@@ -129,6 +133,18 @@ struct InstanceView {
   // looked at after the tier lists, before the scan (large instances).
   const uint16_t *tier2;
 };
+
+// Bytes of an ant's per-node element (k_construct's Unserved): the smallest
+// type that holds every demand below its largest value.
+inline int demand_bytes(int max_demand) {
+  return max_demand < 0xff ? 1 : (max_demand < 0xffff ? 2 : 4);
+}
+// Bytes of one ant's elements (elem = 0: its bitmap), whole 16-byte pieces.
+inline uint32_t unserved_bytes(int n, int elem) {
+  const uint32_t rows = (uint32_t)n + 1u;
+  const uint32_t b = elem ? rows * (uint32_t)elem : (rows + 31u) / 32u * 4u;
+  return (b + 15u) & ~15u;
+}
 
 constexpr int kTierLen = 64;
 // Smallest instance whose construction uses the tier lists.

@@ -318,220 +318,190 @@ cudaError_t launch_weights(const InstanceView &iv, const PheromoneView &pv,
 // Construction
 // ===========================================================================
 
-// Draws of one ant, 128 at a time in a per-warp shared buffer: draw d is
-// word d%4 of Philox({d/4, ant, epoch, stream}, {seed, kDrawKey1}) >> 8;
-// lane L computes block 32 b + L of batch b and stores its 4 words.
-__device__ __forceinline__ void draw_refill(uint32_t *buf, uint32_t d,
-                                            uint32_t seed, uint32_t epoch,
-                                            uint32_t ant, uint32_t stream,
-                                            int lane) {
-  uint32_t r[4];
-  philox4x32_10(((d >> 7) << 5) + (uint32_t)lane, ant, epoch, stream, seed,
-                kDrawKey1, r);
-  __syncwarp();
-  uint4 v = make_uint4(r[0] >> (32 - kDrawBits), r[1] >> (32 - kDrawBits),
-                       r[2] >> (32 - kDrawBits), r[3] >> (32 - kDrawBits));
-  reinterpret_cast<uint4 *>(buf)[lane] = v;
-  __syncwarp();
-}
+// Draws of one ant come 128 at a time into a per-warp shared buffer: draw d
+// is word d%4 of Philox({d/4, ant, epoch, stream}, {seed, kDrawKey1}) >> 8;
+// lane L computes block 32 b + L of batch b and stores its 4 words (kept
+// shifted left, as next_draws writes them).
 
-template <int L, bool UNIT>
+template <int L>
 struct Tables {
-  const uint16_t *tier;  // global, or null
+  const uint16_t *tier;   // global, or null
   const uint16_t *tier2;  // global, or null
+  // This lane's column of the candidate and weight rows: entry nb of cand
+  // (w, rel) is row nb / k's.  Lanes without a candidate (k < 32) read one
+  // fixed zero entry (column step 0).
   const uint16_t *cand;
   const uint32_t *w;
   const uint8_t *rel;
+  uint32_t step;          // 1, or 0 for a lane without a candidate
   const uint32_t *lut;
   const float2 *coords;
-  const int *dem;
 
-  __device__ __forceinline__ uint32_t weight(int idx) const {
-    if (L == kLayoutSmemPacked) return lut[rel[idx]];
-    return w[idx];
+  __device__ __forceinline__ int candidate(uint32_t nb) const {
+    if (L == kLayoutGlobal) return (int)__ldg(cand + nb * step);
+    return (int)cand[nb * step];
+  }
+  __device__ __forceinline__ uint32_t weight(uint32_t nb) const {
+    if (L == kLayoutSmemPacked) return lut[rel[nb * step]];
+    if (L == kLayoutGlobal) return __ldg(w + nb * step);
+    return w[nb * step];
   }
   __device__ __forceinline__ float2 coord(int node) const {
     if (L == kLayoutGlobal) return __ldg(coords + node);
     return coords[node];
   }
-  __device__ __forceinline__ int demand(int node) const {
-    if (UNIT) return 1;
-    if (L == kLayoutGlobal) return __ldg(dem + node);
-    return dem[node];
-  }
 };
 
-// Visited set of one ant.  V = 1 or 2 (n < 2048): registers, transposed so
-// that lane L holds nodes L, L + 32, L + 64, ... (and from 1024 on in a
-// second word): the nodes of any instance spread evenly over the lanes,
-// which keeps the nearest-customer scan short on small instances.  V = 0:
-// the bitmap is in shared memory, word wi holding nodes 32 wi .. 32 wi + 31.
-// The depot and the bits past node n start set.  test/set are collective.
-__device__ __forceinline__ uint32_t vis_init_word(int wi, int n) {
-  uint32_t word = 0u;
-  const int lo = wi << 5;
-  if (lo == 0) word |= 1u;
-  const int valid = n + 1 - lo;  // nodes lo..n in this word
-  if (valid < 32) word |= (valid <= 0) ? 0xffffffffu : (0xffffffffu << valid);
-  return word;
-}
+// What an ant still has to serve: one element per node in shared memory,
+// the customer's demand while it is unvisited and the largest value of the
+// type once it is visited (the depot and the padding from the start).  One
+// load and one compare against the room left answer "unvisited and fits",
+// one store marks a visit, and the loaded element is the demand the step
+// needs.  E = 1, 2 or 4 bytes, the smallest that holds every demand below
+// that largest value; E = 0: a bitmap (word wi holding nodes 32 wi .. 32 wi
+// + 31) with the demands in global memory, for instances whose elements do
+// not fit beside the other ants of the block.
+//
+// The elements replace a bitmap in registers read by a shuffle: that took a
+// shuffle, the bit's forming and testing, a second load for the demand and a
+// test whether demands bind at all, 15 instructions more per step.
+template <int E>
+struct Unserved {
+  static constexpr uint32_t kVisited = E == 1 ? 0xffu : (E == 2 ? 0xffffu : 0xffffffffu);
+  uint32_t base;     // shared address of this ant's elements
+  uint32_t chunks;   // 16-byte pieces
+  const int *dem;    // E = 0
 
-template <int V>
-struct Visited {
-  uint32_t w0, w1;
-  uint32_t *s;
-  int vw;
-
-  __device__ __forceinline__ void init(uint32_t *smem_words, int vw_, int n,
-                                       int lane) {
-    vw = vw_;
-    s = smem_words;
-    w0 = w1 = 0xffffffffu;
-    // Registers hold the bitmap transposed: bit b of lane L's w0 is node
-    // L + 32 b, of its w1 node 1024 + L + 32 b.
-    if (V >= 1) w0 = lane_word(lane, n) | (lane == 0 ? 1u : 0u);
-    if (V == 2) w1 = lane_word(1024 + lane, n);
-    if (V == 0) {
-      for (int wi = lane; wi < vw; wi += 32) s[wi] = vis_init_word(wi, n);
-      __syncwarp();
-    }
-  }
-  // Nodes first + 32 b (b = 0..31) that are beyond n: their bits start set.
-  __device__ __forceinline__ static uint32_t lane_word(int first, int n) {
-    const int cnt = n >= first ? (n - first) / 32 + 1 : 0;  // nodes <= n
-    return cnt >= 32 ? 0u : (0xffffffffu << cnt);
-  }
-  __device__ __forceinline__ bool test(int c) const {
-    if (V == 0) {
-      const uint32_t word = s[c >> 5];
-      return (__funnelshift_r(word, word, c) & 1u) != 0u;  // bit c mod 32
-    }
-    // Lane c mod 32 holds node c (the shuffle takes the source modulo 32),
-    // at bit (c / 32) mod 32.
-    const uint32_t bit = __funnelshift_l(0u, 1u, c >> 5);  // formed while the shuffle flies
-    uint32_t word = __shfl_sync(kFull, w0, c);
-    if (V == 2) {
-      const uint32_t hi = __shfl_sync(kFull, w1, c);
-      word = (c >> 10) ? hi : word;
-    }
-    return (word & bit) != 0u;
-  }
-  __device__ __forceinline__ void set(int node, int lane) {
-    if (V == 0) {
-      const uint32_t bit = __funnelshift_l(0u, 1u, node);  // 1 << (node mod 32)
-      if (lane == 0) s[node >> 5] |= bit;
-      __syncwarp();
+  // The accesses are volatile so that they keep their order: a visit's store
+  // comes before the next step's loads.
+  __device__ __forceinline__ uint32_t get(int node) const {
+    uint32_t v;
+    if (E == 1) {
+      asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(base + (uint32_t)node));
+    } else if (E == 2) {
+      asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(base + 2u * (uint32_t)node));
+    } else if (E == 4) {
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(base + 4u * (uint32_t)node));
     } else {
-      const uint32_t bit = __funnelshift_l(0u, 1u, node >> 5);  // 1 << ((node / 32) mod 32)
-      const bool mine = lane == (node & 31);
-      if (V == 2 && (node >> 10)) w1 |= mine ? bit : 0u;
-      else w0 |= mine ? bit : 0u;
+      const uint32_t d = (uint32_t)__ldg(dem + node);
+      asm volatile("ld.shared.u32 %0, [%1];"
+                   : "=r"(v) : "r"(base + 4u * ((uint32_t)node >> 5)));
+      v = (__funnelshift_r(v, v, node) & 1u) ? kVisited : d;
     }
+    return v;
+  }
+  // Of nodes 2 q and 2 q + 1.
+  __device__ __forceinline__ void get_pair(int q, uint32_t &e0, uint32_t &e1) const {
+    if (E == 1) {
+      uint32_t v;
+      asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(base + 2u * (uint32_t)q));
+      e0 = v & 0xffu;
+      e1 = v >> 8;
+    } else if (E == 2) {
+      uint32_t v;
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(base + 4u * (uint32_t)q));
+      e0 = v & 0xffffu;
+      e1 = v >> 16;
+    } else if (E == 4) {
+      asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];"
+                   : "=r"(e0), "=r"(e1) : "r"(base + 8u * (uint32_t)q));
+    } else {
+      uint32_t v;
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(base + 4u * ((uint32_t)q >> 4)));
+      const int2 d = __ldg(reinterpret_cast<const int2 *>(dem) + q);
+      v >>= (2 * q) & 31;
+      e0 = (v & 1u) ? kVisited : (uint32_t)d.x;
+      e1 = (v & 2u) ? kVisited : (uint32_t)d.y;
+    }
+  }
+  // Every lane calls it with the same node.
+  __device__ __forceinline__ void mark(int node) {
+    if (E == 1) {
+      asm volatile("st.shared.u8 [%0], %1;" ::"r"(base + (uint32_t)node), "r"(kVisited));
+    } else if (E == 2) {
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(base + 2u * (uint32_t)node), "r"(kVisited));
+    } else if (E == 4) {
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(base + 4u * (uint32_t)node), "r"(kVisited));
+    } else {
+      const uint32_t a = base + 4u * ((uint32_t)node >> 5);
+      uint32_t v;
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v | __funnelshift_l(0u, 1u, node)));
+    }
+  }
+  // The room left as the elements are compared with it.
+  __device__ __forceinline__ uint32_t limit(int room) const {
+    return (E == 1 || E == 2) ? min((uint32_t)room, kVisited - 1u) : (uint32_t)room;
+  }
+  // E = 0: the bitmap of an unserved instance (by one warp); the elements
+  // are copied from iv.elems.
+  __device__ __forceinline__ void init_bits(int n, int lane) {
+    for (uint32_t wi = (uint32_t)lane; wi < 4u * chunks; wi += 32u) {
+      const int lo = (int)wi << 5, valid = n + 1 - lo;  // nodes lo..n in this word
+      uint32_t v = lo == 0 ? 1u : 0u;
+      if (valid < 32) v |= valid <= 0 ? 0xffffffffu : (0xffffffffu << valid);
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(base + 4u * wi), "r"(v));
+    }
+    __syncwarp();
   }
 };
 
-// The full scan over a register bitmap of two words per lane (V = 2, the
-// transposed layout of Visited<2>: bit b of word j is node 1024 j + lane +
-// 32 b), in ascending node order, 8 unvisited nodes at a time with their
-// coordinate (and demand) loads issued together; the lane's best node (its
-// squared distance's bits in *best_h_out).  Out of line, as scan_words.
-// (With one word per lane the plain loop is as fast and shorter.)
-template <int L, bool UNIT, int V>
-__device__ __noinline__ uint32_t scan_regs(const float2 *coords, const int *dem, uint32_t w0,
-                                           uint32_t w1, float2 pc, int room, bool check_dem,
-                                           int lane, uint32_t *best_h_out) {
-  uint32_t best_h = 0xffffffffu, best_n = 0xffffffffu;
-  constexpr int kB = 8;
-  int j = 0;
-  uint32_t fr = ~w0;
-  while (true) {
-    int nd[kB];
-#pragma unroll
-    for (int q = 0; q < kB; ++q) {
-      if (V == 2 && fr == 0u && j == 0) { fr = ~w1; j = 1; }
-      nd[q] = -1;
-      if (fr) {
-        nd[q] = 1024 * j + lane + 32 * (__ffs(fr) - 1);
-        fr &= fr - 1;
-      }
-    }
-    float2 pq[kB];
-    int dq[kB];
-#pragma unroll
-    for (int q = 0; q < kB; ++q) {
-      pq[q] = make_float2(0.f, 0.f);
-      dq[q] = 0;
-      if (nd[q] >= 0) {
-        pq[q] = L == kLayoutGlobal ? __ldg(coords + nd[q]) : coords[nd[q]];
-        if (!UNIT && check_dem) dq[q] = L == kLayoutGlobal ? __ldg(dem + nd[q]) : dem[nd[q]];
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < kB; ++q) {
-      if (nd[q] < 0 || (!UNIT && check_dem && dq[q] > room)) continue;
-      const uint32_t h = __float_as_uint(dist2f(pc, pq[q]));
-      if (h < best_h) {
-        best_h = h;
-        best_n = (uint32_t)nd[q];
-      }
-    }
-    if (nd[kB - 1] < 0) break;
-  }
-  *best_h_out = best_h;
-  return best_n;
+// Bits of the squared distance of (x, y) from the point whose negated
+// coordinates are npc, both differences and both squares in one packed
+// operation each: the roundings of dist2f.
+__device__ __forceinline__ uint32_t dist2_bits(float x, float y, unsigned long long npc) {
+  float sx, sy;
+  asm("{\n .reg .b64 p, d;\n"
+      " mov.b64 p, {%2, %3};\n"
+      " add.rn.f32x2 d, p, %4;\n"
+      " mul.rn.f32x2 d, d, d;\n"
+      " mov.b64 {%0, %1}, d;\n}\n"
+      : "=f"(sx), "=f"(sy) : "f"(x), "f"(y), "l"(npc));
+  return __float_as_uint(__fadd_rn(sx, sy));
 }
 
-// The full scan over a bitmap in shared memory (word wi holds nodes 32 wi ..
-// 32 wi + 31): lane L walks words L, L + 32, ... in ascending node order.
-// Its unvisited nodes are taken kScanBatch at a time and their coordinate
-// (and demand) loads issued together, so a lane waits once per batch rather
-// than once per node; they are still compared in ascending order, so the
-// lane's first nearest node wins.  Returns the lane's best node (its
-// squared distance's bits in *best_h_out).  Out of line: the batch's
-// registers do not weigh on the step loop that calls it (the scan is rare).
-template <int L, bool UNIT>
-__device__ __noinline__ uint32_t scan_words(const float2 *coords, const int *dem,
-                                            const uint32_t *s, int vw, float2 pc, int room,
-                                            bool check_dem, int lane, uint32_t *best_h_out) {
+// The full scan: lane L takes the node pairs L, L + 32, ... in ascending
+// order, visited or not, kPairs at a time with their loads issued together
+// (16 bytes of coordinates per lane) and no branch per node; pairs past the
+// last repeat it.  Walking only the unvisited nodes, from a bitmap's set
+// bits, cost more per scan while many are left, and a scan is made when few
+// are left nearby, not overall.  Returns the lane's first nearest eligible
+// node (its squared distance's bits in *best_h_out).  Out of line: the
+// batch's registers do not weigh on the step loop (the scan is rare).
+template <int L, int E, int kPairs>
+__device__ __noinline__ uint32_t scan_pairs(const float2 *coords, Unserved<E> us, int n,
+                                            float2 pc, uint32_t room, int lane,
+                                            uint32_t *best_h_out) {
   uint32_t best_h = 0xffffffffu, best_n = 0xffffffffu;
-  auto visit = [&](int node, float2 p, int dm) {
-    if (!UNIT && check_dem && dm > room) return;
-    const uint32_t h = __float_as_uint(dist2f(pc, p));
-    if (h < best_h) {
-      best_h = h;
-      best_n = (uint32_t)node;
-    }
-  };
-  constexpr int kScanBatch = 16;
-  const int nwords = lane < vw ? (vw - 1 - lane) / 32 + 1 : 0;
-  int j = 0;
-  uint32_t fr = nwords > 0 ? ~s[lane] : 0u;
-  while (true) {
-    int nd[kScanBatch];
+  const int last = n >> 1;
+  unsigned long long npc;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(npc) : "f"(-pc.x), "f"(-pc.y));
+#pragma unroll 1
+  for (int b = lane; b <= last; b += 32 * kPairs) {
+    float4 p[kPairs];
+    uint32_t h[2 * kPairs];
 #pragma unroll
-    for (int q = 0; q < kScanBatch; ++q) {
-      while (fr == 0u && ++j < nwords) fr = ~s[lane + 32 * j];
-      nd[q] = -1;
-      if (fr) {
-        nd[q] = ((lane + 32 * j) << 5) + __ffs(fr) - 1;
-        fr &= fr - 1;
-      }
+    for (int i = 0; i < kPairs; ++i) {
+      const int q = min(b + 32 * i, last);
+      const float4 *c4 = reinterpret_cast<const float4 *>(coords) + q;
+      p[i] = L == kLayoutGlobal ? __ldg(c4) : *c4;
+      us.get_pair(q, h[2 * i], h[2 * i + 1]);
     }
-    float2 pq[kScanBatch];
-    int dq[kScanBatch];
+    uint32_t m = 0xffffffffu;
 #pragma unroll
-    for (int q = 0; q < kScanBatch; ++q) {
-      pq[q] = make_float2(0.f, 0.f);
-      dq[q] = 0;
-      if (nd[q] >= 0) {
-        pq[q] = L == kLayoutGlobal ? __ldg(coords + nd[q]) : coords[nd[q]];
-        if (!UNIT && check_dem) dq[q] = L == kLayoutGlobal ? __ldg(dem + nd[q]) : dem[nd[q]];
-      }
+    for (int i = 0; i < kPairs; ++i) {
+      const uint32_t h0 = dist2_bits(p[i].x, p[i].y, npc);
+      const uint32_t h1 = dist2_bits(p[i].z, p[i].w, npc);
+      h[2 * i] = h[2 * i] <= room ? h0 : 0xffffffffu;
+      h[2 * i + 1] = h[2 * i + 1] <= room ? h1 : 0xffffffffu;
+      m = min(m, min(h[2 * i], h[2 * i + 1]));
     }
+    if (m < best_h) {
+      best_h = m;
 #pragma unroll
-    for (int q = 0; q < kScanBatch; ++q)
-      if (nd[q] >= 0) visit(nd[q], pq[q], dq[q]);
-    if (nd[kScanBatch - 1] < 0) break;
+      for (int i = 2 * kPairs - 1; i >= 0; --i)
+        if (h[i] == m) best_n = (uint32_t)(2 * min(b + 32 * (i >> 1), last) + (i & 1));
+    }
   }
   *best_h_out = best_h;
   return best_n;
@@ -540,120 +510,69 @@ __device__ __noinline__ uint32_t scan_words(const float2 *coords, const int *dem
 // Nearest unvisited customer that fits (find_nearest_unvisited,
 // src/seq/aco_sequential.c:477-493: strict '<' over ascending nodes, so the
 // lowest index wins ties).  0 if none.
-template <int L, bool UNIT, int V>
-__device__ __forceinline__ int nearest_unvisited(const Tables<L, UNIT> &tb,
-                                                 const Visited<V> &vis,
-                                                 float2 pc, int room,
-                                                 bool check_dem, int lane) {
-  uint32_t best_h = 0xffffffffu, best_n = 0xffffffffu;
-  auto visit = [&](int node, float2 p, int dem) {
-    if (!UNIT && check_dem && dem > room) return;
-    const uint32_t h = __float_as_uint(dist2f(pc, p));
-    if (h < best_h) {
-      best_h = h;
-      best_n = (uint32_t)node;
-    }
-  };
-  if (V == 2) {
-    best_n = scan_regs<L, UNIT, V>(tb.coords, tb.dem, vis.w0, vis.w1, pc, room, check_dem, lane,
-                                   &best_h);
-  } else if (V == 1) {
-    // Bit b of w0 is node lane + 32 b (ascending); one node at a time.
-    auto scan = [&](uint32_t fr, int first) {
-      while (fr) {
-        const int b = __ffs(fr) - 1;
-        fr &= fr - 1;
-        const int node = first + b * 32;
-        if (!UNIT && check_dem && tb.demand(node) > room) continue;
-        visit(node, tb.coord(node), 0);
-      }
-    };
-    scan(~vis.w0, lane);
-  } else {
-    best_n = scan_words<L, UNIT>(tb.coords, tb.dem, vis.s, vis.vw, pc, room, check_dem, lane,
-                                 &best_h);
-  }
+template <int L, int E>
+__device__ __forceinline__ int nearest_unvisited(const Tables<L> &tb, const Unserved<E> &us,
+                                                 int n, float2 pc, uint32_t room, int lane) {
+  uint32_t best_h;
+  uint32_t best_n;
+  if (L == kLayoutGlobal) best_n = scan_pairs<L, E, 16>(tb.coords, us, n, pc, room, lane, &best_h);
+  else if (n < 256) best_n = scan_pairs<L, E, 2>(tb.coords, us, n, pc, room, lane, &best_h);
+  else best_n = scan_pairs<L, E, 8>(tb.coords, us, n, pc, room, lane, &best_h);
   const uint32_t mh = __reduce_min_sync(kFull, best_h);
   const uint32_t mn = __reduce_min_sync(kFull, best_h == mh ? best_n : 0xffffffffu);
   return (mh == 0xffffffffu) ? 0 : (int)mn;
 }
 
-// The first eligible node of a second-tier row: the node (> 0); 0 when the
+// The first eligible node of a row of kLen ranks: the node (> 0); 0 when the
 // row lists every remaining customer and none is eligible; -1 when none of
-// the row is eligible and the row is full (customers beyond it remain).  The
-// visited bitmap is read as Visited<V> holds it: V = 0 in shared memory at s
-// (word wi holding nodes 32 wi .. 32 wi + 31), V = 1, 2 in the registers w0,
-// w1 of the lanes (transposed).  All of the row and its demands are loaded
-// at once.  Out of line: it is rare.
-template <int L, bool UNIT, int V>
-__device__ __noinline__ int tier2_first(const uint16_t *row, const uint32_t *s, uint32_t w0,
-                                        uint32_t w1, const int *dem, int room, bool check_dem,
-                                        int lane) {
-  constexpr int kParts = kTier2Len / 32;
-  int nodes[kParts], dq[kParts];
+// the row is eligible and the row is full (customers beyond it remain).  All
+// of the row is loaded at once.
+template <int E, int kLen>
+__device__ __forceinline__ int tier_row_first(const uint16_t *row, const Unserved<E> &us,
+                                              uint32_t room, int lane) {
+  constexpr int kParts = kLen / 32;
+  int nodes[kParts];
+  uint32_t e[kParts];
 #pragma unroll
   for (int r = 0; r < kParts; ++r) nodes[r] = (int)__ldg(row + 32 * r + lane);
 #pragma unroll
-  for (int r = 0; r < kParts; ++r)
-    dq[r] = (!UNIT && check_dem) ? (L == kLayoutGlobal ? __ldg(dem + nodes[r]) : dem[nodes[r]]) : 0;
+  for (int r = 0; r < kParts; ++r) e[r] = us.get(nodes[r]);  // node 0 (empty slot): visited
 #pragma unroll
   for (int r = 0; r < kParts; ++r) {
-    const int node = nodes[r];
-    // node 0 (empty slot) reads as visited: the depot's bit is set
-    bool ok;
-    if (V == 0) {
-      const uint32_t word = s[node >> 5];
-      ok = (__funnelshift_r(word, word, node) & 1u) == 0u;
-    } else {
-      const uint32_t bit = __funnelshift_l(0u, 1u, node >> 5);
-      uint32_t word = __shfl_sync(kFull, w0, node);
-      if (V == 2) {
-        const uint32_t hi = __shfl_sync(kFull, w1, node);
-        word = (node >> 10) ? hi : word;
-      }
-      ok = (word & bit) == 0u;
-    }
-    if (!UNIT && check_dem) ok = ok && dq[r] <= room;
-    const unsigned m = __ballot_sync(kFull, ok);
-    if (m) return __shfl_sync(kFull, node, __ffs(m) - 1);
+    const unsigned m = __ballot_sync(kFull, e[r] <= room);
+    if (m) return __shfl_sync(kFull, nodes[r], __ffs(m) - 1);
   }
   return (__shfl_sync(kFull, nodes[kParts - 1], 31) == 0) ? 0 : -1;
 }
 
+// Second tier: out of line, it is rare.
+template <int E>
+__device__ __noinline__ int tier2_first(const uint16_t *row, Unserved<E> us, uint32_t room,
+                                        int lane) {
+  return tier_row_first<E, kTier2Len>(row, us, room, lane);
+}
+
 // Nearest eligible customer of the fallback, when no candidate of row cur
 // has a weight (find_nearest_unvisited's rule, as nearest_unvisited): the
-// first eligible candidate (okm: the row's eligible candidates; they come
-// first in the order), else the first eligible node of the tier row (the
-// next 64 ranks of the same order), else the full scan; 0 when the
-// candidates and a complete tier row hold no eligible customer.
-template <int L, bool UNIT, int V>
-__device__ __forceinline__ int nearest_eligible(const Tables<L, UNIT> &tb, const Visited<V> &vis,
-                                                int cur, unsigned okm, int c, int room,
-                                                bool check_dem, int lane) {
-  if (okm) return __shfl_sync(kFull, c, __ffs(okm) - 1);
+// first eligible candidate (okm: the row's eligible candidates, the first in
+// the highest lane; they come first in the order), else the first eligible
+// node of the tier row (the next 64 ranks of the same order), else of the
+// second tier row, else the full scan; 0 when the lists hold every customer
+// and none is eligible.
+template <int L, int E>
+__device__ __forceinline__ int nearest_eligible(const Tables<L> &tb, const Unserved<E> &us,
+                                                int n, int cur, unsigned okm, int c,
+                                                uint32_t room, int lane) {
+  if (okm) return __shfl_sync(kFull, c, 31 - __clz(okm));
   if (tb.tier) {
-    const uint16_t *row = tb.tier + (size_t)cur * kTierLen;
-    int nodes[kTierLen / 32];
-#pragma unroll
-    for (int r = 0; r < kTierLen / 32; ++r)  // both halves in flight at once
-      nodes[r] = (int)__ldg(row + 32 * r + lane);
-#pragma unroll
-    for (int r = 0; r < kTierLen / 32; ++r) {
-      const int node = nodes[r];
-      bool ok = !vis.test(node);  // node 0 (empty slot) reads as visited
-      if (!UNIT && check_dem && ok) ok = tb.demand(node) <= room;
-      const unsigned m = __ballot_sync(kFull, ok);
-      if (m) return __shfl_sync(kFull, node, __ffs(m) - 1);
-    }
-    // every customer was listed
-    if (__shfl_sync(kFull, nodes[kTierLen / 32 - 1], 31) == 0) return 0;
+    int r = tier_row_first<E, kTierLen>(tb.tier + (size_t)cur * kTierLen, us, room, lane);
+    if (r >= 0) return r;
     if (tb.tier2) {
-      const int r = tier2_first<L, UNIT, V>(tb.tier2 + (size_t)cur * kTier2Len, vis.s, vis.w0,
-                                            vis.w1, tb.dem, room, check_dem, lane);
+      r = tier2_first<E>(tb.tier2 + (size_t)cur * kTier2Len, us, room, lane);
       if (r >= 0) return r;
     }
   }
-  return nearest_unvisited<L, UNIT, V>(tb, vis, tb.coord(cur), room, check_dem, lane);
+  return nearest_unvisited<L, E>(tb, us, n, tb.coord(cur), room, lane);
 }
 
 struct ConstructArgs {
@@ -670,55 +589,81 @@ struct ConstructArgs {
   uint32_t draw_per_ant;
 };
 
-// Next 128 draws of an ant: Philox, or (test hook) the recorded stream,
-// whose draws past its end read as 0.
-__device__ __forceinline__ void next_draws(const ConstructArgs &a, uint32_t *buf, uint32_t d,
-                                           uint32_t seed, uint32_t epoch, uint32_t gant,
-                                           int ant, int lane) {
+// Next 128 draws of an ant, each in the upper 24 bits of its word, or 1 for
+// a draw of 0: Philox, or (test hook) the recorded stream, whose draws past
+// its end read as 0.
+__device__ __noinline__ void next_draws(const ConstructArgs &a, uint32_t *buf, uint32_t d,
+                                        uint32_t seed, uint32_t epoch, uint32_t gant, int ant,
+                                        int lane) {
+  __syncwarp();
   if (a.draw_src) {
-    __syncwarp();
     const uint32_t *src = a.draw_src + (size_t)ant * a.draw_per_ant;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const uint32_t idx = (d & ~127u) + 4u * (uint32_t)lane + (uint32_t)q;
-      buf[4 * lane + q] = idx < a.draw_per_ant ? (src[idx] & 0xFFFFFFu) : 0u;
+      const uint32_t idx = d + 4u * (uint32_t)lane + (uint32_t)q;
+      buf[4 * lane + q] =
+          max(idx < a.draw_per_ant ? (src[idx] << (32 - kDrawBits)) : 0u, 1u);
     }
-    __syncwarp();
-    return;
+  } else {
+    uint32_t r[4];
+    philox4x32_10((d >> 2) + (uint32_t)lane, gant, epoch, a.stream, seed, kDrawKey1, r);
+    constexpr uint32_t kMask = ~0u << (32 - kDrawBits);
+    reinterpret_cast<uint4 *>(buf)[lane] =
+        make_uint4(max(r[0] & kMask, 1u), max(r[1] & kMask, 1u), max(r[2] & kMask, 1u),
+                   max(r[3] & kMask, 1u));
   }
-  draw_refill(buf, d, seed, epoch, gant, a.stream, lane);
+  __syncwarp();
 }
 
 // FP64 cost of a compact route sequence, summed in route order
 // (solution_cost, src/common/solution.c:126-137).  Lanes compute the arc
 // lengths, the sum runs in order in every lane; the (0,0) pairs between
-// consecutive routes add +0.0, which leaves the sum unchanged.
-template <int L, bool UNIT>
-__device__ __forceinline__ double route_cost(const Tables<L, UNIT> &tb,
-                                             const int *route, int entries,
+// consecutive routes add +0.0, which leaves the sum unchanged.  128 arcs at
+// a time: their end points and square roots overlap (one 32-arc batch at a
+// time the root's latency came on top of every batch's adds: 25 cycles per
+// arc, of which the dependent add is 9), and the next 128 arcs' end points are loaded
+// while the current ones are summed.  A zero length is not given to the
+// square root, whose special-case path a single lane would take the warp to.
+// kB = 1 is for routes of at most 33 entries.
+template <int L, int kB>
+__device__ __forceinline__ double route_cost(const Tables<L> &tb, const int *route, int entries,
                                              int lane) {
   double acc = 0.0;
   const int arcs = entries - 1;
-  // The next 32 arcs' end points are loaded while the current ones are summed.
-  int u = 0, v = 0;
-  if (lane < arcs) {
-    u = route[lane];
-    v = route[lane + 1];
-  }
-  for (int b = 0; b < arcs; b += 32) {
-    double dj = 0.0;
-    if (b + lane < arcs) dj = dist64(tb.coord(u), tb.coord(v));
-    const int j2 = b + 32 + lane;
-    if (j2 < arcs) {
-      u = route[j2];
-      v = route[j2 + 1];
-    }
-    if (arcs - b >= 32) {
+  int u[kB], v[kB];
+  auto load = [&](int b) {
 #pragma unroll
-      for (int t = 0; t < 32; ++t) acc = __dadd_rn(acc, __shfl_sync(kFull, dj, t));
-    } else {
-      const int cnt = arcs - b;
-      for (int t = 0; t < cnt; ++t) acc = __dadd_rn(acc, __shfl_sync(kFull, dj, t));
+    for (int q = 0; q < kB; ++q) {
+      const int j = b + 32 * q + lane;
+      u[q] = j < arcs ? route[j] : 0;
+      v[q] = j < arcs ? route[j + 1] : 0;
+    }
+  };
+  load(0);
+  for (int b = 0; b < arcs; b += 32 * kB) {
+    double dj[kB];
+#pragma unroll
+    for (int q = 0; q < kB; ++q) {
+      const float2 pu = tb.coord(u[q]), pv = tb.coord(v[q]);
+      const double dx = __dsub_rn((double)pu.x, (double)pv.x);
+      const double dy = __dsub_rn((double)pu.y, (double)pv.y);
+      dj[q] = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+    }
+#pragma unroll
+    for (int q = 0; q < kB; ++q) {
+      const double r = __dsqrt_rn(dj[q] == 0.0 ? 1.0 : dj[q]);
+      dj[q] = dj[q] == 0.0 ? 0.0 : r;
+    }
+    load(b + 32 * kB);
+#pragma unroll
+    for (int q = 0; q < kB; ++q) {
+      const int cnt = arcs - b - 32 * q;
+      if (cnt >= 32) {
+#pragma unroll
+        for (int t = 0; t < 32; ++t) acc = __dadd_rn(acc, __shfl_sync(kFull, dj[q], t));
+      } else {
+        for (int t = 0; t < cnt; ++t) acc = __dadd_rn(acc, __shfl_sync(kFull, dj[q], t));
+      }
     }
   }
   return acc;
@@ -734,6 +679,10 @@ __device__ __forceinline__ double depot_weight(int r, const uint32_t *lut) {
   return ldexp((double)__ldg(lut + (r - 16 * q)), -q);
 }
 
+__device__ __forceinline__ int clamp_int(long long v) {
+  return v < 0 ? 0 : (v > INT_MAX ? INT_MAX : (int)v);
+}
+
 // One ant, one warp.  Rules of build_ant_solution
 // (src/seq/aco_sequential.c:616-681) with the demand extension:
 //   vehicle v extends while remaining > 0, remaining demand > (K-v-1) Q and
@@ -747,14 +696,19 @@ __device__ __forceinline__ double depot_weight(int r, const uint32_t *lut) {
 // reference's 2 (1/(0+eps))^beta dwarfs every candidate), with no eligible
 // candidate it closes, and after a roulette draw a second draw u closes it
 // when u (denom + w_depot) >= denom, w_depot = depot_weight(rdep[cur]).
-template <int L, bool UNIT, int V, bool CREF>
-__device__ void build_ant(const ConstructArgs &a, const Tables<L, UNIT> &tb,
-                          Visited<V> &vis, uint32_t *dbuf, int *route_s, int ant,
-                          uint32_t epoch, uint32_t seed, int lane) {
+//
+// What bounds it: the latency of the step's dependent chain (row load, the
+// candidates' elements, sums, choice, next row's address) at one or two
+// warps per scheduler, about 200 cycles of a step's 270 at n=1000.  Candidate t sits in lane
+// 31 - t, so that "the first candidate" is the highest set bit of a ballot
+// (one find-leading-one).
+template <int L, int E, bool CREF>
+__device__ __forceinline__ void build_ant(const ConstructArgs &a, const Tables<L> &tb,
+                                          Unserved<E> &us, uint32_t *dbuf, int *route_s, int ant,
+                                          uint32_t epoch, uint32_t seed, int lane) {
   const InstanceView &iv = a.iv;
   const int k = iv.k, K = iv.K, R = iv.route_stride;
   const int cap = (int)iv.cap;
-  const int max_dem = iv.max_demand;
   // The route is built in shared memory where the plan has room for it
   // (route_s), and copied out once it is complete.
   int *route = route_s ? route_s : a.ab.routes + (size_t)ant * R;
@@ -762,198 +716,240 @@ __device__ void build_ant(const ConstructArgs &a, const Tables<L, UNIT> &tb,
   int *loads = a.ab.loads + (size_t)ant * K;
 
   // Draws are keyed by the ant's global id (ant_base > 0 when the colony is
-  // split over several devices).
+  // split over several devices).  128 at a time in dbuf, from the d0-th on:
+  // r_next is the current one, left counts it and those after it, da is the
+  // next one's shared address.
   const uint32_t gant = (uint32_t)(ant + iv.ant_base);
-  uint32_t d = 0;
-  next_draws(a, dbuf, d, seed, epoch, gant, ant, lane);
-  uint32_t r_next = dbuf[0];
+  uint32_t d0 = 0;
+  int left = 128;
+  uint32_t da = smem_addr(dbuf), r_next;
+  auto next_draw = [&]() {
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r_next) : "r"(da));
+    da += 4u;
+  };
+  auto refill = [&](uint32_t d) {
+    next_draws(a, dbuf, d, seed, epoch, gant, ant, lane);
+    d0 = d;
+    left = 128;
+    da = smem_addr(dbuf);
+    next_draw();
+  };
+  refill(0u);
+  // Lanes 24..31 hold the first 8 candidates.  A shuffle down by o from lane
+  // 31 - j with o > j finds no lane and returns the lane's own weight: 7 - j
+  // of the 7 shuffles below do, which the weight's factor 1 - (7 - j) undoes.
+  const bool first8 = lane >= 24;
+  const uint32_t own = first8 ? 1u - (uint32_t)(lane - 24) : 1u;
 
-  int remaining = iv.n;
   int rem_dem = (int)iv.total_demand;
   int pos = 0;
+  // Length and load of vehicle v in lane v mod 32, of the last 32 vehicles.
+  int len_r = 0, load_r = 0;
 
   for (int v = 0; v < K; ++v) {
     const int start = pos;
     if (lane == 0) route[pos] = 0;
     ++pos;
     int cur = 0;
-    int load = 0;
-    const long long fut64 = (long long)(K - v - 1) * iv.cap;
-    const int future = fut64 > 0x7fffffffLL ? 0x7fffffff : (int)fut64;
-    // room < max_dem  <=>  load > cap - max_dem
-    const int tight_load = cap - max_dem;
-    bool tight = !UNIT && 0 > tight_load;
-    // Row of the current node; the next row's loads are issued as soon as the
-    // next node is known, ahead of this step's bookkeeping.
-    // cb: this lane's candidate's row offset, formed as soon as the row is
-    // loaded, so the selected lane's offset reaches the next row's loads by
-    // one shuffle, with no multiply on the chain.
-    int c = 0, dc = 0, cb = 0;
-    uint32_t w = 0u;
-    if (lane < k) {
-      c = tb.cand[lane];
-      w = tb.weight(lane);
-    }
-    cb = c * k;
-    if (!UNIT) dc = tb.demand(c);
-    // Every demand is >= 1, so rem_dem > future >= 0 implies remaining > 0.
-    const int limit = CREF ? 0 : future;
-    // One step to customer nx (row offset base = nx k) of demand dnx: the
-    // next row's loads first, then the bookkeeping.
-    auto take_step = [&](int nx, int base, int dnx) {
-      c = 0;
-      w = 0u;
-      if (lane < k) {
-        c = tb.cand[base + lane];
-        w = tb.weight(base + lane);
-      }
-      cb = c * k;
-      if (!UNIT) dc = tb.demand(c);
+    int room = cap;
+    // Demand and room fall together, so "remaining demand > limit and load <
+    // Q" is one test of the room against a bound fixed for the vehicle.
+    // (Every demand is >= 1, so remaining demand > 0 implies customers left.)
+    const long long future = (long long)(K - v - 1) * iv.cap;
+    const int floor_room = clamp_int((CREF ? 0 : future) - ((long long)rem_dem - cap));
+    // CREF: the route may close once remaining demand <= future; a vehicle
+    // that may close at the depot does.
+    const long long close64 = future - ((long long)rem_dem - cap);
+    const int close_room = close64 < 0 ? -1 : clamp_int(close64);
+    bool open = !(CREF && room <= close_room);
+    // Row of the current node: candidates, weights and the candidates'
+    // elements, requested as soon as the node is known, ahead of the step's
+    // bookkeeping and loop test.
+    int c = tb.candidate(0u);
+    uint32_t w = tb.weight(0u);
+    uint32_t e = us.get(c);
+    auto take_step = [&](int nx, uint32_t base, uint32_t dnx) {
+      c = tb.candidate(base);
+      w = tb.weight(base);
+      us.mark(nx);
       route[pos] = nx;  // every lane stores the same value
-      vis.set(nx, lane);
       ++pos;
-      --remaining;
-      load += dnx;
-      rem_dem -= dnx;
-      tight = !UNIT && load > tight_load;
+      room -= (int)dnx;
       cur = nx;
     };
-    // One step per loop trip (unrolling by two was 0.9 % slower at n=1000
-    // once the prefix came from independent shuffles).
+    while (open && room > floor_room) {
+      // The step loop proper.  Its one loop test is a vote, so that the
+      // branch is known to be the warp's, and what is rare (new draws, the
+      // fallback) is outside of it: with calls inside, the loop was 37 %
+      // slower per step whether or not they were made.
 #pragma unroll 1
-    while (rem_dem > limit && load < cap) {
-      const bool may_close = CREF && rem_dem <= future;
-      if (CREF && may_close && cur == 0) break;
-      bool ok = !vis.test(c);
-      // Demands only bind when the room left is below the largest demand;
-      // until then the speculative demand load stays off the step's chain.
-      if (!UNIT && tight) ok = ok && dc + load <= cap;
-      const uint32_t wv = ok ? w : 0u;
-      const uint32_t denom = __reduce_add_sync(kFull, wv);
-      // cum * 2^24 >= r * denom  <=>  cum >= ceil(r * denom / 2^24)
-      const uint32_t thr =
-          (uint32_t)(((unsigned long long)r_next * denom + 0xFFFFFFull) >> kDrawBits);
-      // Sum of the 8 masked weights ending at this lane (lanes 0..7: the
-      // inclusive prefix, where most draws land): 7 independent shuffles of
-      // the weights and an add tree, the value three scan steps give with
-      // three dependent shuffles.  The last two scan steps run only if
-      // needed.
-      uint32_t u[8];
-      u[0] = wv;
+      while (__any_sync(kFull, room > floor_room && left > 0)) {
+        const uint32_t lim = us.limit(room);
+        // This lane's candidate's row offset, off the chain, so that the
+        // selected lane's reaches the next row's loads by one shuffle.
+        const uint32_t cb = (uint32_t)c * (uint32_t)k;
+        const uint32_t wv = e <= lim ? w : 0u;
+        const uint32_t denom = __reduce_add_sync(kFull, wv);
+        // cum 2^24 >= r denom  <=>  cum >= ceil(r denom / 2^24)  <=>
+        // cum > floor((R denom - 1) / 2^32) for the draw R = 2^8 r (1 for
+        // r = 0: the first sum that is not 0); no sum passes for denom = 0.
+        const uint32_t thr = (uint32_t)(((unsigned long long)r_next * denom - 1ull) >> 32);
+        // Sum of the 8 masked weights from this lane's on towards lane 31
+        // (lanes 24..31: the inclusive prefix, where most draws land) from 7
+        // independent shuffles and an add tree: one shuffle latency on the
+        // chain instead of the scan's three.  The windows beyond are added
+        // only if needed.
+        uint32_t u[8];
+        u[0] = wv * own;
 #pragma unroll
-      for (int o = 1; o < 8; ++o) {
-        const uint32_t t = __shfl_up_sync(kFull, wv, o);
-        u[o] = lane >= o ? t : 0u;
-      }
-      uint32_t cum = ((u[0] + u[1]) + (u[2] + u[3])) + ((u[4] + u[5]) + (u[6] + u[7]));
-      unsigned msk = __ballot_sync(kFull, lane < 8 && wv != 0u && cum >= thr);
-      if (msk == 0u) {
-#pragma unroll
-        for (int o = 8; o < 32; o <<= 1) {
-          const uint32_t t = __shfl_up_sync(kFull, cum, o);
-          if (lane >= o) cum += t;
+        for (int o = 1; o < 8; ++o) u[o] = __shfl_down_sync(kFull, wv, o);
+        uint32_t cum = ((u[1] + u[2]) + (u[3] + u[4])) + ((u[5] + u[6]) + (u[7] + u[0]));
+        unsigned msk = __ballot_sync(kFull, first8 && cum > thr);
+        if (msk == 0u) {
+          const uint32_t t8 = __shfl_down_sync(kFull, cum, 8);
+          const uint32_t t16 = __shfl_down_sync(kFull, cum, 16);
+          const uint32_t t24 = __shfl_down_sync(kFull, cum, 24);
+          cum += (lane < 24 ? t8 : 0u) + (lane < 16 ? t16 : 0u) + (lane < 8 ? t24 : 0u);
+          msk = __ballot_sync(kFull, cum > thr);
+          if (msk == 0u) break;  // no eligible candidate has a weight
         }
-        msk = __ballot_sync(kFull, wv != 0u && cum >= thr);
-        if (denom == 0u) {
-          // No eligible candidate: the reference-CUDA rule closes the route
-          // when it may; otherwise the nearest eligible customer, which
-          // consumes no draw.
-          if (CREF && may_close) break;
-          const int nx = nearest_eligible<L, UNIT, V>(tb, vis, cur, __ballot_sync(kFull, ok), c,
-                                                      cap - load, tight, lane);
-          if (nx <= 0) break;
-          take_step(nx, nx * k, tb.demand(nx));
-          continue;
+        const int src = 31 - __clz((int)msk);
+        const uint32_t nbase = __shfl_sync(kFull, cb, src);
+        const int next = __shfl_sync(kFull, c, src);
+        const uint32_t dn = __shfl_sync(kFull, e, src);
+        if (CREF && room <= close_room) {
+          // The roulette draw is spent, and a second one decides.
+          if (--left == 0) refill(d0 + 128u); else next_draw();
+          const uint32_t r2 = r_next >> (32 - kDrawBits);
+          const double wd = depot_weight(a.et.rdep[cur], a.et.lut);
+          open = __dmul_rn((double)r2, __dadd_rn((double)denom, wd)) <
+                 (double)denom * 16777216.0;
+          if (!open) {
+            --left;
+            next_draw();
+            break;
+          }
         }
+        take_step(next, nbase, dn);
+        // A draw is consumed only by a roulette selection.
+        --left;
+        next_draw();
+        e = us.get(c);
       }
-      const int src = __ffs(msk) - 1;  // msk != 0 here: denom > 0
-      const int nbase = __shfl_sync(kFull, cb, src);
-      int next = __shfl_sync(kFull, c, src);
-      int dn = UNIT ? 1 : __shfl_sync(kFull, dc, src);
-      bool drawn = false;  // draws of this step already accounted
-      if (CREF && may_close) {
-        d += 1u;  // the roulette draw is spent
-        if ((d & 127u) == 0u) next_draws(a, dbuf, d, seed, epoch, gant, ant, lane);
-        const uint32_t r2 = dbuf[d & 127u];
-        d += 1u;  // and the close draw
-        if ((d & 127u) == 0u) next_draws(a, dbuf, d, seed, epoch, gant, ant, lane);
-        r_next = dbuf[d & 127u];
-        drawn = true;
-        const double wd = depot_weight(a.et.rdep[cur], a.et.lut);
-        if (__dmul_rn((double)r2, __dadd_rn((double)denom, wd)) >= (double)denom * 16777216.0)
-          break;
+      if (!open || room <= floor_room) break;
+      if (left == 0) {
+        refill(d0 + 128u);
+        continue;
       }
-      take_step(next, nbase, dn);
-      // A draw is consumed only by a roulette selection (denom > 0).
-      if (!drawn) {
-        d += 1u;
-        if ((d & 127u) == 0u) next_draws(a, dbuf, d, seed, epoch, gant, ant, lane);
-        r_next = dbuf[d & 127u];
-      }
+      // No eligible candidate has a weight: the reference-CUDA rule closes
+      // the route when it may; otherwise the nearest eligible customer,
+      // which consumes no draw.
+      if (CREF && room <= close_room) break;
+      const uint32_t lim = us.limit(room);
+      const int nx = nearest_eligible<L, E>(tb, us, iv.n, cur, __ballot_sync(kFull, e <= lim), c,
+                                            lim, lane);
+      if (nx <= 0) break;
+      const uint32_t dnx = us.get(nx);
+      __syncwarp();  // every lane has read the element that the step marks
+      take_step(nx, (uint32_t)nx * (uint32_t)k, dnx);
+      e = us.get(c);
     }
+    rem_dem -= cap - room;
     if (lane == 0) {
       route[pos] = 0;
       lens[v] = pos + 1 - start;
-      loads[v] = load;
+      loads[v] = cap - room;
     }
     ++pos;
+    if (lane == (v & 31)) {
+      len_r = pos - start;
+      load_r = cap - room;
+    }
   }
 
+  int remaining = iv.n - (pos - 2 * K);
   if (remaining > 0) {
     // Backward repair (aco_sequential.c:659-680): from the last vehicle down,
-    // reopen the route and append the nearest eligible customers.
+    // reopen the route and append the nearest eligible customers.  The
+    // lengths, loads and additions of 32 vehicles at a time are held by the
+    // lanes; those of the last 32 never leave them.  The additions are listed
+    // in the draw buffer, which is no longer needed, if it holds them all.
     __syncwarp();
-    int *rep = a.ab.rep + (size_t)ant * iv.n;
+    int *rep = remaining <= 128 ? reinterpret_cast<int *>(dbuf) : a.ab.rep + (size_t)ant * iv.n;
     int *repc = a.ab.repc + (size_t)ant * K;
-    for (int v = lane; v < K; v += 32) repc[v] = 0;
-    __syncwarp();
+    const int top = (K - 1) & ~31;  // first vehicle of the last group
+    int cnt_r = 0;
     int nrep = 0;
     int off_end = pos;
-    for (int v = K - 1; v >= 0 && remaining > 0; --v) {
-      const int len_v = lens[v];
-      off_end -= len_v;
-      int cur = route[off_end + len_v - 2];
-      int load = loads[v];
-      int cnt = 0;
-      while (remaining > 0 && load < cap) {
-        const int next = nearest_unvisited<L, UNIT, V>(tb, vis, tb.coord(cur), cap - load,
-                                                       true, lane);
-        if (next <= 0) break;
-        if (lane == 0) rep[nrep + cnt] = next;
-        vis.set(next, lane);
-        ++cnt;
-        load += tb.demand(next);
-        --remaining;
-        cur = next;
+    for (int g = top; g >= 0; g -= 32) {
+      const bool read = g < top;
+      const int len_l = read ? lens[g + lane] : len_r, load_l = read ? loads[g + lane] : load_r;
+      int cnt_l = 0;
+      for (int v = min(K - 1, g + 31); v >= g && remaining > 0; --v) {
+        const int len_v = __shfl_sync(kFull, len_l, v & 31);
+        off_end -= len_v;
+        int cur = route[off_end + len_v - 2];
+        int load = __shfl_sync(kFull, load_l, v & 31);
+        int cnt = 0;
+        while (remaining > 0 && load < cap) {
+          const int next =
+              nearest_unvisited<L, E>(tb, us, iv.n, tb.coord(cur), us.limit(cap - load), lane);
+          if (next <= 0) break;
+          if (lane == 0) rep[nrep + cnt] = next;
+          load += (int)us.get(next);
+          __syncwarp();  // every lane has read the element that mark replaces
+          us.mark(next);
+          __syncwarp();
+          ++cnt;
+          --remaining;
+          cur = next;
+        }
+        if (lane == (v & 31)) cnt_l = cnt;
+        nrep += cnt;
       }
-      if (lane == 0) repc[v] = cnt;
-      nrep += cnt;
+      if (g < top) repc[g + lane] = cnt_l;
+      else cnt_r = cnt_l;
     }
     __syncwarp();
-    if (lane == 0 && nrep > 0) {
+    if (nrep > 0) {
       // Re-lay the compact routes with each vehicle's additions appended
-      // before its closing depot; vehicles are moved right, last first.
+      // before its closing depot: vehicles are moved right, last first, down
+      // to the first vehicle with an addition; each move takes 32 entries at
+      // a time from its end.
       int off_total = pos;
       int add_after = 0;  // additions of vehicles > v (stored first)
       int shift = nrep;   // additions of vehicles <= v
-      for (int v = K - 1; v >= 0; --v) {
-        const int len_v = lens[v];
-        off_total -= len_v;
-        const int cnt = repc[v];
-        shift -= cnt;  // now: additions of vehicles < v
-        const int old_off = off_total, new_off = off_total + shift;
-        const int main_len = len_v - 1;
-        for (int t = main_len - 1; t >= 0; --t) route[new_off + t] = route[old_off + t];
-        for (int j = 0; j < cnt; ++j) route[new_off + main_len + j] = rep[add_after + j];
-        route[new_off + main_len + cnt] = 0;
-        lens[v] = len_v + cnt;
-        add_after += cnt;
+      for (int g = top; g >= 0 && shift > 0; g -= 32) {
+        const bool read = g < top, mine = g + lane < K;
+        const int len_l = read ? lens[g + lane] : len_r, cnt_l = read ? repc[g + lane] : cnt_r;
+        if (mine && cnt_l > 0) lens[g + lane] = len_l + cnt_l;
+        for (int v = min(K - 1, g + 31); v >= g && shift > 0; --v) {
+          const int len_v = __shfl_sync(kFull, len_l, v & 31);
+          const int cnt = __shfl_sync(kFull, cnt_l, v & 31);
+          off_total -= len_v;
+          shift -= cnt;  // now: additions of vehicles < v
+          const int new_off = off_total + shift, main_len = len_v - 1;
+          if (shift > 0) {
+            for (int t0 = (main_len - 1) & ~31; t0 >= 0; t0 -= 32) {
+              const bool in = t0 + lane < main_len;
+              const int x = in ? route[off_total + t0 + lane] : 0;
+              __syncwarp();
+              if (in) route[new_off + t0 + lane] = x;
+              __syncwarp();
+            }
+          }
+          for (int j = lane; j < cnt; j += 32) route[new_off + main_len + j] = rep[add_after + j];
+          if (lane == 0) route[new_off + main_len + cnt] = 0;
+          __syncwarp();
+          add_after += cnt;
+        }
       }
     }
     pos += nrep;
   }
   __syncwarp();
-  const double cost = route_cost<L, UNIT>(tb, route, pos, lane);
+  const double cost = pos <= 33 ? route_cost<L, 1>(tb, route, pos, lane)
+                                : route_cost<L, 4>(tb, route, pos, lane);
   if (route_s) {
     int *g = a.ab.routes + (size_t)ant * R;
     for (int j = lane; j < pos; j += 32) g[j] = route_s[j];
@@ -962,43 +958,73 @@ __device__ void build_ant(const ConstructArgs &a, const Tables<L, UNIT> &tb,
     a.ab.cost[ant] = cost;
     a.ab.feasible[ant] = (remaining == 0) ? 1 : 0;
     a.ab.steps[ant] = pos - K;
-    a.ab.draws[ant] = d;
+    a.ab.draws[ant] = d0 + 128u - (uint32_t)left;
   }
 }
 
-template <int L, bool UNIT, int V, bool CREF>
-__global__ void __launch_bounds__(512, 1) k_construct(ConstructArgs a) {
-  if (a.st && *(volatile int *)&a.st->skip) return;
+// What lanes without a candidate read from the global tables.
+__device__ const uint32_t g_zero_entry = 0u;
+
+template <int L, int E, bool CREF>
+__global__ void __launch_bounds__(512, 1) k_construct(const __grid_constant__ ConstructArgs a) {
+  // Graph replays read the epoch number and the seed from the device state,
+  // so one captured graph serves every solve of a context.
+  uint32_t epoch = a.epoch, seed = a.seed;
+  if (a.st) {
+    const int skip = *(volatile int *)&a.st->skip;
+    if (a.use_state_epoch) {  // requested with the flag: one round trip
+      epoch = *(volatile uint32_t *)&a.st->epoch;
+      seed = *(volatile uint32_t *)&a.st->seed;
+    }
+    if (skip) return;
+  }
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const SmemPlan &pl = a.plan;
   const InstanceView &iv = a.iv;
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
+  const int t = 31 - lane;  // this lane's candidate
+  const bool has = t < iv.k;
 
-  Tables<L, UNIT> tb;
+  Tables<L> tb;
   tb.tier = iv.tier;
   tb.tier2 = iv.tier2;
+  tb.step = has ? 1u : 0u;
+  tb.lut = reinterpret_cast<const uint32_t *>(smem + pl.off_lut);
   if (L == kLayoutGlobal) {
-    tb.cand = iv.cand;
-    tb.w = a.et.w;
+    // (The levels and their weights' table instead of the weights put a
+    // shared load on the chain behind the row's: n=16000 6450 -> 6640 us.)
+    const uint32_t *zero = &g_zero_entry;
+    tb.cand = has ? iv.cand + t : reinterpret_cast<const uint16_t *>(zero);
+    tb.w = has ? a.et.w + t : zero;
     tb.rel = nullptr;
-    tb.lut = nullptr;
     tb.coords = iv.coords;
-    tb.dem = iv.demand;
   } else {
-    tb.cand = reinterpret_cast<const uint16_t *>(smem + pl.off_cand);
-    tb.w = reinterpret_cast<const uint32_t *>(smem + pl.off_w);
-    tb.rel = reinterpret_cast<const uint8_t *>(smem + pl.off_w);
-    tb.lut = reinterpret_cast<const uint32_t *>(smem + pl.off_lut);
+    // Bytes 8..15 of the block's shared memory hold the zero entry.
+    tb.cand = reinterpret_cast<const uint16_t *>(smem + (has ? pl.off_cand + 2u * t : 8u));
+    tb.w = reinterpret_cast<const uint32_t *>(smem + (has ? pl.off_w + 4u * t : 8u));
+    tb.rel = smem + (has ? pl.off_w + t : 12u);
     tb.coords = reinterpret_cast<const float2 *>(smem + pl.off_coords);
-    tb.dem = reinterpret_cast<const int *>(smem + pl.off_dem);
+  }
+  if (L == kLayoutSmemPacked) {
+    uint32_t *lut = reinterpret_cast<uint32_t *>(smem + pl.off_lut);
+    for (int r = threadIdx.x; r < 256; r += blockDim.x) lut[r] = __ldg(a.et.lut + r);
+  }
+  // Staging by bulk copies: the tables (rows from global memory: none) and
+  // every ant's elements (E = 0: none).
+  constexpr bool kStage = L != kLayoutGlobal || E > 0;
+  if (kStage) {
     if (threadIdx.x == 0) {
       mbar_init(bar, 1);
       fence_mbar_init();
+      reinterpret_cast<uint32_t *>(smem)[2] = 0u;
+      reinterpret_cast<uint32_t *>(smem)[3] = kRelMax;  // packed levels: weight 0
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      const uint32_t total = pl.bytes_cand + pl.bytes_w + pl.bytes_coords + (UNIT ? 0u : pl.bytes_dem);
+      const uint32_t ants = blockDim.x >> 5;
+      const uint32_t total = pl.bytes_cand + pl.bytes_w + pl.bytes_coords +
+                             (E > 0 ? ants * pl.vis_bytes : 0u);
       mbar_arrive_expect_tx(bar, total + (uint32_t)iv.stage_extra_tx);
       const uint32_t kChunk = 32768u;
       auto issue = [&](unsigned char *dst, const void *src, uint32_t bytes) {
@@ -1008,25 +1034,26 @@ __global__ void __launch_bounds__(512, 1) k_construct(ConstructArgs a) {
           bulk_g2s(dst + o, sp + o, b, bar);
         }
       };
-      issue(smem + pl.off_cand, iv.cand, pl.bytes_cand);
-      if (L == kLayoutSmemPacked) issue(smem + pl.off_w, a.et.rel, pl.bytes_w);
-      else issue(smem + pl.off_w, a.et.w, pl.bytes_w);
-      issue(smem + pl.off_coords, iv.coords, pl.bytes_coords);
-      if (!UNIT) issue(smem + pl.off_dem, iv.demand, pl.bytes_dem);
-    }
-    if (L == kLayoutSmemPacked) {
-      uint32_t *lut = reinterpret_cast<uint32_t *>(smem + pl.off_lut);
-      for (int r = threadIdx.x; r < 256; r += blockDim.x) lut[r] = __ldg(a.et.lut + r);
-      __syncthreads();
+      if (E > 0)
+        for (uint32_t i = 0; i < ants; ++i)
+          issue(smem + pl.off_vis + i * pl.vis_bytes, iv.elems, pl.vis_bytes);
+      if (L != kLayoutGlobal) {
+        issue(smem + pl.off_cand, iv.cand, pl.bytes_cand);
+        if (L == kLayoutSmemPacked) issue(smem + pl.off_w, a.et.rel, pl.bytes_w);
+        else issue(smem + pl.off_w, a.et.w, pl.bytes_w);
+        issue(smem + pl.off_coords, iv.coords, pl.bytes_coords);
+      }
     }
   }
 
   uint32_t *dbuf = reinterpret_cast<uint32_t *>(smem + pl.off_draw) + (size_t)warp * 128;
-  Visited<V> vis;
-  vis.init(reinterpret_cast<uint32_t *>(smem + pl.off_vis) + (size_t)warp * pl.vis_words,
-           pl.vis_words, iv.n, lane);
+  Unserved<E> us;
+  us.base = smem_addr(smem + pl.off_vis + (size_t)warp * pl.vis_bytes);
+  us.chunks = pl.vis_bytes / 16u;
+  us.dem = iv.demand;
+  if (E == 0) us.init_bits(iv.n, lane);
 
-  if (L != kLayoutGlobal) {
+  if (kStage) {
     // Bounded wait for the staged tables.  The decision is the block's: it
     // goes on only when every thread saw the tables arrive, so no warp
     // enters the full-mask collectives of build_ant with lanes or warps
@@ -1052,14 +1079,10 @@ __global__ void __launch_bounds__(512, 1) k_construct(ConstructArgs a) {
 
   const int ant = blockIdx.x * pl.wpb + warp;
   if (ant >= iv.m) return;
-  // Graph replays read the epoch number and the seed from the device state,
-  // so one captured graph serves every solve of a context.
-  const uint32_t epoch = a.use_state_epoch ? (uint32_t)a.st->epoch : a.epoch;
-  const uint32_t seed = a.use_state_epoch ? a.st->seed : a.seed;
   int *route_s = pl.route_smem
                      ? reinterpret_cast<int *>(smem + pl.off_route) + (size_t)warp * iv.route_stride
                      : nullptr;
-  build_ant<L, UNIT, V, CREF>(a, tb, vis, dbuf, route_s, ant, epoch, seed, lane);
+  build_ant<L, E, CREF>(a, tb, us, dbuf, route_s, ant, epoch, seed, lane);
 }
 
 static int g_max_smem = 0;
@@ -1080,35 +1103,32 @@ SmemPlan plan_construct(const InstanceView &iv, int layout, int num_sms,
                         int max_smem) {
   SmemPlan p = {};
   const size_t rows = (size_t)iv.n + 1;
-  p.vis_words = (int)((rows + 31) / 32);
-  p.vreg = p.vis_words <= 32 ? 1 : (p.vis_words <= 64 ? 2 : 0);
   int wpb = (iv.m + num_sms - 1) / num_sms;
   if (wpb < 1) wpb = 1;
   if (wpb > 16) wpb = 16;
-  p.wpb = wpb;
-  p.bytes_cand = pad16(rows * iv.k * sizeof(uint16_t));
-  p.bytes_coords = pad16(rows * sizeof(float2));
-  p.bytes_dem = iv.unit ? 0u : pad16(rows * sizeof(int));
-  const uint32_t vis_bytes = p.vreg ? 0u : (uint32_t)wpb * p.vis_words * 4u;
-  const uint32_t draw_bytes = (uint32_t)wpb * 512u;
-  auto finish = [&](int lay) {
+  const int elem = demand_bytes(iv.max_demand);
+  auto finish = [&](int lay, int el, int ants) {
     p.layout = lay;
-    uint32_t off = 16;  // mbarrier
+    p.elem = el;
+    p.wpb = ants;
+    p.vis_bytes = unserved_bytes(iv.n, el);
+    uint32_t off = 16;  // mbarrier, zero entry
     if (lay == kLayoutGlobal) {
-      p.bytes_cand = p.bytes_w = p.bytes_coords = p.bytes_dem = 0;
-      p.off_cand = p.off_w = p.off_coords = p.off_dem = p.off_lut = off;
+      p.bytes_cand = p.bytes_w = p.bytes_coords = 0;
+      p.off_cand = p.off_w = p.off_coords = p.off_lut = off;
     } else {
+      p.bytes_cand = pad16(rows * iv.k * sizeof(uint16_t));
+      p.bytes_coords = pad16(rows * sizeof(float2));
       p.bytes_w = (lay == kLayoutSmemPacked) ? pad16(rows * iv.k) : pad16(rows * iv.k * 4);
       p.off_cand = off; off += p.bytes_cand;
       p.off_w = off; off += p.bytes_w;
       p.off_coords = off; off += p.bytes_coords;
-      p.off_dem = off; off += p.bytes_dem;
       p.off_lut = off; off += (lay == kLayoutSmemPacked) ? 1024u : 0u;
     }
     p.off_draw = off;
-    off += draw_bytes;
+    off += (uint32_t)ants * 512u;
     p.off_vis = off;
-    off += vis_bytes;
+    off += (uint32_t)ants * p.vis_bytes;
     p.total = off;
     // Each ant's route in shared memory too, with the tables in shared
     // memory, where it fits and the launch is one block per SM anyway (so
@@ -1117,75 +1137,79 @@ SmemPlan plan_construct(const InstanceView &iv, int layout, int num_sms,
     // the L1 that serves those rows (n=3000 1418 -> 1638 us).
     p.route_smem = 0;
     p.off_route = off;
-    const size_t rb = pad16((size_t)wpb * (size_t)iv.route_stride * 4u);
+    const size_t rb = pad16((size_t)ants * (size_t)iv.route_stride * 4u);
     if (lay != kLayoutGlobal && off + rb <= (size_t)max_smem &&
-        (iv.m + wpb - 1) / wpb <= num_sms) {
+        (iv.m + ants - 1) / ants <= num_sms) {
       p.route_smem = 1;
       p.total = off + (uint32_t)rb;
     }
+    return (int)p.total <= max_smem;
   };
-  if (layout >= 0) {
-    finish(layout);
-    return p;
+  // Rows from global memory with more ants per block than their elements
+  // leave room for: the bitmaps (1/8 byte per node) instead.
+  auto finish_global = [&]() { return finish(kLayoutGlobal, elem, wpb) || finish(kLayoutGlobal, 0, wpb); };
+  if (layout == kLayoutGlobal) {
+    finish_global();
+  } else if (layout >= 0) {
+    // An explicit layout: fewer ants per block where all of them do not fit.
+    int ants = wpb;
+    while (!finish(layout, elem, ants) && ants > 1) --ants;
+  } else if (!finish(kLayoutSmemWeights, elem, wpb) && !finish(kLayoutSmemPacked, elem, wpb)) {
+    finish_global();
   }
-  finish(kLayoutSmemWeights);
-  if ((int)p.total <= max_smem) return p;
-  finish(kLayoutSmemPacked);
-  if ((int)p.total <= max_smem) return p;
-  finish(kLayoutGlobal);
   return p;
 }
 
-template <int L, bool UNIT, int V>
+template <int L, int E>
 static cudaError_t configure_t() {
-  cudaError_t e = cudaFuncSetAttribute(k_construct<L, UNIT, V, false>,
+  cudaError_t e = cudaFuncSetAttribute(k_construct<L, E, false>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        construct_max_smem());
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_construct<L, UNIT, V, true>,
+    e = cudaFuncSetAttribute(k_construct<L, E, true>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, construct_max_smem());
   return e;
 }
 
-template <int L, bool UNIT>
-static cudaError_t configure_lu() {
-  cudaError_t e = configure_t<L, UNIT, 0>();
-  if (e == cudaSuccess) e = configure_t<L, UNIT, 1>();
-  if (e == cudaSuccess) e = configure_t<L, UNIT, 2>();
+template <int L>
+static cudaError_t configure_l() {
+  cudaError_t e = configure_t<L, 1>();
+  if (e == cudaSuccess) e = configure_t<L, 2>();
+  if (e == cudaSuccess) e = configure_t<L, 4>();
   return e;
 }
 
 // Opts every construct instantiation into the full shared-memory carve-out;
 // called once per device before any launch or graph capture.
 cudaError_t prepare_construct_kernels() {
-  cudaError_t e = configure_lu<kLayoutSmemWeights, false>();
-  if (e == cudaSuccess) e = configure_lu<kLayoutSmemWeights, true>();
-  if (e == cudaSuccess) e = configure_lu<kLayoutSmemPacked, false>();
-  if (e == cudaSuccess) e = configure_lu<kLayoutSmemPacked, true>();
-  if (e == cudaSuccess) e = configure_lu<kLayoutGlobal, false>();
-  if (e == cudaSuccess) e = configure_lu<kLayoutGlobal, true>();
+  cudaError_t e = configure_l<kLayoutSmemWeights>();
+  if (e == cudaSuccess) e = configure_l<kLayoutSmemPacked>();
+  if (e == cudaSuccess) e = configure_l<kLayoutGlobal>();
+  if (e == cudaSuccess) e = configure_t<kLayoutGlobal, 0>();
   return e;
 }
 
-template <int L, bool UNIT, bool CREF>
-static cudaError_t launch_construct_luc(const ConstructArgs &a, cudaStream_t s) {
+template <int L, int E>
+static cudaError_t launch_construct_le(const ConstructArgs &a, cudaStream_t s) {
   const int grid = (a.iv.m + a.plan.wpb - 1) / a.plan.wpb;
   const int threads = a.plan.wpb * 32;
-  switch (a.plan.vreg) {
-    case 1: k_construct<L, UNIT, 1, CREF><<<grid, threads, a.plan.total, s>>>(a); break;
-    case 2: k_construct<L, UNIT, 2, CREF><<<grid, threads, a.plan.total, s>>>(a); break;
-    default: k_construct<L, UNIT, 0, CREF><<<grid, threads, a.plan.total, s>>>(a); break;
+  if (a.iv.depot_rule == kDepotRuleCudaRef) {
+    if (!a.et.rdep) return cudaErrorInvalidValue;
+    k_construct<L, E, true><<<grid, threads, a.plan.total, s>>>(a);
+  } else {
+    k_construct<L, E, false><<<grid, threads, a.plan.total, s>>>(a);
   }
   return cudaGetLastError();
 }
 
-template <int L, bool UNIT>
-static cudaError_t launch_construct_lu(const ConstructArgs &a, cudaStream_t s) {
-  if (a.iv.depot_rule == kDepotRuleCudaRef) {
-    if (!a.et.rdep) return cudaErrorInvalidValue;
-    return launch_construct_luc<L, UNIT, true>(a, s);
+template <int L>
+static cudaError_t launch_construct_l(const ConstructArgs &a, cudaStream_t s) {
+  switch (a.plan.elem) {
+    case 1: return launch_construct_le<L, 1>(a, s);
+    case 2: return launch_construct_le<L, 2>(a, s);
+    case 4: return launch_construct_le<L, 4>(a, s);
   }
-  return launch_construct_luc<L, UNIT, false>(a, s);
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_construct(const InstanceView &iv, const EpochTables &et,
@@ -1207,13 +1231,12 @@ cudaError_t launch_construct(const InstanceView &iv, const EpochTables &et,
   a.stream = stream_id;
   a.use_state_epoch = use_state_epoch;
   if ((int)plan.total > construct_max_smem()) return cudaErrorInvalidValue;
-  switch (plan.layout * 2 + (iv.unit ? 1 : 0)) {
-    case 0: return launch_construct_lu<kLayoutSmemWeights, false>(a, s);
-    case 1: return launch_construct_lu<kLayoutSmemWeights, true>(a, s);
-    case 2: return launch_construct_lu<kLayoutSmemPacked, false>(a, s);
-    case 3: return launch_construct_lu<kLayoutSmemPacked, true>(a, s);
-    case 4: return launch_construct_lu<kLayoutGlobal, false>(a, s);
-    case 5: return launch_construct_lu<kLayoutGlobal, true>(a, s);
+  switch (plan.layout) {
+    case kLayoutSmemWeights: return launch_construct_l<kLayoutSmemWeights>(a, s);
+    case kLayoutSmemPacked: return launch_construct_l<kLayoutSmemPacked>(a, s);
+    case kLayoutGlobal:
+      return plan.elem ? launch_construct_l<kLayoutGlobal>(a, s)
+                       : launch_construct_le<kLayoutGlobal, 0>(a, s);
   }
   return cudaErrorInvalidValue;
 }

@@ -398,9 +398,10 @@ int aco_b200_setup(aco_b200_ctx *ctx, const aco_b200_problem *p) {
   const size_t rows = (size_t)n + 1;
   const int R = n + 2 * p->K;
   const unsigned long long tau_total = (unsigned long long)rows * rows;
+  const size_t dem_words = (rows + 3) & ~size_t(3);  // the ants' elements follow, 16-byte aligned
   if (!reuse) {
     TRY_ALLOC(dalloc(&ctx->d_coords, rows));
-    TRY_ALLOC(dalloc(&ctx->d_demand, rows));
+    TRY_ALLOC(dalloc(&ctx->d_demand, dem_words + unserved_bytes(n, 4) / 4));
     TRY_ALLOC(dalloc(&ctx->d_cand, rows * k));
     TRY_ALLOC(dalloc(&ctx->d_lvl, rows * k));
     TRY_ALLOC(dalloc(&ctx->d_tier, rows * kTierLen));
@@ -437,14 +438,18 @@ int aco_b200_setup(aco_b200_ctx *ctx, const aco_b200_problem *p) {
   }
 
   std::vector<float2> xy(rows);
-  std::vector<int> dem(rows, 1);
-  dem[0] = 0;
+  const int eb = demand_bytes(max_demand);
+  std::vector<int> dem(dem_words + unserved_bytes(n, eb) / 4, -1);
+  for (size_t i = 0; i < rows; ++i) dem[i] = i ? 1 : 0;
   for (size_t i = 0; i < rows; ++i) xy[i] = make_float2(p->x[i], p->y[i]);
   if (p->demand) for (size_t i = 0; i < rows; ++i) dem[i] = p->demand[i];
+  uint8_t *elems = reinterpret_cast<uint8_t *>(dem.data() + dem_words);
+  for (int j = 1; j <= n; ++j)  // little-endian: the low bytes are the demand
+    memcpy(elems + (size_t)j * eb, &dem[j], (size_t)eb);
   cudaStream_t s = ctx->stream;
   if (reuse) TRY(cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned int), s));
   TRY(cudaMemcpyAsync(ctx->d_coords, xy.data(), rows * sizeof(float2), cudaMemcpyHostToDevice, s));
-  TRY(cudaMemcpyAsync(ctx->d_demand, dem.data(), rows * sizeof(int), cudaMemcpyHostToDevice, s));
+  TRY(cudaMemcpyAsync(ctx->d_demand, dem.data(), dem.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   TRY(cudaMemcpyAsync(ctx->d_thr, ctx->thr.data(), kThresholds * sizeof(float), cudaMemcpyHostToDevice, s));
   TRY(cudaMemcpyAsync(ctx->d_A, ctx->A, sizeof(ctx->A), cudaMemcpyHostToDevice, s));
   TRY(cudaMemcpyAsync(ctx->d_lut, ctx->lut, sizeof(ctx->lut), cudaMemcpyHostToDevice, s));
@@ -464,6 +469,7 @@ int aco_b200_setup(aco_b200_ctx *ctx, const aco_b200_problem *p) {
   iv.depot_rule = p->depot_rule;
   iv.coords = ctx->d_coords;
   iv.demand = ctx->d_demand;
+  iv.elems = reinterpret_cast<const uint8_t *>(ctx->d_demand + dem_words);
   iv.cand = ctx->d_cand;
   iv.lvl = ctx->d_lvl;
   // The fallback's tier lists pay for their two L2 round trips only where
@@ -818,7 +824,7 @@ int aco_b200_get_plan(aco_b200_ctx *ctx, int out[4]) {
   if (!ctx || !ctx->ready || !out) return ACO_ERR_INVALID_INPUT;
   out[0] = ctx->plan.wpb;
   out[1] = ctx->plan.layout;
-  out[2] = ctx->plan.vreg;
+  out[2] = 0;
   out[3] = (int)ctx->plan.total;
   return ACO_OK;
 }
