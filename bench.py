@@ -895,12 +895,12 @@ def batched_measure(torch, local, _native, insts, seed0, steps, warmup, e2e_step
 
 def batched_h2d_d2h(insts):
     """Bytes copied per end-to-end batched step: coordinates (8 B) and
-    demands (4 B) per node, an 80-byte descriptor, row offset and size
+    demands (4 B) per node, a 72-byte descriptor, row offset and size
     (12 B) and two queue orders (8 B) per instance, the level and weight
     tables (256 + 256 ints) and the 4095 eta thresholds up; every best route
     slot (n + 2K ints), the route lengths (K ints) and the costs (8 B) down."""
     nodes = sum(x.n + 1 for x in insts)
-    h2d = nodes * 12 + len(insts) * (80 + 12 + 8) + 2048 + 4095 * 4
+    h2d = nodes * 12 + len(insts) * (72 + 12 + 8) + 2048 + 4095 * 4
     d2h = sum((x.n + 2 * x.vehicles) * 4 + x.vehicles * 4 + 8 for x in insts)
     return h2d, d2h
 

@@ -311,8 +311,10 @@ typedef struct {
   double min_rel_improvement;
 } aco_b200_batch_problem;
 
-/* Launch shape: lanes per ant (16: two ants per warp, needs cand_k <= 16;
- * 32: one), ants per block, queue order (0: as given, 1: largest first). */
+/* Launch shape: candidate slots per ant (16: needs cand_k <= 16; 32), at four
+ * slots per lane; ants a block must be able to hold (a block builds all ants
+ * of an instance at a time where its threads and shared memory allow); queue
+ * order (0: as given, 1: largest first).  Results do not depend on it. */
 typedef struct {
   int lanes_per_ant;
   int ants_per_block;

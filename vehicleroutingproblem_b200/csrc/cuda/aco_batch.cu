@@ -2,10 +2,11 @@
 //
 // Each block pulls instances from a queue and runs every epoch of an
 // instance by itself: per-epoch weights into shared memory, the ants'
-// construction (one segment of 16 or 32 lanes per ant), iteration/global
-// best and stop rules, evaporation and deposit -- phases separated by
-// __syncthreads only, so the whole batch is one launch with no grid-wide
-// synchronisation and no host round trip.  Instance i is solved exactly as
+// construction (4 or 8 lanes per ant, a whole colony at a time), iteration/
+// global best and stop rules, evaporation and deposit on the candidate cells
+// of the pheromone -- phases separated by __syncthreads only, so the whole
+// batch is one launch with no grid-wide synchronisation and no host round
+// trip.  Instance i is solved exactly as
 // the single-instance path solves it with seed + i (same draws, same rules,
 // same device math), which the tests check route for route.
 #include "aco_internal.cuh"
@@ -31,9 +32,8 @@ namespace {
 
 struct BatchInst {
   int n, K, cap, total_demand, max_demand;
-  int unit;
+  int pad;
   long long node_off;   // coords / demand / rows (cand, lvl at node_off * k)
-  long long tau_off;    // bytes, 16-aligned
   long long route_off;  // m * (n + 2K) ints
   long long lens_off;   // m * K ints
   long long gbest_off;  // n + 2K ints
@@ -57,8 +57,8 @@ struct BatchArgs {
   const uint16_t *tier;      // [rows][kTierLen]: ranks k+1 .. k+64 (fallback)
   const int32_t *A;
   const uint32_t *lut;
-  uint8_t *tau;
-  int *routes, *lens, *loads, *rep, *repc;
+  uint8_t *tau;              // [rows][2 kMaxCand] levels where they do not fit a block
+  int *routes, *lens, *loads, *rep, *last;
   double *cost;
   int *feasible, *steps;
   int *gbest_nodes, *gbest_lens;
@@ -66,327 +66,582 @@ struct BatchArgs {
   int *out_epochs;
   unsigned long long *out_steps;
   unsigned int *queue;       // work counter (scratch, zeroed before launch)
-  int max_rows;              // smem sizing: largest n + 1
-  int max_K;
-};
-
-// Shared-memory layout of a block (bytes).
-struct BatchSmem {
-  uint32_t off_cand, off_lvl, off_w, off_coords, off_dem, off_A, off_lut, off_draw, off_red, off_off;
-  uint32_t total;
 };
 
 __host__ __device__ inline uint32_t pad16u(uint32_t b) { return (b + 15u) & ~15u; }
 
-__host__ __device__ inline BatchSmem batch_smem(int max_rows, int k, int ants_per_block,
-                                                int threads, int max_K) {
-  BatchSmem s;
-  uint32_t o = 0;
-  s.off_cand = o; o += pad16u((uint32_t)max_rows * k * 2);
-  s.off_lvl = o; o += pad16u((uint32_t)max_rows * k * 2);
-  s.off_w = o; o += pad16u((uint32_t)max_rows * k * 4);
-  s.off_coords = o; o += pad16u((uint32_t)max_rows * 8);
-  s.off_dem = o; o += pad16u((uint32_t)max_rows * 4);
-  s.off_A = o; o += 1024;
+// Largest shared memory a block may ask for; bounds which launch shapes and
+// instance sizes the entry points accept.
+inline uint32_t shape_bytes(int max_rows, int k, int ants_per_block, int threads, int max_K) {
+  const uint32_t r = (uint32_t)max_rows;
+  return 2u * pad16u(r * k * 2) + pad16u(r * k * 4) + pad16u(r * 8) + pad16u(r * 4) + 2048u +
+         (uint32_t)ants_per_block * 512u + pad16u((uint32_t)(threads / 32) * 16 + 64) +
+         pad16u((uint32_t)(max_K + 1) * 4) + 64u;
+}
+
+constexpr int kBatchThreads = 512;  // per block at most
+constexpr int kSlotsPerLane = 4;    // candidates per lane
+
+// The launch: an ant takes lpa lanes with 4 candidate slots each (rows are
+// padded to S = 4 ceil(k/4) slots), `round` ants of an instance are built at
+// a time.  Offsets are bytes of dynamic shared memory.
+struct BatchShape {
+  int lpa, S, elem, threads, round;
+  int tau_smem;              // levels in shared memory (else BatchArgs::tau)
+  uint32_t off_lut, off_cand, off_w, off_coords, off_tau, off_el0, off_el, off_draw, off_red;
+  uint32_t el_bytes;         // one ant's elements
+  uint32_t total;
+};
+
+BatchShape batch_shape(int max_rows, int max_n, int k, int m, int elem, int round, bool tau_smem) {
+  BatchShape s = {};
+  s.lpa = k <= 16 ? 4 : 8;
+  s.S = (k + 3) & ~3;
+  s.elem = elem;
+  s.round = round;
+  s.threads = (round * s.lpa + 31) & ~31;
+  if (s.threads < 128) s.threads = 128;
+  s.tau_smem = tau_smem ? 1 : 0;
+  s.el_bytes = unserved_bytes(max_n, elem);
+  const uint32_t r = (uint32_t)max_rows, S = (uint32_t)s.S;
+  uint32_t o = 16;  // zeros, for lanes without candidates
+  o += 1024;        // tau levels
   s.off_lut = o; o += 1024;
-  s.off_draw = o; o += (uint32_t)ants_per_block * 512;
-  s.off_red = o; o += pad16u((uint32_t)(threads / 32) * 16 + 64);
-  s.off_off = o; o += pad16u((uint32_t)(max_K + 1) * 4);
+  s.off_cand = o; o += pad16u(r * S * 2);
+  s.off_w = o; o += r * S * 4;
+  s.off_coords = o; o += pad16u(r * 8);
+  s.off_tau = o; o += tau_smem ? pad16u(r * S * 2) : 0u;
+  s.off_el0 = o; o += s.el_bytes;
+  s.off_el = o; o += (uint32_t)round * s.el_bytes;
+  s.off_draw = o; o += (uint32_t)round * 32u * (uint32_t)s.lpa;
+  // per warp: 32 words of scratch; then the reductions
+  s.off_red = o; o += (uint32_t)(s.threads / 32) * (128u + 16u);
   s.total = o;
   return s;
 }
 
-// Segment collectives: a segment is LANES consecutive lanes of a warp
-// (LANES = 16: two ants per warp; 32: one).  Masks name the segment only, so
-// the two ants of a warp may diverge.
-template <int LANES>
-struct Seg {
-  int lane;       // lane within the segment
-  unsigned mask;  // the segment's lanes
-  int base;       // first warp lane of the segment
-  __device__ __forceinline__ Seg() {
-    const int wl = threadIdx.x & 31;
-    lane = wl & (LANES - 1);
-    base = wl & ~(LANES - 1);
-    mask = (LANES == 32) ? 0xffffffffu : (0xffffu << base);
-  }
-  template <class T>
-  __device__ __forceinline__ T shfl(T v, int src) const { return __shfl_sync(mask, v, src, LANES); }
-  __device__ __forceinline__ uint32_t shfl_up(uint32_t v, int d) const {
-    return __shfl_up_sync(mask, v, d, LANES);
-  }
-  __device__ __forceinline__ unsigned ballot(bool p) const {
-    return (__ballot_sync(mask, p) >> base) & (LANES == 32 ? 0xffffffffu : 0xffffu);
-  }
-  __device__ __forceinline__ uint32_t sum(uint32_t v) const { return __reduce_add_sync(mask, v); }
-  __device__ __forceinline__ int imax(int v) const { return __reduce_max_sync(mask, v); }
-  __device__ __forceinline__ uint32_t umin(uint32_t v) const { return __reduce_min_sync(mask, v); }
-  __device__ __forceinline__ void sync() const { __syncwarp(mask); }
+// One instance's tables as its block sees them.
+template <int E>
+struct BatchTables {
+  const uint16_t *cand;      // [rows][S]
+  const uint32_t *w;         // [rows][S]
+  const float2 *coords;
+  const uint16_t *tier;      // [rows][kTierLen] or null
+  int S;
 };
 
-// Visited bitmap of one ant in the segment's registers, transposed: bit b
-// of lane L's w0 is node L + LANES b, of its w1 node 32 LANES + L + LANES b
-// (V = 2).  The nodes of any instance spread evenly over the lanes, which
-// keeps the nearest-customer scan short.
-template <int LANES, int V>
-struct SegVisited {
-  static constexpr int kShift = (LANES == 16) ? 4 : 5;  // log2(LANES)
-  uint32_t w0, w1;
-  __device__ __forceinline__ void init(const Seg<LANES> &sg, int n) {
-    w0 = lane_word(sg.lane, n) | (sg.lane == 0 ? 1u : 0u);  // the depot starts visited
-    w1 = (V == 2) ? lane_word(32 * LANES + sg.lane, n) : 0xffffffffu;
-  }
-  // Nodes first + LANES b (b = 0..31) beyond n start set.
-  __device__ __forceinline__ static uint32_t lane_word(int first, int n) {
-    const int cnt = n >= first ? (n - first) / LANES + 1 : 0;  // nodes <= n
-    return cnt >= 32 ? 0u : (0xffffffffu << cnt);
-  }
-  __device__ __forceinline__ bool test(const Seg<LANES> &sg, int c) const {
-    // The shuffle takes the source lane modulo the segment width.
-    uint32_t word = sg.shfl(w0, c);
-    if (V == 2) {
-      const uint32_t hi = sg.shfl(w1, c);
-      word = (c >= 32 * LANES) ? hi : word;
-    }
-    return __funnelshift_r(word, word, c >> kShift) & 1u;  // bit (c / LANES) mod 32
-  }
-  __device__ __forceinline__ void set(const Seg<LANES> &sg, int node) {
-    const uint32_t bit = __funnelshift_l(0u, 1u, node >> kShift);
-    if (sg.lane == (node & (LANES - 1))) {
-      if (V == 2 && node >= 32 * LANES) w1 |= bit; else w0 |= bit;
-    }
-  }
-};
-template <int LANES, int V>
-__device__ __forceinline__ int seg_nearest(const Seg<LANES> &sg, const SegVisited<LANES, V> &vis,
-                                           const float2 *coords, const int *dem, bool unit,
-                                           float2 pc, int room, bool check_dem) {
-  uint32_t best_h = 0xffffffffu, best_n = 0xffffffffu;
-  // Bit b of a word is node first + LANES b: ascending within a lane.
-  auto scan = [&](uint32_t fr, int first) {
-    while (fr) {
-      const int b = __ffs(fr) - 1;
-      fr &= fr - 1;
-      const int node = first + b * LANES;
-      if (!unit && check_dem && dem[node] > room) continue;
-      const uint32_t h = __float_as_uint(dist2f(pc, coords[node]));
-      if (h < best_h) {
-        best_h = h;
-        best_n = (uint32_t)node;
-      }
-    }
-  };
-  scan(~vis.w0, sg.lane);
-  if (V == 2) scan(~vis.w1, 32 * LANES + sg.lane);
-  const uint32_t mh = sg.umin(best_h);
-  const uint32_t mn = sg.umin(best_h == mh ? best_n : 0xffffffffu);
-  return (mh == 0xffffffffu) ? 0 : (int)mn;
+// Smallest instance whose fallback looks in the tier lists before it scans
+// every node: a scan by the whole warp takes n/64 loads and compares per lane
+// against one row's way from L2 (512-instance batch, 100 epochs: 47.5 ms with
+// the lists from n=64 or 256 on, 55.9 ms from 512 on; below 128 the scan is
+// two batches).
+constexpr int kBatchTierMinCustomers = 128;
+
+// Nearest eligible customer of one ant by the scan of every node, made by the
+// whole warp (all arguments but lane are the warp's).  0 if none.
+template <int E>
+__device__ __noinline__ int coop_scan(const float2 *coords, uint32_t el_base, int n, int cur,
+                                      uint32_t lim, int lane) {
+  Unserved<E> us;
+  us.base = el_base;
+  us.chunks = 0;
+  us.dem = nullptr;
+  uint32_t best_h;
+  const float2 pc = coords[cur];
+  const uint32_t best_n = scan_pairs<false, E, 2>(coords, us, n, pc, lim, lane, &best_h);
+  const uint32_t mh = __reduce_min_sync(kFull, best_h);
+  const uint32_t mn = __reduce_min_sync(kFull, best_h == mh ? best_n : 0xffffffffu);
+  return mh == 0xffffffffu ? 0 : (int)mn;
 }
 
-// Smallest instance whose fallback uses the tier lists (a lane of a 16-lane
-// segment walks (n+1)/16 bitmap bits in the full scan).
-constexpr int kBatchTierMinCustomers = 256;
-
-// The fallback of a row none of whose candidates has a weight, exactly as
-// seg_nearest: the first eligible candidate (okm), else the first eligible
-// node of the tier row (the next 64 ranks), else the scan of every node; 0
-// when a complete tier row lists no eligible customer.
-template <int LANES, int V>
-__device__ __forceinline__ int seg_nearest_eligible(const Seg<LANES> &sg,
-                                                    const SegVisited<LANES, V> &vis,
-                                                    const uint16_t *tier_row, unsigned okm, int c,
-                                                    const float2 *coords, const int *dem,
-                                                    bool unit, float2 pc, int room,
-                                                    bool check_dem) {
-  if (okm) return sg.shfl(c, __ffs(okm) - 1);
-  int nodes[kTierLen / LANES];
-#pragma unroll
-  for (int q = 0; q < kTierLen / LANES; ++q)  // every part of the row in flight at once
-    nodes[q] = (int)__ldg(tier_row + q * LANES + sg.lane);
-#pragma unroll
-  for (int q = 0; q < kTierLen / LANES; ++q) {
-    const int node = nodes[q];
-    bool ok = !vis.test(sg, node);  // node 0 (empty slot) reads as visited
-    if (!unit && check_dem && ok) ok = dem[node] <= room;
-    const unsigned m = sg.ballot(ok);
-    if (m) return sg.shfl(node, __ffs(m) - 1);
-  }
-  // every customer was listed
-  if (sg.shfl(nodes[kTierLen / LANES - 1], LANES - 1) == 0) return 0;
-  return seg_nearest<LANES, V>(sg, vis, coords, dem, unit, pc, room, check_dem);
+// The first eligible node of a tier row, which lane holds two ranks of; 0
+// when the row lists every remaining customer and none is eligible, -1 when
+// it is full and none is.
+template <int E>
+__device__ __forceinline__ int coop_tier(uint32_t two, uint32_t el_base, uint32_t lim) {
+  Unserved<E> us;
+  us.base = el_base;
+  us.chunks = 0;
+  us.dem = nullptr;
+  const int n0 = (int)(two & 0xffffu), n1 = (int)(two >> 16);
+  const bool ok0 = us.get(n0) <= lim, ok1 = us.get(n1) <= lim;
+  const unsigned m = __ballot_sync(kFull, ok0 || ok1);
+  const int at = m ? __ffs(m) - 1 : 31;
+  const int node = __shfl_sync(kFull, m && ok0 ? n0 : n1, at);
+  return m || node == 0 ? node : -1;
 }
 
-__device__ __forceinline__ void seg_draw_refill(uint32_t *buf, uint32_t d, uint32_t seed,
-                                                uint32_t epoch, uint32_t ant, int lane,
-                                                int lanes, unsigned mask) {
-  // 128 draws: lane L of the segment computes Philox blocks L, L + lanes, ...
-  __syncwarp(mask);
-  for (int b = lane; b < 32; b += lanes) {
-    uint32_t r[4];
-    philox4x32_10(((d >> 7) << 5) + (uint32_t)b, ant, epoch, 0u, seed, kDrawKey1, r);
-    reinterpret_cast<uint4 *>(buf)[b] =
-        make_uint4(r[0] >> (32 - kDrawBits), r[1] >> (32 - kDrawBits),
-                   r[2] >> (32 - kDrawBits), r[3] >> (32 - kDrawBits));
-  }
-  __syncwarp(mask);
-}
-
-// One ant on one segment: the rules of build_ant in aco_kernels.cu
-// (src/seq/aco_sequential.c:616-681 with the demand extension), on the
-// block's shared tables.  UNIT: every customer's demand is 1 (instance flag).
-template <int LANES, int V, bool UNIT>
-__device__ void seg_build_ant(const BatchArgs &a, const BatchInst &I, const Seg<LANES> &sg,
-                              const uint16_t *cand, const uint32_t *wt, const float2 *coords,
-                              const int *dem, uint32_t *dbuf, uint32_t seed, int ant,
-                              uint32_t epoch, long long ai) {
-  const int k = a.k, K = I.K, n = I.n, R = n + 2 * K, cap = I.cap;
-  constexpr bool unit = UNIT;
-  int *route = a.routes + I.route_off + (long long)ant * R;
-  int *lens = a.lens + I.lens_off + (long long)ant * K;
-  int *loads = a.loads + I.lens_off + (long long)ant * K;
-  SegVisited<LANES, V> vis;
-  vis.init(sg, n);
-  uint32_t d = 0;
-  seg_draw_refill(dbuf, d, seed, epoch, (uint32_t)ant, sg.lane, LANES, sg.mask);
-  uint32_t r_next = dbuf[0];
-  int remaining = n, rem_dem = I.total_demand, pos = 0;
-  const int tight_load = cap - I.max_demand;
-  for (int v = 0; v < K; ++v) {
-    const int start = pos;
-    route[pos] = 0;
-    ++pos;
-    int cur = 0, load = 0;
-    const long long fut64 = (long long)(K - v - 1) * cap;
-    const int future = fut64 > 0x7fffffffLL ? 0x7fffffff : (int)fut64;
-    while (rem_dem > future && load < cap) {
-      // room < max demand  <=>  load > cap - max demand
-      const bool tight = !unit && load > tight_load;
-      int c = 0;
-      uint32_t w = 0u;
-      if (sg.lane < k) {
-        c = cand[cur * k + sg.lane];
-        w = wt[cur * k + sg.lane];
-      }
-      bool ok = !vis.test(sg, c);
-      if (tight) ok = ok && dem[c] + load <= cap;
-      const uint32_t wv = ok ? w : 0u;
-      const uint32_t denom = sg.sum(wv);
-      uint32_t cum = wv;
-#pragma unroll
-      for (int o = 1; o < LANES; o <<= 1) {
-        const uint32_t t = sg.shfl_up(cum, o);
-        if (sg.lane >= o) cum += t;
-      }
-      int next;
-      if (denom != 0u) {
-        const uint32_t thr =
-            (uint32_t)(((unsigned long long)r_next * denom + 0xFFFFFFull) >> kDrawBits);
-        const unsigned msk = sg.ballot(wv != 0u && cum >= thr);
-        next = sg.shfl(c, __ffs(msk) - 1);  // msk != 0 when denom != 0
-        ++d;
-        if ((d & 127u) == 0u) seg_draw_refill(dbuf, d, seed, epoch, (uint32_t)ant, sg.lane, LANES, sg.mask);
-        r_next = dbuf[d & 127u];
-      } else {
-        next = (n >= kBatchTierMinCustomers)
-                   ? seg_nearest_eligible<LANES, V>(
-                         sg, vis, a.tier + (size_t)(I.node_off + cur) * kTierLen, sg.ballot(ok),
-                         c, coords, dem, unit, coords[cur], cap - load, tight)
-                   : seg_nearest<LANES, V>(sg, vis, coords, dem, unit, coords[cur], cap - load,
-                                           tight);
-        if (next <= 0) break;
-      }
-      route[pos] = next;
-      vis.set(sg, next);
-      ++pos;
-      --remaining;
-      const int dn = unit ? 1 : dem[next];
-      load += dn;
-      rem_dem -= dn;
-      cur = next;
+// Backward repair of one ant by the whole warp (aco_sequential.c:659-680, as
+// in build_ant of aco_kernels.cu): from the last vehicle down, the nearest
+// customers that fit are appended; then the compact route is laid out again
+// in place.  left customers are unserved; returns how many of them were
+// added.  With at most 32 of them each lane holds one (ascending), and no
+// search looks at another node.
+template <int E>
+__device__ __noinline__ int coop_repair(const float2 *coords, uint32_t el_base, int n, int K,
+                                        int cap, int pos, int left, int *route, int *lens,
+                                        const int *loads, const int *last, int *rep,
+                                        int *scratch, int lane) {
+  Unserved<E> us;
+  us.base = el_base;
+  us.chunks = 0;
+  us.dem = nullptr;
+  const bool few = left <= 32;
+  int mine = 0;
+  uint32_t mdem = Unserved<E>::kVisited;
+  float2 mp = make_float2(0.f, 0.f);
+  if (few) {
+    int found = 0;
+    for (int b = 0; b <= n; b += 32) {
+      const int node = min(b + lane, n);
+      const bool open = b + lane <= n && us.get(node) != Unserved<E>::kVisited;
+      const unsigned m = __ballot_sync(kFull, open);
+      if (open) scratch[found + __popc(m & ((1u << lane) - 1u))] = node;
+      found += __popc(m);
     }
-    route[pos] = 0;
-    if (sg.lane == 0) {
-      lens[v] = pos + 1 - start;
-      loads[v] = load;
+    __syncwarp();
+    if (lane < left) {
+      mine = scratch[lane];
+      mdem = us.get(mine);
+      mp = coords[mine];
     }
-    ++pos;
+    __syncwarp();
+    rep = scratch;
   }
-  if (remaining > 0) {
-    // Backward repair (aco_sequential.c:659-680), as in build_ant.
-    sg.sync();
-    int *rep = a.rep + I.rep_off + (long long)ant * n;
-    int *repc = a.repc + I.lens_off + (long long)ant * K;
-    for (int v = sg.lane; v < K; v += LANES) repc[v] = 0;
-    sg.sync();
-    int nrep = 0, off_end = pos;
-    for (int v = K - 1; v >= 0 && remaining > 0; --v) {
-      const int len_v = lens[v];
-      off_end -= len_v;
-      int cur = route[off_end + len_v - 2];
-      int load = loads[v], cnt = 0;
-      while (remaining > 0 && load < cap) {
-        const int next = seg_nearest<LANES, V>(sg, vis, coords, dem, unit, coords[cur],
-                                               cap - load, true);
-        if (next <= 0) break;
-        if (sg.lane == 0) rep[nrep + cnt] = next;
-        vis.set(sg, next);
+  int nrep = 0;
+  const int top = (K - 1) & ~31;
+  int cnt_top = 0, len_top = 0;
+  for (int g = top; g >= 0; g -= 32) {
+    const bool in = g + lane < K;
+    const int len_l = in ? lens[g + lane] : 0, load_l = in ? loads[g + lane] : 0;
+    const int last_l = in ? last[g + lane] : 0;
+    int cnt_l = 0;
+    for (int v = min(K - 1, g + 31); v >= g && left > 0; --v) {
+      int cur = __shfl_sync(kFull, last_l, v & 31), load = __shfl_sync(kFull, load_l, v & 31);
+      int cnt = 0;
+      while (left > 0 && load < cap) {
+        const uint32_t lim = us.limit(cap - load);
+        int next;
+        uint32_t dn;
+        if (few) {
+          const uint32_t h =
+              mdem <= lim ? __float_as_uint(dist2f(coords[cur], mp)) : 0xffffffffu;
+          const uint32_t mh = __reduce_min_sync(kFull, h);
+          if (mh == 0xffffffffu) break;
+          const int src = __ffs(__ballot_sync(kFull, h == mh)) - 1;
+          next = __shfl_sync(kFull, mine, src);
+          dn = __shfl_sync(kFull, mdem, src);
+          if (lane == src) mdem = Unserved<E>::kVisited;
+        } else {
+          next = coop_scan<E>(coords, el_base, n, cur, lim, lane);
+          if (next <= 0) break;
+          dn = us.get(next);
+          __syncwarp();
+          us.mark(next);
+          __syncwarp();
+        }
+        if (lane == 0) rep[nrep + cnt] = next;
         ++cnt;
-        load += unit ? 1 : dem[next];
-        --remaining;
+        load += (int)dn;
+        --left;
         cur = next;
       }
-      if (sg.lane == 0) repc[v] = cnt;
+      if (lane == (v & 31)) cnt_l = cnt;
       nrep += cnt;
     }
-    sg.sync();
-    if (sg.lane == 0 && nrep > 0) {
-      int off_total = pos, add_after = 0, shift = nrep;
-      for (int v = K - 1; v >= 0; --v) {
-        const int len_v = lens[v];
-        off_total -= len_v;
-        const int cnt = repc[v];
-        shift -= cnt;
-        const int old_off = off_total, new_off = off_total + shift, main_len = len_v - 1;
-        for (int t = main_len - 1; t >= 0; --t) route[new_off + t] = route[old_off + t];
-        for (int j = 0; j < cnt; ++j) route[new_off + main_len + j] = rep[add_after + j];
-        route[new_off + main_len + cnt] = 0;
-        lens[v] = len_v + cnt;
-        add_after += cnt;
-      }
+    // The additions of a lower group wait in `last`, which it has read.
+    if (g == top) {
+      cnt_top = cnt_l;
+      len_top = len_l;
+    } else if (in) {
+      const_cast<int *>(last)[g + lane] = cnt_l;
     }
-    pos += nrep;
   }
-  sg.sync();
-  // FP64 cost in route order (boundary (0,0) pairs add +0.0).
-  // The next LANES arcs' end points are loaded while the current ones are
-  // summed.
-  double acc = 0.0;
-  const int arcs = pos - 1;
-  int ru = 0, rv = 0;
-  if (sg.lane < arcs) {
-    ru = route[sg.lane];
-    rv = route[sg.lane + 1];
-  }
-  for (int b = 0; b < arcs; b += LANES) {
-    double dj = 0.0;
-    if (b + sg.lane < arcs) dj = dist64(coords[ru], coords[rv]);
-    const int j2 = b + LANES + sg.lane;
-    if (j2 < arcs) {
-      ru = route[j2];
-      rv = route[j2 + 1];
-    }
-    if (arcs - b >= LANES) {
+  __syncwarp();
+  int off_total = pos, add_after = 0, shift = nrep;
+  for (int g = top; g >= 0 && shift > 0; g -= 32) {
+    const bool in = g + lane < K;
+    const int len_l = g == top ? len_top : (in ? lens[g + lane] : 0);
+    const int cnt_l = g == top ? cnt_top : (in ? last[g + lane] : 0);
+    if (in && cnt_l > 0) lens[g + lane] = len_l + cnt_l;
+    for (int v = min(K - 1, g + 31); v >= g && shift > 0; --v) {
+      const int len_v = __shfl_sync(kFull, len_l, v & 31);
+      const int cnt = __shfl_sync(kFull, cnt_l, v & 31);
+      off_total -= len_v;
+      shift -= cnt;  // now: additions of vehicles < v
+      const int new_off = off_total + shift, main_len = len_v - 1;
+      if (shift > 0) {
+        // From the end, 256 entries at a time with their loads in flight.
+        for (int t0 = (main_len - 1) & ~255; t0 >= 0; t0 -= 256) {
+          int x[8];
 #pragma unroll
-      for (int t = 0; t < LANES; ++t) acc = __dadd_rn(acc, sg.shfl(dj, t));
-    } else {
-      const int cnt = arcs - b;
-      for (int t = 0; t < cnt; ++t) acc = __dadd_rn(acc, sg.shfl(dj, t));
+          for (int i = 0; i < 8; ++i) {
+            const int t = t0 + 32 * i + lane;
+            x[i] = t < main_len ? route[off_total + t] : 0;
+          }
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int t = t0 + 32 * i + lane;
+            if (t < main_len) route[new_off + t] = x[i];
+          }
+          __syncwarp();
+        }
+      }
+      for (int j = lane; j < cnt; j += 32) route[new_off + main_len + j] = rep[add_after + j];
+      if (lane == 0) route[new_off + main_len + cnt] = 0;
+      __syncwarp();
+      add_after += cnt;
     }
   }
-  if (sg.lane == 0) {
+  return nrep;
+}
+
+// The 4 LPA draws from number d on of an ant into its ring of 8 LPA words
+// (each in the upper 24 bits, or 1 for a draw of 0: see next_draws in
+// aco_kernels.cu); lane l computes one Philox block.
+template <int LPA>
+__device__ __forceinline__ void ring_fill(uint32_t ring, uint32_t d, uint32_t seed, uint32_t epoch,
+                                          uint32_t ant, int l) {
+  uint32_t r[4];
+  const uint32_t block = (d >> 2) + (uint32_t)l;
+  philox4x32_10(block, ant, epoch, 0u, seed, kDrawKey1, r);
+  constexpr uint32_t kMask = ~0u << (32 - kDrawBits);
+  const uint32_t at = ring + ((16u * block) & (32u * LPA - 1u));
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(max(r[0] & kMask, 1u)),
+               "r"(max(r[1] & kMask, 1u)), "r"(max(r[2] & kMask, 1u)), "r"(max(r[3] & kMask, 1u))
+               : "memory");
+}
+
+// The ants of one warp, 32 / LPA at a time, in lockstep: the rules of
+// build_ant in aco_kernels.cu (src/seq/aco_sequential.c:616-681 with the
+// demand extension).  Each ant is LPA lanes with 4 candidates per lane (the
+// first ones in its highest lane), so that a warp instruction serves 8 (4)
+// ants and a step's sums take 2 (3) shuffles; what only one ant needs (the
+// fallback, the repair) is done for it by the whole warp.  With one ant per
+// 16 lanes and two ants drifting apart in a warp the step took 103 warp
+// instructions per ant and the batch was bound by their issue (100 epochs of
+// the 512-instance batch 110 ms); here it is about 95 for 8 ants, and as much
+// again for their fallbacks, repairs and costs (40 ms, 2.2 instructions per
+// cycle and SM at 16 warps).
+template <int LPA, int E>
+__device__ __forceinline__ void build_ants(const BatchArgs &a, const BatchShape &sh,
+                                           const BatchInst &I, const BatchTables<E> &tb,
+                                           unsigned char *smem, uint32_t seed, uint32_t epoch,
+                                           int ant0, int ii) {
+  constexpr int kApw = 32 / LPA;
+  const int lane = threadIdx.x & 31, l = lane & (LPA - 1), seg = lane / LPA;
+  const int warp = threadIdx.x >> 5;
+  const int slot = warp * kApw + seg, ant = ant0 + slot;
+  const bool valid = slot < sh.round && ant < a.m;
+  if (!__any_sync(kFull, valid)) return;
+  const unsigned seg_mask = ((LPA == 4 ? 0xfu : 0xffu) << (lane & ~(LPA - 1)));
+  const int n = I.n, K = I.K, R = n + 2 * K, cap = I.cap, S = tb.S;
+  const int use = valid ? ant : ant0;  // lanes without an ant read the first one's addresses
+  int *route = a.routes + I.route_off + (long long)use * R;
+  int *lens = a.lens + I.lens_off + (long long)use * K;
+  int *loads = a.loads + I.lens_off + (long long)use * K;
+  int *last = a.last + I.lens_off + (long long)use * K;
+  Unserved<E> us;
+  us.base = smem_addr(smem + sh.off_el) + (uint32_t)(valid ? slot : 0) * sh.el_bytes;
+  us.chunks = 0;
+  us.dem = nullptr;
+  const uint32_t ring = smem_addr(smem + sh.off_draw) + (uint32_t)(valid ? slot : 0) * 32u * LPA;
+  // The elements from the instance's, and the first draws.
+  if (valid) {
+    const uint32_t src = smem_addr(smem + sh.off_el0);
+    for (uint32_t o = 16u * (uint32_t)l; o < sh.el_bytes; o += 16u * LPA) {
+      uint32_t x[4];
+      asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(src + o));
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(us.base + o), "r"(x[0]),
+                   "r"(x[1]), "r"(x[2]), "r"(x[3]) : "memory");
+    }
+    ring_fill<LPA>(ring, 0u, seed, epoch, (uint32_t)ant, l);
+    ring_fill<LPA>(ring, 4u * LPA, seed, epoch, (uint32_t)ant, l);
+  }
+  __syncwarp();
+
+  // This lane's slots: 4 (LPA - 1 - l) ..  A lane past the row's end reads
+  // zeros.
+  const int s0 = kSlotsPerLane * (LPA - 1 - l);
+  const bool has = s0 < S;
+  const uint32_t cbase = has ? smem_addr(tb.cand) + 2u * s0 : smem_addr(smem);
+  const uint32_t wbase = has ? smem_addr(tb.w) + 4u * s0 : smem_addr(smem);
+  const uint32_t cstep = has ? 2u * S : 0u, wstep = has ? 4u * S : 0u;
+
+  uint32_t d = 0, dbase = 0;  // draws spent; number of the ring's oldest
+  int rem_dem = I.total_demand, pos = 0, v = 0, start = 0, cur = 0, room = 0, floor_room = 0;
+  bool active = valid;
+  // The route's last entries wait in the lanes (entry p in lane p mod LPA) and
+  // leave LPA at a time: one entry per step per ant touched a line of its own
+  // with every store (100 epochs of the 512-instance batch 47.8 -> 41.7 ms).
+  int held = 0;
+  auto put = [&](int node) {
+    if (l == (pos & (LPA - 1))) held = node;
+    ++pos;
+    if ((pos & (LPA - 1)) == 0) route[pos - LPA + l] = held;
+  };
+  auto open_vehicle = [&]() {
+    start = pos;
+    put(0);
+    cur = 0;
+    room = cap;
+    // "remaining demand > (K - v - 1) Q and load < Q" as one bound on the
+    // room (see build_ant).
+    const long long f = (long long)(K - v - 1) * cap - ((long long)rem_dem - cap);
+    floor_room = f < 0 ? 0 : (f > INT_MAX ? INT_MAX : (int)f);
+  };
+  if (active) open_vehicle();
+
+  uint32_t tick = 0;
+  while (true) {
+    bool closing = active && room <= floor_room;
+    if (__any_sync(kFull, closing)) {
+      while (closing) {
+        if (l == 0) {
+          lens[v] = pos + 1 - start;
+          loads[v] = cap - room;
+          last[v] = cur;
+        }
+        put(0);
+        rem_dem -= cap - room;
+        ++v;
+        active = v < K;
+        if (!active) break;
+        open_vehicle();
+        closing = room <= floor_room;
+      }
+      __syncwarp();
+      if (!__any_sync(kFull, active)) break;
+    }
+    uint32_t c01, c23, w[4];
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];"
+                 : "=r"(c01), "=r"(c23) : "r"(cbase + (uint32_t)cur * cstep));
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                 : "r"(wbase + (uint32_t)cur * wstep));
+    uint32_t r;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(ring + ((4u * d) & (32u * LPA - 1u))));
+    uint32_t c[4] = {c01 & 0xffffu, c01 >> 16, c23 & 0xffffu, c23 >> 16};
+    uint32_t e[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) e[i] = us.get((int)c[i]);
+    const uint32_t lim = us.limit(room);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = e[i] <= lim ? w[i] : 0u;
+    const uint32_t p1 = w[0] + w[1], p2 = p1 + w[2], p3 = p2 + w[3];
+    // Sum over the ant's lanes and over the lanes above this one (those hold
+    // the candidates before this lane's).
+    const uint32_t x1 = __shfl_xor_sync(kFull, p3, 1);
+    const uint32_t t1 = p3 + x1;
+    const uint32_t x2 = __shfl_xor_sync(kFull, t1, 2);
+    uint32_t denom = t1 + x2;
+    uint32_t before = ((l & 1) ? 0u : x1) + ((l & 2) ? 0u : x2);
+    if (LPA == 8) {
+      const uint32_t x4 = __shfl_xor_sync(kFull, denom, 4);
+      denom += x4;
+      before += (l & 4) ? 0u : x4;
+    }
+    // As in build_ant: the first candidate whose inclusive sum exceeds thr;
+    // none for denom = 0.
+    const uint32_t thr = (uint32_t)(((unsigned long long)r * denom - 1ull) >> 32);
+    const unsigned msk = __ballot_sync(kFull, active && before + p3 > thr) & seg_mask;
+    const uint32_t need = thr - before;  // in the lane chosen: before <= thr
+    const bool b0 = w[0] > need, b1 = p1 > need, b2 = p2 > need;
+    uint32_t cs = b0 ? c[0] : (b1 ? c[1] : (b2 ? c[2] : c[3]));
+    uint32_t es = b0 ? e[0] : (b1 ? e[1] : (b2 ? e[2] : e[3]));
+    const int src = 31 - __clz((int)msk);
+    int next;
+    uint32_t dn;
+    if (E == 4) {
+      next = (int)__shfl_sync(kFull, cs, src);
+      dn = __shfl_sync(kFull, es, src);
+    } else {
+      const uint32_t ce = __shfl_sync(kFull, cs | (es << 16), src);
+      next = (int)(ce & 0xffffu);
+      dn = ce >> 16;
+    }
+    bool take = msk != 0u;
+    d += take ? 1u : 0u;  // only a roulette selection spends a draw
+    unsigned none = __ballot_sync(kFull, active && !take && l == 0);
+    if (none) {
+      // The nearest eligible customer (the rule of nearest_eligible in
+      // aco_kernels.cu), one ant after another by the whole warp.  An
+      // eligible candidate whose weight is 0 would come before the tier row:
+      // an ant that has one is left to the scan.
+      const unsigned zero = __ballot_sync(
+          kFull, e[0] <= lim || e[1] <= lim || e[2] <= lim || e[3] <= lim);
+      do {
+        const int b = __ffs(none) - 1;
+        none &= none - 1u;
+        const int fc = __shfl_sync(kFull, cur, b);
+        const uint32_t fl = __shfl_sync(kFull, lim, b), fb = __shfl_sync(kFull, us.base, b);
+        int nx = -1;
+        if (tb.tier && ((zero >> b) & (LPA == 4 ? 0xfu : 0xffu)) == 0u) {
+          const uint32_t two =
+              __ldg(reinterpret_cast<const uint32_t *>(tb.tier + (size_t)fc * kTierLen) + lane);
+          nx = coop_tier<E>(two, fb, fl);
+        }
+        if (nx < 0) nx = coop_scan<E>(tb.coords, fb, n, fc, fl, lane);
+        if ((lane & ~(LPA - 1)) == b) {
+          next = nx;
+          take = nx > 0;
+          if (take) dn = us.get(nx);
+          else floor_room = INT_MAX;  // no customer fits: the route ends
+        }
+      } while (none);
+      __syncwarp();  // the elements are read before they are marked
+    }
+    // The step, without a branch: an ant that takes none marks the depot,
+    // which is marked from the start.
+    us.mark(take ? next : 0);
+    held = take && l == (pos & (LPA - 1)) ? next : held;
+    pos += take ? 1 : 0;
+    if (take && (pos & (LPA - 1)) == 0) route[pos - LPA + l] = held;
+    room -= take ? (int)dn : 0;
+    cur = take ? next : cur;
+    // Every 4 LPA steps each ant that has spent its ring's older half
+    // replaces it: no ant can spend more than the other half until then.
+    if (((++tick) & (4u * LPA - 1u)) == 0u) {
+      __syncwarp();
+      if (active && d - dbase >= 4u * LPA) {
+        ring_fill<LPA>(ring, dbase + 8u * LPA, seed, epoch, (uint32_t)ant, l);
+        dbase += 4u * LPA;
+      }
+      __syncwarp();
+    }
+  }
+
+  if (valid && l < (pos & (LPA - 1))) route[(pos & ~(LPA - 1)) + l] = held;
+  int left = valid ? n - (pos - 2 * K) : 0;
+  unsigned rm = __ballot_sync(kFull, left > 0 && l == 0);
+  if (rm) {
+    __syncwarp();
+    int *scratch = reinterpret_cast<int *>(smem + sh.off_red) + 32 * warp;
+    do {
+      const int b = __ffs(rm) - 1;
+      rm &= rm - 1u;
+      const int who = ant0 + warp * kApw + b / LPA;
+      const long long lo = I.lens_off + (long long)who * K;
+      const int added = coop_repair<E>(
+          tb.coords, __shfl_sync(kFull, us.base, b), n, K, cap, __shfl_sync(kFull, pos, b),
+          __shfl_sync(kFull, left, b), a.routes + I.route_off + (long long)who * R, a.lens + lo,
+          a.loads + lo, a.last + lo, a.rep + I.rep_off + (long long)who * n, scratch, lane);
+      if ((lane & ~(LPA - 1)) == b) {
+        pos += added;
+        left -= added;
+      }
+      __syncwarp();
+    } while (rm);
+  }
+
+  // FP64 cost in route order (boundary (0,0) pairs add +0.0), 4 LPA arcs at a
+  // time: a lane forms 4 consecutive arcs and the ant's lanes add all of them
+  // in order; the next ones' end points are loaded meanwhile.  An ant with
+  // customers left has no cost anyone reads.
+  const int arcs = valid && left == 0 ? pos - 1 : 0;
+  double acc = 0.0;
+  int nd[kSlotsPerLane + 1];
+  auto load_nodes = [&](int b) {
+#pragma unroll
+    for (int i = 0; i <= kSlotsPerLane; ++i) {
+      const int j = b + kSlotsPerLane * l + i;
+      nd[i] = j <= arcs ? route[j] : 0;
+    }
+  };
+  load_nodes(0);
+  for (int b = 0; __any_sync(kFull, b < arcs); b += kSlotsPerLane * LPA) {
+    double dj[kSlotsPerLane];
+    float2 p = tb.coords[nd[0]];
+#pragma unroll
+    for (int i = 0; i < kSlotsPerLane; ++i) {
+      const float2 q = tb.coords[nd[i + 1]];
+      const double dx = __dsub_rn((double)p.x, (double)q.x);
+      const double dy = __dsub_rn((double)p.y, (double)q.y);
+      dj[i] = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+      p = q;
+    }
+    load_nodes(b + kSlotsPerLane * LPA);
+#pragma unroll
+    for (int i = 0; i < kSlotsPerLane; ++i) {
+      const double s = __dsqrt_rn(dj[i] == 0.0 ? 1.0 : dj[i]);
+      // Arcs past the end join node 0 to the depot or to itself: no length.
+      dj[i] = dj[i] == 0.0 || b + kSlotsPerLane * l + i >= arcs ? 0.0 : s;
+    }
+#pragma unroll
+    for (int t = 0; t < LPA; ++t)
+#pragma unroll
+      for (int i = 0; i < kSlotsPerLane; ++i)
+        acc = __dadd_rn(acc, __shfl_sync(kFull, dj[i], t, LPA));
+  }
+  if (valid && l == 0) {
+    const long long ai = (long long)ii * a.m + ant;
     a.cost[ai] = acc;
-    a.feasible[ai] = remaining == 0 ? 1 : 0;
+    a.feasible[ai] = left == 0 ? 1 : 0;
     a.steps[ai] = pos - K;
+  }
+}
+
+// Slot of `node` (> 0) in a candidate row of S slots, or -1.
+__device__ __forceinline__ int slot_of(const uint16_t *row, int S, int node) {
+  int t = -1;
+  for (int q = 0; q < S; q += 4) {
+    const uint2 v = *reinterpret_cast<const uint2 *>(row + q);
+    if ((int)(v.x & 0xffffu) == node) t = q;
+    if ((int)(v.x >> 16) == node) t = q + 1;
+    if ((int)(v.y & 0xffffu) == node) t = q + 2;
+    if ((int)(v.y >> 16) == node) t = q + 3;
+  }
+  return t;
+}
+
+// Pheromone of an instance inside its block.  Only the levels of candidate
+// cells are ever read (by the weights), and a deposit on arc (u, c) reads
+// tau[u][c] and raises it and tau[c][u]; so the cells kept are those of the
+// candidate pairs in both directions: fwd[i][t] = tau[i][cand[i][t]] and
+// rev[i][t] = tau[cand[i][t]][i].  A cell that is in both (two mutual
+// candidates) is written to both.  The full matrix would be (n+1)^2 bytes in
+// L2, evaporated as a whole every epoch.
+struct BatchTau {
+  uint8_t *fwd, *rev;
+  const uint16_t *cand;
+  int S;
+  float log_min, log_step;
+  uint8_t q_min, q_max;
+};
+
+__device__ __forceinline__ void batch_deposit_arc(const BatchTau &t, int u, int c, float dep) {
+  const int i = c > 0 ? slot_of(t.cand + u * t.S, t.S, c) : -1;  // c among u's candidates
+  const int j = u > 0 ? slot_of(t.cand + c * t.S, t.S, u) : -1;  // u among c's
+  if (i < 0 && j < 0) return;  // neither cell is ever read
+  const int at_u = u * t.S + i, at_c = c * t.S + j;
+  const uint8_t old = i >= 0 ? t.fwd[at_u] : t.rev[at_c];
+  const uint8_t nq = quant(dequant(old, t.log_min, t.log_step) + dep, t.log_min, t.log_step,
+                           t.q_min, t.q_max);
+  if (nq > old) {
+    if (i >= 0) t.fwd[at_u] = nq;
+    if (j >= 0) t.rev[at_c] = nq;
+  }
+  const uint8_t oldr = j >= 0 ? t.fwd[at_c] : t.rev[at_u];
+  if (nq > oldr) {
+    if (j >= 0) t.fwd[at_c] = nq;
+    if (i >= 0) t.rev[at_u] = nq;
+  }
+}
+
+// Deposit of a complete solution (total = n + 2K compact entries) by the
+// block: one arc per thread (the cells of different arcs differ), but the two
+// arcs of a one-customer route, which share their cells, by one thread in
+// order.  (0,0) pairs (empty routes, route boundaries) are no candidate cell.
+__device__ __forceinline__ void batch_deposit(const BatchTau &t, const int *nodes, int total,
+                                              float dep) {
+  for (int j = 1 + (int)threadIdx.x; j < total; j += blockDim.x) {
+    const int p = nodes[j - 1], q = nodes[j];
+    if (p == 0 && q == 0) continue;
+    if (q == 0 && nodes[j - 2] == 0) continue;  // second arc of [0 p 0]
+    batch_deposit_arc(t, p, q, dep);
+    if (p == 0 && nodes[j + 1] == 0) batch_deposit_arc(t, q, 0, dep);
   }
 }
 
@@ -398,20 +653,59 @@ __device__ __forceinline__ bool b_significant(double prev, double next, double m
   return __dadd_rn(rel, 1e-9) >= min_rel;
 }
 
-template <int LANES, int V>
-__global__ void __launch_bounds__(1024) k_batch_solve(BatchArgs a, BatchSmem ly,
-                                                      int ants_per_block) {
+// Per-epoch weights of one instance (k_weights in aco_kernels.cu), LPA lanes
+// per row.
+template <int LPA>
+__device__ __forceinline__ void batch_weights(const BatchArgs &a, const BatchInst &I,
+                                              const uint16_t *cand, const uint8_t *fwd,
+                                              const int32_t *A, const uint32_t *lut, uint32_t *w,
+                                              int rows, int S) {
+  const int l = threadIdx.x & (LPA - 1), seg = threadIdx.x / LPA, nseg = blockDim.x / LPA;
+  const int s0 = kSlotsPerLane * l, k = a.k;
+  const uint16_t *lvl = a.lvl + I.node_off * k;
+#pragma unroll 2
+  for (int r0 = 0; r0 < rows; r0 += nseg) {
+    const int r = r0 + seg;
+    const bool in = r < rows && s0 < S;
+    uint2 cc = make_uint2(0u, 0u);
+    uint32_t f = 0u;
+    int lv[4] = {0, 0, 0, 0};
+    if (in) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (s0 + i < k) lv[i] = (int)__ldg(lvl + (long long)r * k + s0 + i);
+      cc = *reinterpret_cast<const uint2 *>(cand + r * S + s0);
+      f = *reinterpret_cast<const uint32_t *>(fwd + r * S + s0);
+    }
+    const uint32_t c[4] = {cc.x & 0xffffu, cc.x >> 16, cc.y & 0xffffu, cc.y >> 16};
+    int e[4], emax = INT_MIN;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      e[i] = c[i] ? A[(f >> (8 * i)) & 0xffu] - lv[i] : INT_MIN;
+      emax = max(emax, e[i]);
+    }
+#pragma unroll
+    for (int o = 1; o < LPA; o <<= 1) emax = max(emax, __shfl_xor_sync(kFull, emax, o));
+    if (in) {
+      uint32_t x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = c[i] ? lut[min(emax - e[i], kRelMax)] : 0u;
+      *reinterpret_cast<uint4 *>(w + r * S + s0) = make_uint4(x[0], x[1], x[2], x[3]);
+    }
+  }
+}
+
+template <int LPA, int E>
+__global__ void __launch_bounds__(kBatchThreads)
+    k_batch_solve(const __grid_constant__ BatchArgs a, const __grid_constant__ BatchShape sh) {
   extern __shared__ __align__(16) unsigned char smem[];
-  uint16_t *s_cand = reinterpret_cast<uint16_t *>(smem + ly.off_cand);
-  uint16_t *s_lvl = reinterpret_cast<uint16_t *>(smem + ly.off_lvl);
-  uint32_t *s_w = reinterpret_cast<uint32_t *>(smem + ly.off_w);
-  float2 *s_coords = reinterpret_cast<float2 *>(smem + ly.off_coords);
-  int *s_dem = reinterpret_cast<int *>(smem + ly.off_dem);
-  int32_t *s_A = reinterpret_cast<int32_t *>(smem + ly.off_A);
-  uint32_t *s_lut = reinterpret_cast<uint32_t *>(smem + ly.off_lut);
-  double *s_redc = reinterpret_cast<double *>(smem + ly.off_red);
-  int *s_reda = reinterpret_cast<int *>(smem + ly.off_red + (blockDim.x / 32) * 8);
-  int *s_off = reinterpret_cast<int *>(smem + ly.off_off);
+  int32_t *s_A = reinterpret_cast<int32_t *>(smem + 16);
+  uint32_t *s_lut = reinterpret_cast<uint32_t *>(smem + sh.off_lut);
+  uint16_t *s_cand = reinterpret_cast<uint16_t *>(smem + sh.off_cand);
+  uint32_t *s_w = reinterpret_cast<uint32_t *>(smem + sh.off_w);
+  float2 *s_coords = reinterpret_cast<float2 *>(smem + sh.off_coords);
+  double *s_redc = reinterpret_cast<double *>(smem + sh.off_red + (blockDim.x / 32) * 128);
+  int *s_reda = reinterpret_cast<int *>(s_redc + blockDim.x / 32);
   __shared__ int s_inst, s_best, s_found, s_improved, s_stop;
   __shared__ double s_gbest;
   __shared__ int s_since;
@@ -420,8 +714,8 @@ __global__ void __launch_bounds__(1024) k_batch_solve(BatchArgs a, BatchSmem ly,
 
   const int tid = threadIdx.x, nthr = blockDim.x;
   const int warp = tid >> 5, nwarps = nthr >> 5;
-  const Seg<LANES> sg;
-  const int seg = tid / LANES;  // ant slot of this segment
+  const int S = sh.S;
+  if (tid < 4) reinterpret_cast<uint32_t *>(smem)[tid] = 0u;
   for (int i = tid; i < 256; i += nthr) {
     s_A[i] = a.A[i];
     s_lut[i] = a.lut[i];
@@ -437,25 +731,38 @@ __global__ void __launch_bounds__(1024) k_batch_solve(BatchArgs a, BatchSmem ly,
     if (ii < 0) return;
     const BatchInst I = a.inst[ii];
     const int n = I.n, k = a.k, rows = n + 1, K = I.K;
-    const size_t stride = (size_t)n + 1;
     const uint32_t seed = a.seed + (uint32_t)ii;
-    uint8_t *tau = a.tau + I.tau_off;
-    // Stage the instance.
-    for (int e = tid; e < rows * k; e += nthr) {
-      s_cand[e] = a.cand[I.node_off * k + e];
-      s_lvl[e] = a.lvl[I.node_off * k + e];
+    BatchTables<E> tb;
+    tb.cand = s_cand;
+    tb.w = s_w;
+    tb.coords = s_coords;
+    tb.tier = n >= kBatchTierMinCustomers ? a.tier + I.node_off * kTierLen : nullptr;
+    tb.S = S;
+    BatchTau bt;
+    bt.fwd = sh.tau_smem ? smem + sh.off_tau : a.tau + I.node_off * 2 * kMaxCand;
+    bt.rev = bt.fwd + rows * S;
+    bt.cand = s_cand;
+    bt.S = S;
+    bt.log_min = a.log_min;
+    bt.log_step = a.log_step;
+    bt.q_min = 0;
+    bt.q_max = 255;
+    // Stage the instance: rows at stride S (empty slots 0), coordinates, the
+    // elements of an unserved instance, the initial pheromone.
+    for (int e = tid; e < rows * S; e += nthr) {
+      const int r = e / S, t = e - r * S;
+      s_cand[e] = t < k ? a.cand[(I.node_off + r) * k + t] : (uint16_t)0;
     }
-    for (int e = tid; e < rows; e += nthr) {
-      s_coords[e] = a.coords[I.node_off + e];
-      s_dem[e] = a.demand[I.node_off + e];
+    for (int e = tid; e < rows; e += nthr) s_coords[e] = a.coords[I.node_off + e];
+    for (uint32_t e = tid; e < sh.el_bytes / E; e += nthr) {
+      const uint32_t x = e >= 1 && e <= (uint32_t)n ? (uint32_t)a.demand[I.node_off + e]
+                                                    : Unserved<E>::kVisited;
+      if (E == 1) smem[sh.off_el0 + e] = (unsigned char)x;
+      else if (E == 2) reinterpret_cast<uint16_t *>(smem + sh.off_el0)[e] = (uint16_t)x;
+      else reinterpret_cast<uint32_t *>(smem + sh.off_el0)[e] = x;
     }
-    {
-      const unsigned long long total = (unsigned long long)rows * rows;
-      const uint32_t w4 = 0x01010101u * a.q_tau0;
-      uint4 *t4 = reinterpret_cast<uint4 *>(tau);
-      for (unsigned long long e = tid; e < total / 16; e += nthr) __stcg(t4 + e, make_uint4(w4, w4, w4, w4));
-      for (unsigned long long e = total / 16 * 16 + tid; e < total; e += nthr) st_cg_u8(tau + e, a.q_tau0);
-    }
+    for (int e = tid; e < rows * S / 2; e += nthr)
+      reinterpret_cast<uint32_t *>(bt.fwd)[e] = 0x01010101u * a.q_tau0;
     if (tid == 0) {
       s_gbest = DBL_MAX;
       s_since = 0;
@@ -465,39 +772,10 @@ __global__ void __launch_bounds__(1024) k_batch_solve(BatchArgs a, BatchSmem ly,
     __syncthreads();
     int epoch = 0;
     for (; epoch < a.epochs && !s_stop; ++epoch) {
-      // Weights (k_weights): segment per row.
-      for (int r = seg; r < rows; r += nthr / LANES) {
-        int c = 0, e = INT_MIN;
-        if (sg.lane < k) {
-          c = s_cand[r * k + sg.lane];
-          if (c > 0) e = s_A[ld_cg_u8(tau + (size_t)r * stride + c)] - (int)s_lvl[r * k + sg.lane];
-        }
-        const int emax = sg.imax(e);
-        if (sg.lane < k) {
-          uint32_t w = 0u;
-          if (c > 0) {
-            const int rr = emax - e;
-            w = s_lut[rr > kRelMax ? kRelMax : rr];
-          }
-          s_w[r * k + sg.lane] = w;
-        }
-      }
+      batch_weights<LPA>(a, I, s_cand, bt.fwd, s_A, s_lut, s_w, rows, S);
       __syncthreads();
-      // Construction, ants_per_block ants at a time.
-      uint32_t *dbuf = reinterpret_cast<uint32_t *>(smem + ly.off_draw) + seg * 128;
-      for (int a0 = 0; a0 < a.m; a0 += ants_per_block) {
-        const int ant = a0 + seg;
-        if (seg < ants_per_block && ant < a.m) {
-          const long long ai = (long long)ii * a.m + ant;
-          if (I.unit) {
-            if (V == 1) seg_build_ant<LANES, 1, true>(a, I, sg, s_cand, s_w, s_coords, s_dem, dbuf, seed, ant, (uint32_t)epoch, ai);
-            else seg_build_ant<LANES, 2, true>(a, I, sg, s_cand, s_w, s_coords, s_dem, dbuf, seed, ant, (uint32_t)epoch, ai);
-          } else {
-            if (V == 1) seg_build_ant<LANES, 1, false>(a, I, sg, s_cand, s_w, s_coords, s_dem, dbuf, seed, ant, (uint32_t)epoch, ai);
-            else seg_build_ant<LANES, 2, false>(a, I, sg, s_cand, s_w, s_coords, s_dem, dbuf, seed, ant, (uint32_t)epoch, ai);
-          }
-        }
-      }
+      for (int a0 = 0; a0 < a.m; a0 += sh.round)
+        build_ants<LPA, E>(a, sh, I, tb, smem, seed, (uint32_t)epoch, a0, ii);
       __syncthreads();
       // Iteration best: first minimum among feasible ants (k_best).
       {
@@ -563,52 +841,24 @@ __global__ void __launch_bounds__(1024) k_batch_solve(BatchArgs a, BatchSmem ly,
         }
         __syncthreads();
       }
-      const int R = n + 2 * K;
+      const int total = n + 2 * K;  // entries of a feasible ant's routes
+      const int *it_nodes = a.routes + I.route_off + (long long)s_best * total;
       if (s_improved) {
-        const int *src = a.routes + I.route_off + (long long)s_best * R;
         const int *sl = a.lens + I.lens_off + (long long)s_best * K;
-        int total = 0;
-        for (int v = 0; v < K; ++v) total += sl[v];
-        for (int t = tid; t < total; t += nthr) a.gbest_nodes[I.gbest_off + t] = src[t];
+        for (int t = tid; t < total; t += nthr) a.gbest_nodes[I.gbest_off + t] = it_nodes[t];
         for (int v = tid; v < K; v += nthr) a.gbest_lens[I.gblens_off + v] = sl[v];
       }
-      __syncthreads();
       if (s_found) {
-        // Evaporation (k_evap_deposit's sweep), then both deposits.
-        PheromoneView pv;
-        pv.tau = tau;
-        pv.total = (unsigned long long)rows * rows;
-        pv.log_min = a.log_min;
-        pv.log_step = a.log_step;
-        pv.q_min = 0;
-        pv.q_max = 255;
-        pv.delta = a.delta;
-        pv.pad = 0;
-        const int fl = (int)a.delta;
-        const uint32_t floor4 = 0x01010101u * (uint32_t)fl, delta4 = 0x01010101u * a.delta;
-        uint4 *t4 = reinterpret_cast<uint4 *>(tau);
-        const unsigned long long nvec = pv.total / 16;
-        for (unsigned long long e = tid; e < nvec; e += nthr) {
-          uint4 x = __ldcg(t4 + e);
-          x.x = __vsub4(__vmaxu4(x.x, floor4), delta4);
-          x.y = __vsub4(__vmaxu4(x.y, floor4), delta4);
-          x.z = __vsub4(__vmaxu4(x.z, floor4), delta4);
-          x.w = __vsub4(__vmaxu4(x.w, floor4), delta4);
-          __stcg(t4 + e, x);
-        }
-        for (unsigned long long e = nvec * 16 + tid; e < pv.total; e += nthr) {
-          const uint8_t q = ld_cg_u8(tau + e);
-          st_cg_u8(tau + e, ((int)q > fl) ? (uint8_t)(q - a.delta) : (uint8_t)0);
+        // Evaporation max(q, delta) - delta (q_min = 0), then both deposits.
+        const uint32_t delta4 = 0x01010101u * a.delta;
+        for (int e = tid; e < rows * S / 2; e += nthr) {
+          uint32_t *x = reinterpret_cast<uint32_t *>(bt.fwd) + e;
+          *x = __vsub4(__vmaxu4(*x, delta4), delta4);
         }
         __syncthreads();
-        deposit_solution(pv, stride,
-                         CompactNodes{a.routes + I.route_off + (long long)s_best * R},
-                         a.lens + I.lens_off + (long long)s_best * K, K, s_dep_i,
-                         K <= a.max_K ? s_off : nullptr);
+        batch_deposit(bt, it_nodes, total, s_dep_i);
         __syncthreads();
-        deposit_solution(pv, stride, CompactNodes{a.gbest_nodes + I.gbest_off},
-                         a.gbest_lens + I.gblens_off, K, s_dep_g,
-                         K <= a.max_K ? s_off : nullptr);
+        batch_deposit(bt, a.gbest_nodes + I.gbest_off, total, s_dep_g);
         __syncthreads();
       }
     }
@@ -620,38 +870,29 @@ __global__ void __launch_bounds__(1024) k_batch_solve(BatchArgs a, BatchSmem ly,
   }
 }
 
-template <int LANES>
-cudaError_t launch_batch_lanes(const BatchArgs &a, const BatchSmem &ly, int grid, int threads,
-                               int apb, int v, cudaStream_t s) {
-  if (v == 1) k_batch_solve<LANES, 1><<<grid, threads, ly.total, s>>>(a, ly, apb);
-  else k_batch_solve<LANES, 2><<<grid, threads, ly.total, s>>>(a, ly, apb);
-  return cudaGetLastError();
+using BatchKernel = void (*)(BatchArgs, BatchShape);
+
+BatchKernel batch_kernel(int lpa, int elem) {
+  if (lpa == 4) {
+    return elem == 1 ? k_batch_solve<4, 1> : (elem == 2 ? k_batch_solve<4, 2> : k_batch_solve<4, 4>);
+  }
+  return elem == 1 ? k_batch_solve<8, 1> : (elem == 2 ? k_batch_solve<8, 2> : k_batch_solve<8, 4>);
 }
 
-// Opts the kernel into the largest dynamic shared memory its static shared
-// variables leave free.
-template <int LANES, int V>
+// Opts the kernels into the largest dynamic shared memory their static
+// shared variables leave free.
 cudaError_t configure_batch() {
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, k_batch_solve<LANES, V>);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_batch_solve<LANES, V>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              construct_max_smem() - (int)fa.sharedSizeBytes);
-}
-
-template <int LANES, int V>
-int batch_static_smem() {
-  cudaFuncAttributes fa;
-  if (cudaFuncGetAttributes(&fa, k_batch_solve<LANES, V>) != cudaSuccess) return 1 << 20;
-  return (int)fa.sharedSizeBytes;
-}
-
-template <int LANES, int V>
-int occupancy_batch(int threads, size_t smem) {
-  int blocks = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_batch_solve<LANES, V>, threads, smem);
-  return blocks;
+  for (int lpa : {4, 8})
+    for (int elem : {1, 2, 4}) {
+      cudaFuncAttributes fa;
+      const void *f = reinterpret_cast<const void *>(batch_kernel(lpa, elem));
+      cudaError_t e = cudaFuncGetAttributes(&fa, f);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 construct_max_smem() - (int)fa.sharedSizeBytes);
+      if (e != cudaSuccess) return e;
+    }
+  return cudaSuccess;
 }
 
 }  // namespace
@@ -665,7 +906,7 @@ struct aco_b200_batch {
   cudaStream_t stream = nullptr;
   bool own_stream = true;
   bool ready = false;
-  int count = 0, m = 0, k = 0, epochs = 0, max_rows = 0, max_K = 0, max_n = 0;
+  int count = 0, m = 0, k = 0, epochs = 0, max_rows = 0, max_K = 0, max_n = 0, max_demand = 0;
   BatchArgs args = {};
   std::vector<BatchInst> inst;
   std::vector<int> sizes;  // work estimate per instance
@@ -722,6 +963,38 @@ static int batch_v_for(int lanes, int max_rows) {
   return 0;
 }
 
+// The launch for the batch: every ant of a colony at a time where a block's
+// threads and shared memory allow; of the ways to do that, the one with the
+// most blocks resident at once that the instances can use, and then with the
+// pheromone levels in shared memory.
+static bool choose_shape(const aco_b200_batch *b, BatchShape *out, int *grid) {
+  const int elem = demand_bytes(b->max_demand), lpa = b->k <= 16 ? 4 : 8;
+  const int most = kBatchThreads / lpa;
+  const int rounds = (b->m + most - 1) / most;
+  const int useful = (b->count + b->num_sms - 1) / b->num_sms;  // blocks per SM with work
+  int best = 0;
+  for (int round = (b->m + rounds - 1) / rounds; round >= 1 && best == 0;
+       round = round > 8 ? round * 3 / 4 : round - 1) {
+    for (int tau_smem = 1; tau_smem >= 0; --tau_smem) {
+      const BatchShape sh =
+          batch_shape(b->max_rows, b->max_n, b->k, b->m, elem, round, tau_smem != 0);
+      if ((int)sh.total + 64 > construct_max_smem()) continue;
+      int per_sm = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+              &per_sm, reinterpret_cast<const void *>(batch_kernel(sh.lpa, elem)), sh.threads,
+              sh.total) != cudaSuccess)
+        return false;
+      per_sm = std::min(per_sm, useful);
+      if (per_sm > best) {
+        best = per_sm;
+        *out = sh;
+      }
+    }
+  }
+  *grid = std::min(best * b->num_sms, b->count);
+  return best > 0;
+}
+
 extern "C" {
 
 int aco_b200_batch_create(aco_b200_batch **out, int device) {
@@ -735,10 +1008,7 @@ int aco_b200_batch_create(aco_b200_batch **out, int device) {
   cudaSetDevice(device);
   cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, device);
   cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = configure_batch<16, 1>();
-  if (e == cudaSuccess) e = configure_batch<16, 2>();
-  if (e == cudaSuccess) e = configure_batch<32, 1>();
-  if (e == cudaSuccess) e = configure_batch<32, 2>();
+  if (e == cudaSuccess) e = configure_batch();
   if (e != cudaSuccess) {
     fprintf(stderr, "aco_b200_batch_create: %s\n", cudaGetErrorString(e));
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -784,8 +1054,8 @@ int aco_b200_batch_setup(aco_b200_batch *b, const aco_b200_batch_problem *p) {
   const int m = p->ants > 0 ? p->ants : 64;
   b->inst.assign(count, BatchInst{});
   b->sizes.assign(count, 0);
-  long long node = 0, taub = 0, route = 0, lensn = 0, gb = 0, gbl = 0, rep = 0;
-  int max_rows = 0, max_K = 0, max_n = 0;
+  long long node = 0, route = 0, lensn = 0, gb = 0, gbl = 0, rep = 0;
+  int max_rows = 0, max_K = 0, max_n = 0, max_demand = 1;
   std::vector<float2> xy;
   std::vector<int> dem;
   std::vector<long long> seg_off(count);
@@ -804,14 +1074,12 @@ int aco_b200_batch_setup(aco_b200_batch *b, const aco_b200_batch_problem *p) {
     I.cap = (int)cap;
     long long tot = 0;
     int mx = 1;
-    bool unit = true;
     for (int j = 0; j <= n; ++j) {
       const int d = p->demand ? p->demand[node + j] : (j ? 1 : 0);
       if ((j == 0 && d != 0) || (j > 0 && d < 1)) return ACO_ERR_INVALID_INPUT;
       if (j > 0) {
         tot += d;
         mx = d > mx ? d : mx;
-        unit = unit && d == 1;
       }
       xy.push_back(make_float2(p->x[node + j], p->y[node + j]));
       dem.push_back(d);
@@ -819,18 +1087,16 @@ int aco_b200_batch_setup(aco_b200_batch *b, const aco_b200_batch_problem *p) {
     if (tot > 0x7fffffffLL) return ACO_ERR_INVALID_INPUT;
     I.total_demand = (int)tot;
     I.max_demand = mx;
-    I.unit = unit ? 1 : 0;
+    max_demand = std::max(max_demand, mx);
     I.node_off = node;
     seg_off[i] = node;
     seg_n[i] = n;
-    I.tau_off = taub;
     I.route_off = route;
     I.lens_off = lensn;
     I.gbest_off = gb;
     I.gblens_off = gbl;
     I.rep_off = rep;
     node += n + 1;
-    taub += (((long long)(n + 1) * (n + 1)) + 15) & ~15LL;
     route += (long long)m * (n + 2 * K);
     lensn += (long long)m * K;
     gb += n + 2 * K;
@@ -852,6 +1118,7 @@ int aco_b200_batch_setup(aco_b200_batch *b, const aco_b200_batch_problem *p) {
   b->max_rows = max_rows;
   b->max_K = max_K;
   b->max_n = max_n;
+  b->max_demand = max_demand;
 
   float lmin = logf(0.0001f), lmax = logf(100.0f);
   float step = (lmax - lmin) / 255.0f;
@@ -888,8 +1155,6 @@ int aco_b200_batch_setup(aco_b200_batch *b, const aco_b200_batch_problem *p) {
   a.delta = delta;
   a.q_tau0 = q0;
   a.seed = p->seed;
-  a.max_rows = max_rows;
-  a.max_K = max_K;
   BatchInst *d_inst;
   int *d_order;
   float2 *d_coords;
@@ -916,11 +1181,11 @@ int aco_b200_batch_setup(aco_b200_batch *b, const aco_b200_batch_problem *p) {
     b->carve(&d_thr, kThresholds);
     b->carve(&d_soff, count);
     b->carve(&d_sn, count);
-    b->carve(&a.tau, taub);
+    b->carve(&a.tau, node * 2 * kMaxCand);
     b->carve(&a.routes, route);
     b->carve(&a.lens, lensn);
     b->carve(&a.loads, lensn);
-    b->carve(&a.repc, lensn);
+    b->carve(&a.last, lensn);
     b->carve(&a.rep, rep);
     b->carve(&a.cost, (long long)count * m);
     b->carve(&a.feasible, (long long)count * m);
@@ -982,8 +1247,8 @@ int aco_b200_batch_set_tuning(aco_b200_batch *b, const aco_b200_batch_tuning *t)
   if ((t->ants_per_block * t->lanes_per_ant) % 32) return ACO_ERR_INVALID_INPUT;
   if (batch_v_for(t->lanes_per_ant, b->max_rows) == 0) return ACO_ERR_INVALID_INPUT;
   const int threads = t->ants_per_block * t->lanes_per_ant;
-  const BatchSmem ly = batch_smem(b->max_rows, b->k, t->ants_per_block, threads, b->max_K);
-  if ((int)ly.total + batch_static_smem<32, 2>() > construct_max_smem()) return ACO_ERR_INVALID_INPUT;
+  if ((int)shape_bytes(b->max_rows, b->k, t->ants_per_block, threads, b->max_K) > construct_max_smem())
+    return ACO_ERR_INVALID_INPUT;
   // Queue order: 0 = as given, 1 = largest work first.
   std::vector<int> order(b->count);
   std::iota(order.begin(), order.end(), 0);
@@ -1008,22 +1273,14 @@ int aco_b200_batch_get_tuning(aco_b200_batch *b, aco_b200_batch_tuning *t) {
 int aco_b200_batch_enqueue(aco_b200_batch *b) {
   if (!b || !b->ready) return ACO_ERR_INVALID_INPUT;
   cudaSetDevice(b->device);
-  const aco_b200_batch_tuning &t = b->tuning;
-  const int threads = t.ants_per_block * t.lanes_per_ant;
-  const BatchSmem ly = batch_smem(b->max_rows, b->k, t.ants_per_block, threads, b->max_K);
-  const int v = batch_v_for(t.lanes_per_ant, b->max_rows);
-  int per_sm = 0;
-  if (t.lanes_per_ant == 16) per_sm = v == 1 ? occupancy_batch<16, 1>(threads, ly.total) : occupancy_batch<16, 2>(threads, ly.total);
-  else per_sm = v == 1 ? occupancy_batch<32, 1>(threads, ly.total) : occupancy_batch<32, 2>(threads, ly.total);
-  if (per_sm < 1) return ACO_ERR_INVALID_INPUT;
-  int grid = per_sm * b->num_sms;
-  if (grid > b->count) grid = b->count;
+  BatchShape sh;
+  int grid = 0;
+  if (!choose_shape(b, &sh, &grid)) return ACO_ERR_INVALID_INPUT;
   auto record = [&](cudaStream_t s) -> cudaError_t {
     cudaError_t e = cudaMemsetAsync(b->args.queue, 0, sizeof(unsigned int), s);
     if (e != cudaSuccess) return e;
-    return (t.lanes_per_ant == 16)
-               ? launch_batch_lanes<16>(b->args, ly, grid, threads, t.ants_per_block, v, s)
-               : launch_batch_lanes<32>(b->args, ly, grid, threads, t.ants_per_block, v, s);
+    batch_kernel(sh.lpa, sh.elem)<<<grid, sh.threads, sh.total, s>>>(b->args, sh);
+    return cudaGetLastError();
   };
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   BTRY(cudaStreamIsCapturing(b->stream, &cap));
@@ -1034,11 +1291,10 @@ int aco_b200_batch_enqueue(aco_b200_batch *b) {
     return ACO_OK;
   }
   // The key: every argument of the two graph nodes.
-  std::vector<unsigned char> key(sizeof(BatchArgs) + sizeof(BatchSmem) + 4 * sizeof(int));
-  const int shape[4] = {grid, threads, t.ants_per_block, v * 64 + t.lanes_per_ant};
+  std::vector<unsigned char> key(sizeof(BatchArgs) + sizeof(BatchShape) + sizeof(int));
   memcpy(key.data(), &b->args, sizeof(BatchArgs));
-  memcpy(key.data() + sizeof(BatchArgs), &ly, sizeof(BatchSmem));
-  memcpy(key.data() + sizeof(BatchArgs) + sizeof(BatchSmem), shape, sizeof(shape));
+  memcpy(key.data() + sizeof(BatchArgs), &sh, sizeof(BatchShape));
+  memcpy(key.data() + sizeof(BatchArgs) + sizeof(BatchShape), &grid, sizeof(int));
   if (!b->graph || key != b->graph_key) {
     b->drop_graph();
     cudaGraph_t g = nullptr;

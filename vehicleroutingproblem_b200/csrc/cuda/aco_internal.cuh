@@ -412,6 +412,162 @@ __device__ inline unsigned long long warp_knn(const float2 *coords, int n, int k
   return list;
 }
 
+// What an ant still has to serve: one element per node in shared memory,
+// the customer's demand while it is unvisited and the largest value of the
+// type once it is visited (the depot and the padding from the start).  One
+// load and one compare against the room left answer "unvisited and fits",
+// one store marks a visit, and the loaded element is the demand the step
+// needs.  E = 1, 2 or 4 bytes, the smallest that holds every demand below
+// that largest value; E = 0: a bitmap (word wi holding nodes 32 wi .. 32 wi
+// + 31) with the demands in global memory, for instances whose elements do
+// not fit beside the other ants of the block.
+//
+// The elements replace a bitmap in registers read by a shuffle: that took a
+// shuffle, the bit's forming and testing, a second load for the demand and a
+// test whether demands bind at all, 15 instructions more per step.
+template <int E>
+struct Unserved {
+  static constexpr uint32_t kVisited = E == 1 ? 0xffu : (E == 2 ? 0xffffu : 0xffffffffu);
+  uint32_t base;     // shared address of this ant's elements
+  uint32_t chunks;   // 16-byte pieces
+  const int *dem;    // E = 0
+
+  // The accesses are volatile so that they keep their order: a visit's store
+  // comes before the next step's loads.
+  __device__ __forceinline__ uint32_t get(int node) const {
+    uint32_t v;
+    if (E == 1) {
+      asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(base + (uint32_t)node));
+    } else if (E == 2) {
+      asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(base + 2u * (uint32_t)node));
+    } else if (E == 4) {
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(base + 4u * (uint32_t)node));
+    } else {
+      const uint32_t d = (uint32_t)__ldg(dem + node);
+      asm volatile("ld.shared.u32 %0, [%1];"
+                   : "=r"(v) : "r"(base + 4u * ((uint32_t)node >> 5)));
+      v = (__funnelshift_r(v, v, node) & 1u) ? kVisited : d;
+    }
+    return v;
+  }
+  // Of nodes 2 q and 2 q + 1.
+  __device__ __forceinline__ void get_pair(int q, uint32_t &e0, uint32_t &e1) const {
+    if (E == 1) {
+      uint32_t v;
+      asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(base + 2u * (uint32_t)q));
+      e0 = v & 0xffu;
+      e1 = v >> 8;
+    } else if (E == 2) {
+      uint32_t v;
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(base + 4u * (uint32_t)q));
+      e0 = v & 0xffffu;
+      e1 = v >> 16;
+    } else if (E == 4) {
+      asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];"
+                   : "=r"(e0), "=r"(e1) : "r"(base + 8u * (uint32_t)q));
+    } else {
+      uint32_t v;
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(base + 4u * ((uint32_t)q >> 4)));
+      const int2 d = __ldg(reinterpret_cast<const int2 *>(dem) + q);
+      v >>= (2 * q) & 31;
+      e0 = (v & 1u) ? kVisited : (uint32_t)d.x;
+      e1 = (v & 2u) ? kVisited : (uint32_t)d.y;
+    }
+  }
+  // Every lane calls it with the same node.
+  __device__ __forceinline__ void mark(int node) {
+    if (E == 1) {
+      asm volatile("st.shared.u8 [%0], %1;" ::"r"(base + (uint32_t)node), "r"(kVisited));
+    } else if (E == 2) {
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(base + 2u * (uint32_t)node), "r"(kVisited));
+    } else if (E == 4) {
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(base + 4u * (uint32_t)node), "r"(kVisited));
+    } else {
+      const uint32_t a = base + 4u * ((uint32_t)node >> 5);
+      uint32_t v;
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v | __funnelshift_l(0u, 1u, node)));
+    }
+  }
+  // The room left as the elements are compared with it.
+  __device__ __forceinline__ uint32_t limit(int room) const {
+    return (E == 1 || E == 2) ? min((uint32_t)room, kVisited - 1u) : (uint32_t)room;
+  }
+  // E = 0: the bitmap of an unserved instance (by one warp); the elements
+  // are copied from iv.elems.
+  __device__ __forceinline__ void init_bits(int n, int lane) {
+    for (uint32_t wi = (uint32_t)lane; wi < 4u * chunks; wi += 32u) {
+      const int lo = (int)wi << 5, valid = n + 1 - lo;  // nodes lo..n in this word
+      uint32_t v = lo == 0 ? 1u : 0u;
+      if (valid < 32) v |= valid <= 0 ? 0xffffffffu : (0xffffffffu << valid);
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(base + 4u * wi), "r"(v));
+    }
+    __syncwarp();
+  }
+};
+
+// Bits of the squared distance of (x, y) from the point whose negated
+// coordinates are npc, both differences and both squares in one packed
+// operation each: the roundings of dist2f.
+__device__ __forceinline__ uint32_t dist2_bits(float x, float y, unsigned long long npc) {
+  float sx, sy;
+  asm("{\n .reg .b64 p, d;\n"
+      " mov.b64 p, {%2, %3};\n"
+      " add.rn.f32x2 d, p, %4;\n"
+      " mul.rn.f32x2 d, d, d;\n"
+      " mov.b64 {%0, %1}, d;\n}\n"
+      : "=f"(sx), "=f"(sy) : "f"(x), "f"(y), "l"(npc));
+  return __float_as_uint(__fadd_rn(sx, sy));
+}
+
+// The full scan: lane L takes the node pairs L, L + 32, ... in ascending
+// order, visited or not, kPairs at a time with their loads issued together
+// (16 bytes of coordinates per lane) and no branch per node; pairs past the
+// last repeat it.  Walking only the unvisited nodes, from a bitmap's set
+// bits, cost more per scan while many are left, and a scan is made when few
+// are left nearby, not overall.  Returns the lane's first nearest eligible
+// node (its squared distance's bits in *best_h_out).  Out of line: the
+// batch's registers do not weigh on the step loop (the scan is rare).
+// kGlobal: the coordinates are in global memory.
+template <bool kGlobal, int E, int kPairs>
+__device__ __noinline__ uint32_t scan_pairs(const float2 *coords, Unserved<E> us, int n,
+                                            float2 pc, uint32_t room, int lane,
+                                            uint32_t *best_h_out) {
+  uint32_t best_h = 0xffffffffu, best_n = 0xffffffffu;
+  const int last = n >> 1;
+  unsigned long long npc;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(npc) : "f"(-pc.x), "f"(-pc.y));
+#pragma unroll 1
+  for (int b = lane; b <= last; b += 32 * kPairs) {
+    float4 p[kPairs];
+    uint32_t h[2 * kPairs];
+#pragma unroll
+    for (int i = 0; i < kPairs; ++i) {
+      const int q = min(b + 32 * i, last);
+      const float4 *c4 = reinterpret_cast<const float4 *>(coords) + q;
+      p[i] = kGlobal ? __ldg(c4) : *c4;
+      us.get_pair(q, h[2 * i], h[2 * i + 1]);
+    }
+    uint32_t m = 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < kPairs; ++i) {
+      const uint32_t h0 = dist2_bits(p[i].x, p[i].y, npc);
+      const uint32_t h1 = dist2_bits(p[i].z, p[i].w, npc);
+      h[2 * i] = h[2 * i] <= room ? h0 : 0xffffffffu;
+      h[2 * i + 1] = h[2 * i + 1] <= room ? h1 : 0xffffffffu;
+      m = min(m, min(h[2 * i], h[2 * i + 1]));
+    }
+    if (m < best_h) {
+      best_h = m;
+#pragma unroll
+      for (int i = 2 * kPairs - 1; i >= 0; --i)
+        if (h[i] == m) best_n = (uint32_t)(2 * min(b + 32 * (i >> 1), last) + (i & 1));
+    }
+  }
+  *best_h_out = best_h;
+  return best_n;
+}
+
 // ---------------------------------------------------------------------------
 // Pheromone deposit (shared by the native kernels and the drop-in kernels)
 // ---------------------------------------------------------------------------
