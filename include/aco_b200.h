@@ -392,16 +392,11 @@ ACO_API int aco_b200_batch_apply_prior(aco_b200_batch *batch, aco_b200_prior *pr
  * the evaporation step as in the reference (src/cuda/aco_cuda.cu:214-215).
  * Same result as aco_b200_evaporate_deposit.
  *
- * The kernel's scratch is a fixed array in the library's device memory
- * (16.6 KB per GPU), so K may be at most 4096 routes; larger K is rejected
- * with ACO_ERR_INVALID_INPUT and a message on stderr.  Every call on a GPU
- * shares that array: calls whose kernels overlap on the GPU race, so issue
- * them on one stream or otherwise order them.  The first call on each
- * device looks up the array's device address (cudaGetSymbolAddress); make
- * that first call before capturing a stream into a CUDA graph.  The address
- * is kept for the life of the process: it does not survive a device reset
- * (cudaDeviceReset, or the primary context destroyed and made again), after
- * which this entry point must not be called in the same process.
+ * Three launches (the sweep, one per deposit; no scratch in device memory).
+ * The route offsets are kept in shared memory, so K may be at most 4096
+ * routes; larger K is rejected with ACO_ERR_INVALID_INPUT and a message on
+ * stderr.  Calls on different matrices are independent; calls on one matrix
+ * are ordered by their stream.
  */
 ACO_API int aco_b200_evaporate_deposit_noalloc(uint8_t *d_tau, int n, int K,
                                                const int *d_iter_nodes,

@@ -734,5 +734,91 @@ __device__ void deposit_solution(const PheromoneView &pv, size_t stride,
 
 constexpr int kDepositSmemRoutes = 4096;
 
+__device__ __forceinline__ uint32_t evap4(uint32_t x, uint32_t floor4,
+                                          uint32_t delta4) {
+  return __vsub4(__vmaxu4(x, floor4), delta4);
+}
+
+// Evaporation sweep of pv.total bytes from src to dst (src == dst: in
+// place), q > q_min + delta ? q - delta : q_min as max(q, q_min + delta) -
+// delta on 16 bytes at a time (kernel_evaporate_tau,
+// src/cuda/aco_cuda_kernels.cu:145-155).  HBM bounds it.  Each thread keeps
+// kUnroll 16-byte loads in flight before its stores (a block covers
+// kUnroll * blockDim.x vectors per trip), and the loads and stores are
+// streaming (evict-first), so a matrix larger than L2 passes through without
+// displacing the construction's tables.  Block 0 also does the tail past the
+// last whole vector.
+template <int kUnroll>
+__device__ __forceinline__ void evap_sweep(const uint8_t *src, uint8_t *dst,
+                                           unsigned long long total, uint8_t q_min,
+                                           uint8_t delta) {
+  const int fl = (int)q_min + (int)delta;
+  const bool sat_all = fl > 255;
+  const uint32_t floor4 = 0x01010101u * (uint32_t)(sat_all ? 0 : fl);
+  const uint32_t delta4 = 0x01010101u * (uint32_t)delta;
+  const uint32_t qmin4 = 0x01010101u * (uint32_t)q_min;
+  const unsigned long long nvec = total / 16;
+  const uint4 *s4 = reinterpret_cast<const uint4 *>(src);
+  uint4 *d4 = reinterpret_cast<uint4 *>(dst);
+  const unsigned long long tile = (unsigned long long)kUnroll * blockDim.x;
+  const unsigned long long step = tile * gridDim.x;
+  for (unsigned long long base = blockIdx.x * tile + threadIdx.x; base < nvec; base += step) {
+    uint4 v[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const unsigned long long i = base + (unsigned long long)u * blockDim.x;
+      if (i < nvec) v[u] = __ldcs(s4 + i);
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const unsigned long long i = base + (unsigned long long)u * blockDim.x;
+      if (i < nvec) {
+        uint4 r = v[u];
+        if (sat_all) {
+          r = make_uint4(qmin4, qmin4, qmin4, qmin4);
+        } else {
+          r.x = evap4(r.x, floor4, delta4);
+          r.y = evap4(r.y, floor4, delta4);
+          r.z = evap4(r.z, floor4, delta4);
+          r.w = evap4(r.w, floor4, delta4);
+        }
+        __stcs(d4 + i, r);
+      }
+    }
+  }
+  if (blockIdx.x == 0) {
+    for (unsigned long long i = nvec * 16 + threadIdx.x; i < total; i += blockDim.x) {
+      const uint8_t q = src[i];
+      dst[i] = ((int)q > fl) ? (uint8_t)(q - delta) : q_min;
+    }
+  }
+}
+
+// Programmatic launches: the kernel may start while the one before it on the
+// stream ends (launch_after), reads only what no kernel in flight writes, and
+// waits here before it touches what that one wrote.
+__device__ __forceinline__ void wait_for_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void let_next_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                                cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
 }  // namespace acob200
 #endif

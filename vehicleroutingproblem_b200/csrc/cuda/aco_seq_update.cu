@@ -12,7 +12,7 @@
 // of traffic per cell instead of 32-48), and a small kernel does 2-5 on the
 // touched cells only:
 //   k_seq_mark     sets the bit of every deposit cell (i != j)
-//   k_seq_sweep    the matrix two cells (16 bytes) at a time, four pairs per
+//   k_seq_sweep    the matrix two cells (16 bytes) at a time, three pairs per
 //                  thread in flight: evaporate; unmarked cells also clamp
 //                  and reset
 //   k_seq_add      the adds of one solution, one launch for the iteration
@@ -42,8 +42,14 @@ using namespace acob200;
 namespace {
 
 constexpr int kSeqMaxRoutes = 8192;
-constexpr int kSweepThreads = 256;
-constexpr int kSweepUnroll = 4;
+// The sweep's tile: 64 threads with 3 cell pairs each, a block per tile.  HBM
+// bounds it, and what matters is that the blocks in flight read and write
+// close to each other: one resident wave of 256-thread blocks striding over
+// the matrix took 706 us per update at n=16000 (337 at n=11001, 146 at
+// n=7000), tiles of 256 x 4 751, 256 x 2 748, 128 x 4 673, 128 x 3 626,
+// 64 x 4 657 and 64 x 3 619 (302, 132).
+constexpr int kSweepThreads = 64;
+constexpr int kSweepUnroll = 3;
 
 struct SeqArgs {
   double *tau;
@@ -56,6 +62,7 @@ struct SeqArgs {
   int reset;
   double tau0;
   unsigned int *marks;            // (n+1)^2 bits, zero between calls
+  double inv_n2;                  // 1 / (n + 2)
 };
 
 __device__ __forceinline__ double clamp_reset(double x, const SeqArgs &a) {
@@ -67,20 +74,30 @@ __device__ __forceinline__ double clamp_reset(double x, const SeqArgs &a) {
 
 // Arc offsets of one solution in shared memory: route v's arcs are
 // [off[v], off[v+1]) in the solution's arc order, its first entry is at
-// off[v] + v.  Returns the number of arcs.
-__device__ int load_arc_offsets(const int *lens, int K, int *off) {
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int v = 0; v < K; ++v) {
-      off[v] = acc;
-      acc += lens[v] - 1;
-    }
-    off[K] = acc;
+// off[v] + v.  By one warp.
+__device__ __forceinline__ void load_arc_offsets(const int *lens, int K, int *off) {
+  const int lane = threadIdx.x & 31;
+  int carry = 0;
+  for (int b = 0; b < K; b += 32) {
+    const int v = b + lane;
+    const int arcs = v < K ? lens[v] - 1 : 0;
+    const int inc = (int)warp_incl_scan((uint32_t)arcs, lane);
+    if (v < K) off[v + 1] = carry + inc;
+    carry += __shfl_sync(kFull, inc, 31);
   }
+  if (lane == 0) off[0] = 0;
+}
+
+// Both solutions' offsets (the global best's behind the iteration best's, if
+// there is one), by a warp each; the numbers of their arcs.
+__device__ __forceinline__ void load_both_offsets(const SeqArgs &a, int *off, int *total_it,
+                                                  int *total_gb) {
+  const int warp = threadIdx.x >> 5;
+  if (warp == 0) load_arc_offsets(a.it_lens, a.K, off);
+  if (warp == 1 && a.gb_nodes) load_arc_offsets(a.gb_lens, a.K, off + a.K + 1);
   __syncthreads();
-  const int total = off[K];
-  __syncthreads();
-  return total;
+  *total_it = off[a.K];
+  *total_gb = a.gb_nodes ? off[2 * a.K + 1] : 0;
 }
 
 // Arc j of a solution: (u, v) = (nodes[e], nodes[e+1]).
@@ -105,20 +122,17 @@ constexpr int kArcThreads = 256;
 __global__ void __launch_bounds__(kArcThreads) k_seq_mark(SeqArgs a) {
   extern __shared__ int s_off[];
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, gn = gridDim.x * blockDim.x;
-  for (int which = 0; which < 2; ++which) {
-    const int *nodes = which ? a.gb_nodes : a.it_nodes;
-    const int *lens = which ? a.gb_lens : a.it_lens;
-    if (!nodes) break;
-    const int total = load_arc_offsets(lens, a.K, s_off);
-    for (int j = gt; j < total; j += gn) {
-      int u, v;
-      arc_of(nodes, s_off, a.K, j, &u, &v);
-      if (u == v) continue;  // the diagonal is never swept
-      const unsigned long long c1 = cell(a.n, u, v), c2 = cell(a.n, v, u);
-      atomicOr(a.marks + (c1 >> 5), 1u << (c1 & 31));
-      atomicOr(a.marks + (c2 >> 5), 1u << (c2 & 31));
-    }
-    __syncthreads();
+  int t_it, t_gb;
+  load_both_offsets(a, s_off, &t_it, &t_gb);
+  for (int j = gt; j < t_it + t_gb; j += gn) {
+    const bool gb = j >= t_it;
+    int u, v;
+    arc_of(gb ? a.gb_nodes : a.it_nodes, gb ? s_off + a.K + 1 : s_off, a.K, gb ? j - t_it : j, &u,
+           &v);
+    if (u == v) continue;  // the diagonal is never swept
+    const unsigned long long c1 = cell(a.n, u, v), c2 = cell(a.n, v, u);
+    atomicOr(a.marks + (c1 >> 5), 1u << (c1 & 31));
+    atomicOr(a.marks + (c2 >> 5), 1u << (c2 & 31));
   }
 }
 
@@ -148,7 +162,7 @@ __device__ __forceinline__ double sweep_cell(double x, unsigned long long e, uns
 __global__ void __launch_bounds__(kSweepThreads) k_seq_sweep(SeqArgs a) {
   const unsigned long long cells = (unsigned long long)(a.n + 1) * (unsigned long long)(a.n + 1);
   const unsigned long long n2 = (unsigned long long)a.n + 2;
-  const double inv_n2 = 1.0 / (double)n2;
+  const double inv_n2 = a.inv_n2;
   const unsigned long long nvec = cells / 2;
   double2 *t2 = reinterpret_cast<double2 *>(a.tau);
   const unsigned long long tile = (unsigned long long)kSweepUnroll * blockDim.x;
@@ -163,7 +177,7 @@ __global__ void __launch_bounds__(kSweepThreads) k_seq_sweep(SeqArgs a) {
       m[q] = 0u;
       if (i < nvec) {
         v[q] = __ldcs(t2 + i);
-        m[q] = __ldg(a.marks + ((2 * i) >> 5));
+        m[q] = __ldcg(a.marks + ((2 * i) >> 5));
       }
     }
 #pragma unroll
@@ -189,7 +203,11 @@ __global__ void __launch_bounds__(kArcThreads) k_seq_add(SeqArgs a, int which) {
   const int *nodes = which ? a.gb_nodes : a.it_nodes;
   const int *lens = which ? a.gb_lens : a.it_lens;
   const double d = which ? a.d_gb : a.d_it;
-  const int total = load_arc_offsets(lens, a.K, s_off);
+  let_next_start();
+  if (threadIdx.x < 32) load_arc_offsets(lens, a.K, s_off);
+  __syncthreads();
+  const int total = s_off[a.K];
+  wait_for_previous();
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, gn = gridDim.x * blockDim.x;
   for (int j = gt; j < total; j += gn) {
     int u, v;
@@ -203,26 +221,28 @@ __global__ void __launch_bounds__(kArcThreads) k_seq_add(SeqArgs a, int which) {
 __global__ void __launch_bounds__(kArcThreads) k_seq_clamp(SeqArgs a) {
   extern __shared__ int s_off[];
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, gn = gridDim.x * blockDim.x;
-  for (int which = 0; which < 2; ++which) {
-    const int *nodes = which ? a.gb_nodes : a.it_nodes;
-    const int *lens = which ? a.gb_lens : a.it_lens;
-    if (!nodes) break;
-    const int total = load_arc_offsets(lens, a.K, s_off);
-    for (int j = gt; j < total; j += gn) {
-      int u, v;
-      arc_of(nodes, s_off, a.K, j, &u, &v);
-      if (u == v) continue;
+  int t_it, t_gb;
+  load_both_offsets(a, s_off, &t_it, &t_gb);
+  wait_for_previous();
+  for (int j = gt; j < t_it + t_gb; j += gn) {
+    const bool gb = j >= t_it;
+    int u, v;
+    arc_of(gb ? a.gb_nodes : a.it_nodes, gb ? s_off + a.K + 1 : s_off, a.K, gb ? j - t_it : j, &u,
+           &v);
+    if (u == v) continue;
+    // Both cells' bits are asked for together.
+    unsigned long long c[2] = {cell(a.n, u, v), cell(a.n, v, u)};
+    unsigned int was[2];
 #pragma unroll
-      for (int side = 0; side < 2; ++side) {
-        const unsigned long long c = side ? cell(a.n, v, u) : cell(a.n, u, v);
-        const unsigned int bit = 1u << (c & 31);
-        if (atomicAnd(a.marks + (c >> 5), ~bit) & bit) {
-          double *p = a.tau + c;
-          p[0] = clamp_reset(__ldcg(p), a);
-        }
+    for (int side = 0; side < 2; ++side)
+      was[side] = atomicAnd(a.marks + (c[side] >> 5), ~(1u << (c[side] & 31)));
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      if ((was[side] >> (c[side] & 31)) & 1u) {
+        double *p = a.tau + c[side];
+        p[0] = clamp_reset(__ldcg(p), a);
       }
     }
-    __syncthreads();
   }
 }
 
@@ -264,29 +284,38 @@ extern "C" ACO_API int aco_b200_seq_pheromone_update(
   a.tau_max = tau_max;
   a.reset = reset ? 1 : 0;
   a.tau0 = tau0;
+  a.inv_n2 = 1.0 / (double)(n + 2);
   a.marks = static_cast<unsigned int *>(d_scratch);
   cudaStream_t s = (cudaStream_t)stream;
   const size_t smem = sizeof(int) * (size_t)(K + 1);
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // The sweep: a block per tile.
   const unsigned long long pairs = (unsigned long long)(n + 1) * (unsigned long long)(n + 1) / 2;
   const unsigned long long per_block = (unsigned long long)kSweepUnroll * kSweepThreads;
   unsigned long long g = (pairs + per_block - 1) / per_block;
-  if (g > (unsigned long long)sms * 8) g = (unsigned long long)sms * 8;
   if (g < 1) g = 1;
-  const int grid = (int)g;
-  // The arc kernels: enough blocks for one arc per thread (a solution has
-  // n + K arcs at most), at most 4 per SM.
-  unsigned long long ga = ((unsigned long long)n + K + kArcThreads - 1) / kArcThreads;
-  if (ga > (unsigned long long)sms * 4) ga = (unsigned long long)sms * 4;
-  const int arc_grid = (int)ga;
-  k_seq_mark<<<arc_grid, kArcThreads, smem, s>>>(a);
-  k_seq_sweep<<<grid, kSweepThreads, 0, s>>>(a);
-  k_seq_add<<<arc_grid, kArcThreads, smem, s>>>(a, 0);
-  if (a.gb_nodes) k_seq_add<<<arc_grid, kArcThreads, smem, s>>>(a, 1);
-  k_seq_clamp<<<arc_grid, kArcThreads, smem, s>>>(a);
-  const cudaError_t e = cudaGetLastError();
+  // The arc kernels: one arc per thread (a solution has n + K arcs at most).
+  // Both solutions' offsets fit the default 48 KB of shared memory up to 6143
+  // routes.
+  const int one = (n + K + kArcThreads - 1) / kArcThreads, two = 2 * one;
+  cudaError_t e = cudaSuccess;
+  if (2 * smem > 48 * 1024) {
+    e = cudaFuncSetAttribute(k_seq_mark, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(2 * smem));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_seq_clamp, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(2 * smem));
+  }
+  if (e == cudaSuccess) {
+    k_seq_mark<<<two, kArcThreads, 2 * smem, s>>>(a);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) {
+    k_seq_sweep<<<(unsigned)g, kSweepThreads, 0, s>>>(a);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = launch_after(k_seq_add, one, kArcThreads, smem, s, a, 0);
+  if (e == cudaSuccess && a.gb_nodes) e = launch_after(k_seq_add, one, kArcThreads, smem, s, a, 1);
+  if (e == cudaSuccess) e = launch_after(k_seq_clamp, two, kArcThreads, 2 * smem, s, a);
   if (e != cudaSuccess) {
     fprintf(stderr, "aco_b200_seq_pheromone_update: %s\n", cudaGetErrorString(e));
     return ACO_ERR_BACKEND;
