@@ -794,6 +794,7 @@ __device__ __forceinline__ void evap_sweep(const uint8_t *src, uint8_t *dst,
   }
 }
 
+
 // Programmatic launches: the kernel may start while the one before it on the
 // stream ends (launch_after), reads only what no kernel in flight writes, and
 // waits here before it touches what that one wrote.

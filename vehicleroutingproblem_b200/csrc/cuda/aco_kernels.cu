@@ -243,22 +243,35 @@ cudaError_t launch_fill_u8(uint8_t *p, unsigned long long count, uint8_t v,
 // Per-epoch weights
 // ===========================================================================
 
-__global__ void __launch_bounds__(256) k_weights(InstanceView iv,
-                                                 PheromoneView pv,
-                                                 EpochTables et,
-                                                 DevState *st) {
+// Weights of every row, a warp per row.  Bound by the round trips to L2 (row
+// and state, then pheromone cells); the level and weight tables are in shared
+// memory, fetched before this launch waits for the previous epoch.
+// (Evaporating a small matrix in further blocks of this launch, which leaves
+// the side stream out, measured the same: n=24 14.9 -> 14.7 us per epoch,
+// n=250 64.1 -> 64.7; so did evaporation, deposits and the next weights in
+// one launch: n=24 15.1 -> 15.3, n=1000 214 -> 227.)
+constexpr int kWeightThreads = 256;
+
+__global__ void __launch_bounds__(kWeightThreads) k_weights(InstanceView iv, PheromoneView pv,
+                                                            EpochTables et, DevState *st) {
+  __shared__ int32_t s_A[256];
+  __shared__ uint32_t s_lut[256];
   const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
   const int k = iv.k;
   const size_t stride = (size_t)iv.n + 1;
+  let_next_start();
+  s_A[threadIdx.x] = __ldg(et.A + threadIdx.x);
+  s_lut[threadIdx.x] = __ldg(et.lut + threadIdx.x);
+  wait_for_previous();
   // This warp's first row's candidates and levels, the buffer selector and
   // the stop flag are all requested before any of them is used, so that
   // their round trips overlap.
+  const int warps = gridDim.x * (blockDim.x >> 5);
   const int i0 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  int c0 = 0, l0 = 0;
+  int c = 0, lv = 0;
   if (i0 <= iv.n && lane < k) {
-    c0 = iv.cand[(size_t)i0 * k + lane];
-    l0 = iv.lvl[(size_t)i0 * k + lane];
+    c = iv.cand[(size_t)i0 * k + lane];
+    lv = iv.lvl[(size_t)i0 * k + lane];
   }
   const uint8_t *tau = cur_tau(pv.tau, et.tau_alt, st);
   if (st) {
@@ -269,24 +282,15 @@ __global__ void __launch_bounds__(256) k_weights(InstanceView iv,
     }
     if (stop) return;
   }
+  __syncthreads();
   for (int i = i0; i <= iv.n; i += warps) {
-    int c = 0;
-    int e = INT_MIN;
-    if (lane < k) {
-      int lv;
-      if (i == i0) {
-        c = c0;
-        lv = l0;
-      } else {
-        c = iv.cand[(size_t)i * k + lane];
-        lv = iv.lvl[(size_t)i * k + lane];
-      }
-      if (c > 0) {
-        uint8_t q = tau[(size_t)i * stride + c];
-        e = __ldg(et.A + q) - lv;
-      }
+    if (i != i0 && lane < k) {
+      c = iv.cand[(size_t)i * k + lane];
+      lv = iv.lvl[(size_t)i * k + lane];
     }
-    int emax = __reduce_max_sync(kFull, e);
+    const int q = c > 0 ? (int)tau[(size_t)i * stride + c] : 0;
+    const int e = c > 0 ? s_A[q] - lv : INT_MIN;
+    const int emax = __reduce_max_sync(kFull, e);
     if (et.rdep && lane == 0)
       et.rdep[i] = (emax == INT_MIN) ? 0 : emax - (et.e_dep - (int)et.lvl0[i]);
     if (lane < k) {
@@ -296,7 +300,7 @@ __global__ void __launch_bounds__(256) k_weights(InstanceView iv,
         int r = emax - e;
         if (r > kRelMax) r = kRelMax;
         rel = (uint8_t)r;
-        w = __ldg(et.lut + r);
+        w = s_lut[r];
       }
       et.w[(size_t)i * k + lane] = w;
       et.rel[(size_t)i * k + lane] = rel;
@@ -310,8 +314,7 @@ cudaError_t launch_weights(const InstanceView &iv, const PheromoneView &pv,
   int rows = iv.n + 1;
   int blocks = (rows + 7) / 8;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  k_weights<<<blocks, 256, 0, s>>>(iv, pv, et, st);
-  return cudaGetLastError();
+  return launch_after(k_weights, blocks, kWeightThreads, 0, s, iv, pv, et, st);
 }
 
 // ===========================================================================
@@ -813,22 +816,12 @@ __device__ const uint32_t g_zero_entry = 0u;
 
 template <int L, int E, bool CREF>
 __global__ void __launch_bounds__(512, 1) k_construct(const __grid_constant__ ConstructArgs a) {
-  // Graph replays read the epoch number and the seed from the device state,
-  // so one captured graph serves every solve of a context.
-  uint32_t epoch = a.epoch, seed = a.seed;
-  if (a.st) {
-    const int skip = *(volatile int *)&a.st->skip;
-    if (a.use_state_epoch) {  // requested with the flag: one round trip
-      epoch = *(volatile uint32_t *)&a.st->epoch;
-      seed = *(volatile uint32_t *)&a.st->seed;
-    }
-    if (skip) return;
-  }
+  let_next_start();
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const SmemPlan &pl = a.plan;
   const InstanceView &iv = a.iv;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem);  // fixed tables; weights
   const int t = 31 - lane;  // this lane's candidate
   const bool has = t < iv.k;
 
@@ -846,49 +839,43 @@ __global__ void __launch_bounds__(512, 1) k_construct(const __grid_constant__ Co
     tb.rel = nullptr;
     tb.coords = iv.coords;
   } else {
-    // Bytes 8..15 of the block's shared memory hold the zero entry.
-    tb.cand = reinterpret_cast<const uint16_t *>(smem + (has ? pl.off_cand + 2u * t : 8u));
-    tb.w = reinterpret_cast<const uint32_t *>(smem + (has ? pl.off_w + 4u * t : 8u));
-    tb.rel = smem + (has ? pl.off_w + t : 12u);
+    // Bytes 16..23 of the block's shared memory hold the zero entry.
+    tb.cand = reinterpret_cast<const uint16_t *>(smem + (has ? pl.off_cand + 2u * t : 16u));
+    tb.w = reinterpret_cast<const uint32_t *>(smem + (has ? pl.off_w + 4u * t : 16u));
+    tb.rel = smem + (has ? pl.off_w + t : 20u);
     tb.coords = reinterpret_cast<const float2 *>(smem + pl.off_coords);
   }
   if (L == kLayoutSmemPacked) {
     uint32_t *lut = reinterpret_cast<uint32_t *>(smem + pl.off_lut);
     for (int r = threadIdx.x; r < 256; r += blockDim.x) lut[r] = __ldg(a.et.lut + r);
   }
-  // Staging by bulk copies: the tables (rows from global memory: none) and
-  // every ant's elements (E = 0: none).
-  constexpr bool kStage = L != kLayoutGlobal || E > 0;
-  if (kStage) {
-    if (threadIdx.x == 0) {
-      mbar_init(bar, 1);
-      fence_mbar_init();
-      reinterpret_cast<uint32_t *>(smem)[2] = 0u;
-      reinterpret_cast<uint32_t *>(smem)[3] = kRelMax;  // packed levels: weight 0
+  // Staging by bulk copies: the tables that no epoch changes and every ant's
+  // elements on the first barrier, before this launch waits for the kernel
+  // that makes the weights; the weights on the second one.
+  constexpr bool kFixed = L != kLayoutGlobal || E > 0, kWeights = L != kLayoutGlobal;
+  const uint32_t kChunk = 32768u;
+  auto issue = [&](unsigned char *dst, const void *src, uint32_t bytes, uint64_t *on) {
+    const unsigned char *sp = reinterpret_cast<const unsigned char *>(src);
+    for (uint32_t o = 0; o < bytes; o += kChunk) {
+      const uint32_t b = bytes - o < kChunk ? bytes - o : kChunk;
+      bulk_g2s(dst + o, sp + o, b, on);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const uint32_t ants = blockDim.x >> 5;
-      const uint32_t total = pl.bytes_cand + pl.bytes_w + pl.bytes_coords +
-                             (E > 0 ? ants * pl.vis_bytes : 0u);
-      mbar_arrive_expect_tx(bar, total + (uint32_t)iv.stage_extra_tx);
-      const uint32_t kChunk = 32768u;
-      auto issue = [&](unsigned char *dst, const void *src, uint32_t bytes) {
-        const unsigned char *sp = reinterpret_cast<const unsigned char *>(src);
-        for (uint32_t o = 0; o < bytes; o += kChunk) {
-          const uint32_t b = bytes - o < kChunk ? bytes - o : kChunk;
-          bulk_g2s(dst + o, sp + o, b, bar);
-        }
-      };
-      if (E > 0)
-        for (uint32_t i = 0; i < ants; ++i)
-          issue(smem + pl.off_vis + i * pl.vis_bytes, iv.elems, pl.vis_bytes);
-      if (L != kLayoutGlobal) {
-        issue(smem + pl.off_cand, iv.cand, pl.bytes_cand);
-        if (L == kLayoutSmemPacked) issue(smem + pl.off_w, a.et.rel, pl.bytes_w);
-        else issue(smem + pl.off_w, a.et.w, pl.bytes_w);
-        issue(smem + pl.off_coords, iv.coords, pl.bytes_coords);
-      }
+  };
+  if (kFixed && threadIdx.x == 0) {
+    mbar_init(bar, 1);
+    mbar_init(bar + 1, 1);
+    fence_mbar_init();
+    reinterpret_cast<uint32_t *>(smem)[4] = 0u;
+    reinterpret_cast<uint32_t *>(smem)[5] = kRelMax;  // packed levels: weight 0
+    const uint32_t ants = blockDim.x >> 5;
+    mbar_arrive_expect_tx(bar, pl.bytes_cand + pl.bytes_coords + (E > 0 ? ants * pl.vis_bytes : 0u) +
+                                   (uint32_t)iv.stage_extra_tx);
+    if (E > 0)
+      for (uint32_t i = 0; i < ants; ++i)
+        issue(smem + pl.off_vis + i * pl.vis_bytes, iv.elems, pl.vis_bytes, bar);
+    if (L != kLayoutGlobal) {
+      issue(smem + pl.off_cand, iv.cand, pl.bytes_cand, bar);
+      issue(smem + pl.off_coords, iv.coords, pl.bytes_coords, bar);
     }
   }
 
@@ -899,7 +886,24 @@ __global__ void __launch_bounds__(512, 1) k_construct(const __grid_constant__ Co
   us.dem = iv.demand;
   if (E == 0) us.init_bits(iv.n, lane);
 
-  if (kStage) {
+  wait_for_previous();
+  // Graph replays read the epoch number and the seed from the device state,
+  // so one captured graph serves every solve of a context.
+  uint32_t epoch = a.epoch, seed = a.seed;
+  int skip = 0;
+  if (a.st) {
+    skip = *(volatile int *)&a.st->skip;
+    if (a.use_state_epoch) {  // requested with the flag: one round trip
+      epoch = *(volatile uint32_t *)&a.st->epoch;
+      seed = *(volatile uint32_t *)&a.st->seed;
+    }
+  }
+  if (kWeights && threadIdx.x == 0) {
+    mbar_arrive_expect_tx(bar + 1, pl.bytes_w);
+    issue(smem + pl.off_w, L == kLayoutSmemPacked ? (const void *)a.et.rel : (const void *)a.et.w,
+          pl.bytes_w, bar + 1);
+  }
+  if (kFixed) {
     // Bounded wait for the staged tables.  The decision is the block's: it
     // goes on only when every thread saw the tables arrive, so no warp
     // enters the full-mask collectives of build_ant with lanes or warps
@@ -908,20 +912,26 @@ __global__ void __launch_bounds__(512, 1) k_construct(const __grid_constant__ Co
     // expects stage_extra_tx bytes that no copy brings; thread 0 marks them
     // arrived, so that second wait ends once the real copies have landed.
     // After a genuine time-out the second wait may run out as well; the
-    // block then exits with the error flag set.
+    // block then exits with the error flag set.  A skipped epoch waits too:
+    // the copies have to land before the block leaves.
+    __syncthreads();  // the barriers are initialised
     const uint32_t limit = iv.stage_extra_tx ? (1u << 14) : (1u << 22);
-    const bool ok = __syncthreads_and(mbar_wait_bounded(bar, 0, limit) ? 1 : 0) != 0;
+    bool here = mbar_wait_bounded(bar, 0, limit);
+    if (kWeights) here = mbar_wait_bounded(bar + 1, 0, limit) && here;
+    const bool ok = __syncthreads_and(here ? 1 : 0) != 0;
     if (!ok) {
       if (threadIdx.x == 0) {
-        if (a.st) atomicOr(&a.st->error, kErrStageTimeout);
+        if (a.st && !skip) atomicOr(&a.st->error, kErrStageTimeout);
         if (iv.stage_extra_tx) mbar_complete_tx(bar, (uint32_t)iv.stage_extra_tx);
       }
       __syncthreads();
       mbar_wait_bounded(bar, 0, limit << 2);
+      if (kWeights) mbar_wait_bounded(bar + 1, 0, limit << 2);
       __syncthreads();
       return;
     }
   }
+  if (skip) return;
 
   const int ant = blockIdx.x * pl.wpb + warp;
   if (ant >= iv.m) return;
@@ -958,7 +968,7 @@ SmemPlan plan_construct(const InstanceView &iv, int layout, int num_sms,
     p.elem = el;
     p.wpb = ants;
     p.vis_bytes = unserved_bytes(iv.n, el);
-    uint32_t off = 16;  // mbarrier, zero entry
+    uint32_t off = 32;  // two barriers, zero entry
     if (lay == kLayoutGlobal) {
       p.bytes_cand = p.bytes_w = p.bytes_coords = 0;
       p.off_cand = p.off_w = p.off_coords = p.off_lut = off;
@@ -1041,11 +1051,9 @@ static cudaError_t launch_construct_le(const ConstructArgs &a, cudaStream_t s) {
   const int threads = a.plan.wpb * 32;
   if (a.iv.depot_rule == kDepotRuleCudaRef) {
     if (!a.et.rdep) return cudaErrorInvalidValue;
-    k_construct<L, E, true><<<grid, threads, a.plan.total, s>>>(a);
-  } else {
-    k_construct<L, E, false><<<grid, threads, a.plan.total, s>>>(a);
+    return launch_after(k_construct<L, E, true>, grid, threads, a.plan.total, s, a);
   }
-  return cudaGetLastError();
+  return launch_after(k_construct<L, E, false>, grid, threads, a.plan.total, s, a);
 }
 
 template <int L>
@@ -1262,6 +1270,53 @@ __global__ void __launch_bounds__(1024) k_best(InstanceView iv, AntBuffers ab,
 constexpr int kBestCluster = 8;
 constexpr int kBestThreads = 256;
 
+// Deposit of a complete solution (n + 2K entries) over gthreads threads, this
+// one gtid: one arc (p, q) of consecutive entries per thread, both cells
+// loaded together; the arcs of different customers' pairs touch different
+// cells, but the two arcs of a one-customer route [0 p 0] share theirs and go
+// to one thread in order.  (0, 0) pairs are route boundaries and empty
+// routes; the empty routes' own cell (0, 0) is raised once per empty route by
+// the thread with gtid 0's warp.
+__device__ __forceinline__ void deposit_pair(const PheromoneView &pv, size_t stride, int u, int c,
+                                             float dep) {
+  uint8_t *fwd = pv.tau + (size_t)u * stride + c, *rev = pv.tau + (size_t)c * stride + u;
+  const uint8_t old = ld_cg_u8(fwd), oldr = ld_cg_u8(rev);
+  const uint8_t nq = quant(dequant(old, pv.log_min, pv.log_step) + dep, pv.log_min, pv.log_step,
+                           pv.q_min, pv.q_max);
+  if (nq > old) st_cg_u8(fwd, nq);
+  if (nq > oldr) st_cg_u8(rev, nq);
+}
+
+__device__ __forceinline__ void deposit_complete(const PheromoneView &pv, size_t stride,
+                                                 const int *nodes, const int *lens, int n, int K,
+                                                 float dep, int gtid, int gthreads) {
+  const int total = n + 2 * K;
+  for (int j = 1 + gtid; j < total; j += gthreads) {
+    const int p = nodes[j - 1], q = nodes[j];
+    const int before = j >= 2 ? nodes[j - 2] : 0, after = j + 1 < total ? nodes[j + 1] : 0;
+    if (p == 0 && q == 0) continue;
+    if (q == 0 && before == 0) continue;  // second arc of [0 p 0]
+    deposit_pair(pv, stride, p, q, dep);
+    if (p == 0 && after == 0) deposit_pair(pv, stride, q, 0, dep);
+  }
+  if (gtid < 32) {
+    int empty = 0;
+    for (int b = 0; b < K; b += 32)
+      empty += __popc(__ballot_sync(kFull, b + gtid < K && lens[b + gtid] == 2));
+    if (gtid == 0 && empty > 0) {
+      const uint8_t old = ld_cg_u8(pv.tau);
+      uint8_t q = old;
+      for (int i = 0; i < empty; ++i) {
+        const uint8_t nq = quant(dequant(q, pv.log_min, pv.log_step) + dep, pv.log_min,
+                                 pv.log_step, pv.q_min, pv.q_max);
+        if (nq <= q) break;  // and so would every further one be
+        q = nq;
+      }
+      if (q > old) st_cg_u8(pv.tau, q);
+    }
+  }
+}
+
 // The epoch's two deposits over the cluster, into the buffer evaporated
 // beside the construction: the iteration best, a cluster barrier (its stores
 // before the next deposit's loads, release / acquire at cluster scope), the
@@ -1276,14 +1331,10 @@ __device__ __forceinline__ void cluster_deposits(cooperative_groups::cluster_gro
   PheromoneView pd = pv;
   pd.tau = sel ? pv.tau : tau_alt;  // the evaporated copy
   const size_t stride_n = (size_t)iv.n + 1;
-  extern __shared__ int s_off[];
-  int *offs = (iv.K <= kDepositSmemRoutes) ? s_off : nullptr;
   const int gt = rank * kBestThreads + (int)threadIdx.x, gn = kBestCluster * kBestThreads;
-  deposit_solution(pd, stride_n, CompactNodes{it_nodes}, it_lens, iv.K, s_st->dep_iter, offs, gt,
-                   gn);
+  deposit_complete(pd, stride_n, it_nodes, it_lens, iv.n, iv.K, s_st->dep_iter, gt, gn);
   cluster.sync();
-  deposit_solution(pd, stride_n, CompactNodes{gb_nodes}, gb_lens, iv.K, s_st->dep_global, offs,
-                   gt, gn);
+  deposit_complete(pd, stride_n, gb_nodes, gb_lens, iv.n, iv.K, s_st->dep_global, gt, gn);
   if (rank == 0) {
     __syncthreads();
     if (threadIdx.x == 0) s_st->tau_sel = sel ? 0 : 1;
@@ -1303,6 +1354,7 @@ __global__ void __cluster_dims__(kBestCluster, 1, 1) __launch_bounds__(kBestThre
   __shared__ int s_ant[kBestThreads / 32];
   __shared__ unsigned long long s_steps[kBestThreads / 32];
   __shared__ int s_improved, s_best;
+  let_next_start();
   state_load(&s_st, st);
   double bc;
   int ba;
@@ -1352,9 +1404,8 @@ cudaError_t launch_best_deposit(const InstanceView &iv, const AntBuffers &ab,
                                 const PheromoneView &pv, uint8_t *tau_alt, DevState *st,
                                 int *gbest_nodes, int *gbest_lens, EpochRec *log,
                                 cudaStream_t s) {
-  const size_t smem = iv.K <= kDepositSmemRoutes ? sizeof(int) * (iv.K + 1) : 0;
-  k_best_cluster<<<kBestCluster, kBestThreads, smem, s>>>(iv, ab, st, gbest_nodes, gbest_lens,
-                                                          log, pv, tau_alt);
+  k_best_cluster<<<kBestCluster, kBestThreads, 0, s>>>(iv, ab, st, gbest_nodes, gbest_lens, log,
+                                                       pv, tau_alt);
   return cudaGetLastError();
 }
 
@@ -1634,8 +1685,7 @@ cudaError_t launch_shard_select(const InstanceView &iv, DevState *st, const int 
                                 int world, int *iter_nodes, int *iter_lens,
                                 int *gbest_nodes, int *gbest_lens, EpochRec *log,
                                 const PheromoneView &pv, uint8_t *tau_alt, cudaStream_t s) {
-  const size_t smem = iv.K <= kDepositSmemRoutes ? sizeof(int) * (iv.K + 1) : 0;
-  k_shard_select<<<kBestCluster, kBestThreads, smem, s>>>(iv, st, recv, world, iter_nodes,
+  k_shard_select<<<kBestCluster, kBestThreads, 0, s>>>(iv, st, recv, world, iter_nodes,
                                                           iter_lens, gbest_nodes, gbest_lens,
                                                           log, pv, tau_alt);
   return cudaGetLastError();

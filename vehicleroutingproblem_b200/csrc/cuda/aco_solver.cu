@@ -234,7 +234,8 @@ static int build_graph(aco_b200_ctx *ctx, int epochs, cudaGraphExec_t *out) {
   cudaError_t err = cudaSuccess;
   // One epoch: weights, then the construction and (on the side stream) the
   // evaporation into the other pheromone buffer, then iteration best, global
-  // best, stop rules and the deposits, which switch the buffers.
+  // best, stop rules and the deposits, which switch the buffers.  The weights
+  // and the construction start while the launch before them ends.
   for (int e = 0; e < epochs && err == cudaSuccess; ++e) {
     err = launch_weights(ctx->iv, ctx->pv, ctx->et, ctx->d_state, ctx->stream);
     if (err == cudaSuccess) err = cudaEventRecord(ctx->ev_fork, ctx->stream);
