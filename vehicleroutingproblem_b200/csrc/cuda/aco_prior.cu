@@ -15,7 +15,7 @@
 //             + backward for training
 //   loss      softmax cross-entropy over each row's valid slots against the
 //             successor taken by an elite route
-//   optimiser Adam (k_prior_adam)
+//   optimiser Adam (k_prior_reduce)
 //
 // Layer 1 carries its bias as the weight of a constant-one input (input 8
 // of the 16-wide K of the first MMA), so one GEMM
@@ -52,6 +52,15 @@ static_assert(kParams == ACO_B200_PRIOR_PARAMS, "parameter count");
 constexpr int kSlots = 32;      // candidate slots per row (k <= 32); a tile is 4 rows
 constexpr uint32_t kPolls = 1u << 24;
 
+// K-chunk distance of the two transposed operand tiles, 16 bytes more than
+// the packed layout's: a warp's 32 edges are 4 chunks of a row, and with the
+// packed distances (multiples of 128 bytes) their stores met in the same
+// banks.
+constexpr uint32_t kLboA = 128 / 8 * 128 + 16, kLboB = 80 / 8 * 128 + 16;
+__device__ __forceinline__ uint32_t edge_offset(int row, int edge, uint32_t lbo) {
+  return (uint32_t)(edge >> 3) * lbo + (uint32_t)((row >> 3) * 128 + (row & 7) * 16 + (edge & 7) * 2);
+}
+
 // Shared-memory layout of k_prior_mlp (bytes, K-major operand tiles).
 constexpr uint32_t kSB1 = 0;                         // W1|b1   64 x 16
 constexpr uint32_t kSB2 = kSB1 + 64 * 16 * 2;         // W2      64 x 64 [o][j]
@@ -59,8 +68,8 @@ constexpr uint32_t kSB2T = kSB2 + 64 * 64 * 2;        // W2^T    64 x 64 [j][o]
 constexpr uint32_t kSA1 = kSB2T + 64 * 64 * 2;        // X       128 x 16
 constexpr uint32_t kSA2 = kSA1 + 128 * 16 * 2;        // H1, then dZ2  128 x 64
 constexpr uint32_t kSAdw = kSA2 + 128 * 64 * 2;       // [dZ2^T; dZ1^T] 128 x 128
-constexpr uint32_t kSBdw = kSAdw + 128 * 128 * 2;     // [H1^T; X^T]   80 x 128
-constexpr uint32_t kSF32 = kSBdw + 80 * 128 * 2;      // b2[64], w3[64]
+constexpr uint32_t kSBdw = kSAdw + 16 * kLboA;        // [H1^T; X^T]   80 x 128
+constexpr uint32_t kSF32 = kSBdw + 16 * kLboB;        // b2[64], w3[64]
 constexpr uint32_t kSRed = kSF32 + 128 * 4;           // 4 warps x 65 partial sums
 constexpr uint32_t kSBar = kSRed + 4 * 65 * 4 + 48;    // mbarrier, TMEM base
 constexpr uint32_t kSmemTrain = kSBar + 64;
@@ -222,6 +231,37 @@ struct MlpArgs {
   int *error;
 };
 
+// The feature row of one warp's edges in a tile (beyond the last tile or
+// example: row 0, not live) and, in training, its target slot.
+struct RowRef {
+  long long row;
+  int tgt;
+  bool live;
+};
+
+template <bool TRAIN>
+__device__ __forceinline__ RowRef row_ref(const MlpArgs &a, int tile, int warp) {
+  RowRef r;
+  if (TRAIN) {
+    const int ex = tile * 4 + warp;
+    r.live = ex < a.count;
+    const int2 e2 = r.live ? a.examples[a.order[ex]] : make_int2(0, -1);
+    r.row = e2.x;
+    r.tgt = e2.y;
+  } else {
+    r.row = (long long)tile * 4 + warp;
+    r.live = r.row < a.rows;
+    if (!r.live) r.row = 0;
+    r.tgt = -1;
+  }
+  return r;
+}
+
+__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
+  return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(lo)) |
+         ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi)) << 16);
+}
+
 template <bool TRAIN>
 __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -234,6 +274,7 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr uint32_t kCols = TRAIN ? 256u : 128u;
 
+  let_next_start();
   if (warp == 0) {
     umma::tmem_alloc(s_tmem, kCols);
     umma::tmem_relinquish();
@@ -242,33 +283,56 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
     mbar_init(bar, 1);
     fence_mbar_init();
   }
-  // Weights into their operand layouts (BF16), biases of layers 2-3 in FP32.
-  const float *P = a.params;
-  for (int e = tid; e < 64 * 16; e += 128) {
-    const int o = e >> 4, f = e & 15;
-    const float w = f < 8 ? P[kW1 + o * 8 + f] : (f == 8 ? P[kB1 + o] : 0.f);
-    st_bf16(sB1, umma::kmajor_offset(o, f, 64), w);
-  }
-  for (int e = tid; e < 64 * 64; e += 128) {
-    const int o = e >> 6, j = e & 63;
-    const float w = P[kW2 + e];
-    st_bf16(sB2, umma::kmajor_offset(o, j, 64), w);
-    if (TRAIN) st_bf16(sB2T, umma::kmajor_offset(j, o, 64), w);
-  }
-  if (tid < 64) {
-    s_b2[tid] = P[kB2 + tid];
-    s_w3[tid] = P[kW3 + tid];
-  }
-  const float b3 = P[kB3];
   // Constant input 8 = 1 (layer-1 bias), inputs 9-15 = 0, for every edge.
   *reinterpret_cast<uint4 *>(sA1 + umma::kmajor_offset(tid, 8, 128)) =
       make_uint4(0x3F80u, 0u, 0u, 0u);
   if (TRAIN) {
     for (int e = tid; e < 8 * 128; e += 128) {
       const int f = 8 + (e >> 7), col = e & 127;
-      st_bf16(sBdw, umma::kmajor_offset(64 + f, col, 80), f == 8 ? 1.f : 0.f);
+      st_bf16(sBdw, edge_offset(64 + f, col, kLboB), f == 8 ? 1.f : 0.f);
     }
   }
+  // The first tile's rows: features and examples are fixed, so they are on
+  // their way before this launch waits for the parameters' update.
+  int tile = blockIdx.x;
+  RowRef now = row_ref<TRAIN>(a, tile, warp), next = row_ref<TRAIN>(a, tile + gridDim.x, warp);
+  int kvr = now.live ? (int)a.kv[now.row] : 0;
+  uint4 fv = a.feat[now.row * kSlots + lane];
+  wait_for_previous();
+  // Weights into their operand layouts (BF16), 8 along K at a time (16-byte
+  // stores); biases of layers 2-3 in FP32.
+  const float *P = a.params;
+  for (int e = tid; e < 64 * 16; e += 128) {
+    const int o = e >> 4, f = e & 15;
+    const float w = f < 8 ? P[kW1 + o * 8 + f] : (f == 8 ? P[kB1 + o] : 0.f);
+    st_bf16(sB1, umma::kmajor_offset(o, f, 64), w);
+  }
+#pragma unroll
+  for (int e = tid; e < 64 * 8; e += 128) {
+    const int o = e >> 3, j = (e & 7) * 8;
+    const float4 lo = *reinterpret_cast<const float4 *>(P + kW2 + o * 64 + j);
+    const float4 hi = *reinterpret_cast<const float4 *>(P + kW2 + o * 64 + j + 4);
+    *reinterpret_cast<uint4 *>(sB2 + umma::kmajor_offset(o, j, 64)) =
+        make_uint4(bf16_pair(lo.x, lo.y), bf16_pair(lo.z, lo.w), bf16_pair(hi.x, hi.y),
+                   bf16_pair(hi.z, hi.w));
+  }
+  if (TRAIN) {
+#pragma unroll
+    for (int e = tid; e < 64 * 8; e += 128) {
+      const int j = e & 63, o = (e >> 6) * 8;  // row j of W2^T, elements o .. o + 7
+      float w[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) w[i] = P[kW2 + (o + i) * 64 + j];
+      *reinterpret_cast<uint4 *>(sB2T + umma::kmajor_offset(j, o, 64)) =
+          make_uint4(bf16_pair(w[0], w[1]), bf16_pair(w[2], w[3]), bf16_pair(w[4], w[5]),
+                     bf16_pair(w[6], w[7]));
+    }
+  }
+  if (tid < 64) {
+    s_b2[tid] = P[kB2 + tid];
+    s_w3[tid] = P[kW3 + tid];
+  }
+  const float b3 = P[kB3];
   umma::fence_async_smem();
   umma::fence_before_sync();
   __syncthreads();
@@ -276,8 +340,7 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
   const uint32_t tm = *s_tmem;
   const uint32_t tl = tm + ((uint32_t)(warp * 32) << 16);  // this warp's lanes
 
-  const uint32_t lbo128 = umma::kmajor_lbo(128), lbo64 = umma::kmajor_lbo(64),
-                 lbo80 = umma::kmajor_lbo(80);
+  const uint32_t lbo128 = umma::kmajor_lbo(128), lbo64 = umma::kmajor_lbo(64);
   const uint32_t idesc64 = umma::idesc_bf16_f32(128, 64);
   const uint32_t idesc80 = umma::idesc_bf16_f32(128, 80);
   const uint32_t aA1 = umma::smem_u32(sA1), aA2 = umma::smem_u32(sA2),
@@ -293,30 +356,24 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
   bool ok = true;
   int done = 0;
 
-  for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
-    long long row;
-    int tgt = -1;
-    bool live;
-    if (TRAIN) {
-      const int ex = tile * 4 + warp;
-      live = ex < a.count;
-      const int2 e2 = live ? a.examples[a.order[ex]] : make_int2(0, -1);
-      row = e2.x;
-      tgt = e2.y;
-    } else {
-      row = (long long)tile * 4 + warp;
-      live = row < a.rows;
-    }
-    const int kvr = live ? (int)a.kv[row] : 0;
-    const bool valid = live && lane < kvr;
-    const uint4 fv = valid ? a.feat[row * kSlots + lane] : make_uint4(0u, 0u, 0u, 0u);
+  for (; tile < a.tiles; tile += gridDim.x) {
+    const bool live = now.live, valid = live && lane < kvr;
+    const long long row = now.row;
+    const int tgt = now.tgt;
+    if (!valid) fv = make_uint4(0u, 0u, 0u, 0u);
     *reinterpret_cast<uint4 *>(sA1 + umma::kmajor_offset(tid, 0, 128)) = fv;
     if (TRAIN) {
       const __nv_bfloat16 *fb = reinterpret_cast<const __nv_bfloat16 *>(&fv);
 #pragma unroll
       for (int f = 0; f < 8; ++f)
-        *reinterpret_cast<__nv_bfloat16 *>(sBdw + umma::kmajor_offset(64 + f, tid, 80)) = fb[f];
+        *reinterpret_cast<__nv_bfloat16 *>(sBdw + edge_offset(64 + f, tid, kLboB)) = fb[f];
     }
+    // The next tile's rows while this one is worked on, and where the rows
+    // after those are.
+    now = next;
+    kvr = now.live ? (int)a.kv[now.row] : 0;
+    fv = a.feat[now.row * kSlots + lane];
+    next = row_ref<TRAIN>(a, tile + 2 * gridDim.x, warp);
     umma::fence_async_smem();
     umma::fence_before_sync();
     __syncthreads();
@@ -344,8 +401,8 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
         const __nv_bfloat16 hi = __float2bfloat16_rn(fmaxf(z[2 * i + 1], 0.f));
         w[i] = (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
         if (TRAIN) {
-          *reinterpret_cast<__nv_bfloat16 *>(sBdw + umma::kmajor_offset(16 * q + 2 * i, tid, 80)) = lo;
-          *reinterpret_cast<__nv_bfloat16 *>(sBdw + umma::kmajor_offset(16 * q + 2 * i + 1, tid, 80)) = hi;
+          *reinterpret_cast<__nv_bfloat16 *>(sBdw + edge_offset(16 * q + 2 * i, tid, kLboB)) = lo;
+          *reinterpret_cast<__nv_bfloat16 *>(sBdw + edge_offset(16 * q + 2 * i + 1, tid, kLboB)) = hi;
         }
       }
       *reinterpret_cast<uint4 *>(sA2 + umma::kmajor_offset(tid, 16 * q, 128)) =
@@ -412,8 +469,8 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
           const __nv_bfloat16 lo = __float2bfloat16_rn(d2[0]);
           const __nv_bfloat16 hi = __float2bfloat16_rn(d2[1]);
           w[i] = (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
-          *reinterpret_cast<__nv_bfloat16 *>(sAdw + umma::kmajor_offset(16 * q + 2 * i, tid, 128)) = lo;
-          *reinterpret_cast<__nv_bfloat16 *>(sAdw + umma::kmajor_offset(16 * q + 2 * i + 1, tid, 128)) = hi;
+          *reinterpret_cast<__nv_bfloat16 *>(sAdw + edge_offset(16 * q + 2 * i, tid, kLboA)) = lo;
+          *reinterpret_cast<__nv_bfloat16 *>(sAdw + edge_offset(16 * q + 2 * i + 1, tid, kLboA)) = hi;
         }
         *reinterpret_cast<uint4 *>(sA2 + umma::kmajor_offset(tid, 16 * q, 128)) =
             make_uint4(w[0], w[1], w[2], w[3]);
@@ -446,7 +503,7 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
         umma::tmem_wait_ld();
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          st_bf16(sAdw, umma::kmajor_offset(64 + 16 * q + i, tid, 128), z[i] > 0.f ? dh[i] : 0.f);
+          st_bf16(sAdw, edge_offset(64 + 16 * q + i, tid, kLboA), z[i] > 0.f ? dh[i] : 0.f);
       }
       umma::fence_async_smem();
       umma::fence_before_sync();
@@ -456,8 +513,8 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
         umma::fence_after_sync();
 #pragma unroll
         for (int s = 0; s < 8; ++s)
-          umma::mma_bf16(tm + kColDW, umma::smem_desc(aAdw + 2 * s * lbo128, lbo128, 128),
-                         umma::smem_desc(aBdw + 2 * s * lbo80, lbo80, 128), idesc80,
+          umma::mma_bf16(tm + kColDW, umma::smem_desc(aAdw + 2 * s * kLboA, kLboA, 128),
+                         umma::smem_desc(aBdw + 2 * s * kLboB, kLboB, 128), idesc80,
                          (done > 0 || s > 0) ? 1u : 0u);
         umma::commit(bar);
       }
@@ -486,26 +543,43 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
       float d[16];
       umma::tmem_ld16(tl + kColDW + 16 * q, d);
       umma::tmem_wait_ld();
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int col = 16 * q + i;
+      if (q < 4) {
         if (warp < 2) {
-          if (col < 64) out[kW2 + tid * 64 + col] = d[i];
-          else if (col == 72) out[kB2 + tid] = d[i];
-        } else {
-          const int j = tid - 64;
-          if (col >= 64 && col < 72) out[kW1 + j * 8 + (col - 64)] = d[i];
-          else if (col == 72) out[kB1 + j] = d[i];
+          float4 *o4 = reinterpret_cast<float4 *>(out + kW2 + tid * 64 + 16 * q);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            o4[i] = make_float4(d[4 * i], d[4 * i + 1], d[4 * i + 2], d[4 * i + 3]);
         }
+      } else if (warp < 2) {
+        out[kB2 + tid] = d[8];
+      } else {
+        float4 *o4 = reinterpret_cast<float4 *>(out + kW1 + (tid - 64) * 8);
+        o4[0] = make_float4(d[0], d[1], d[2], d[3]);
+        o4[1] = make_float4(d[4], d[5], d[6], d[7]);
+        out[kB1 + tid - 64] = d[8];
       }
     }
-    // w3 and the loss: warp sums, then the four warps in order.
+    // w3 and the loss: warp sums, then the four warps in order.  The 64 sums
+    // by halving: at each step a lane keeps half of its values and adds the
+    // partner's (the sums of a butterfly over all 32 lanes, with 62 shuffles
+    // instead of 320); lane L ends with values 2 rev(L) and 2 rev(L) + 1.
     float *s_red = reinterpret_cast<float *>(smem + kSRed);
+    int at = 0;
 #pragma unroll
-    for (int j = 0; j < 64; ++j) {
-      const float v = warp_sum(acc_w3[j]);
-      if (lane == 0) s_red[warp * 65 + j] = v;
+    for (int o = 16, half = 32; o > 0; o >>= 1, half >>= 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        if (j < half) {
+          const float keep = up ? acc_w3[j + half] : acc_w3[j];
+          const float give = up ? acc_w3[j] : acc_w3[j + half];
+          acc_w3[j] = keep + __shfl_xor_sync(kFull, give, o);
+        }
+      }
+      at += up ? half : 0;
     }
+    s_red[warp * 65 + at] = acc_w3[0];
+    s_red[warp * 65 + at + 1] = acc_w3[1];
     const float vl = warp_sum(acc_loss);
     if (lane == 0) s_red[warp * 65 + 64] = vl;
     __syncthreads();
@@ -523,22 +597,40 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
   if (warp == 0) umma::tmem_dealloc(tm, kCols);
 }
 
-// Sum of the blocks' partial gradients in block order; the loss goes to
-// *loss (accumulated over a training epoch).
-__global__ void k_prior_reduce(const float *gpart, int blocks, float *grad, float *loss) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > kParams) return;
-  float v = 0.f;
-  for (int r = 0; r < blocks; ++r) v += gpart[(size_t)r * kGradStride + i];
-  if (i < kParams) grad[i] = v;
-  else *loss += v;
-}
+// Sum of the blocks' partial gradients in block order, into grad or (params
+// given) taken as Adam's step; the loss goes to *loss.  A block takes 32
+// parameters: all its threads bring the rows' values to shared memory at once,
+// one warp adds them in order, so that training stays bit-reproducible.  (One
+// thread per parameter loading row after row, and the step in a launch of its
+// own, took 15 + 4 us behind every 48 us of gradients.)
+constexpr int kReduceThreads = 256;
 
-__global__ void k_prior_adam(float *params, float *m, float *v, float *grad, int count, float lr,
-                             float bc1, float bc2) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const float g = grad[i];
+__global__ void __launch_bounds__(kReduceThreads)
+    k_prior_reduce(const float *gpart, int blocks, float *grad, float *loss, float *params,
+                   float *m, float *v, float lr, float bc1, float bc2) {
+  extern __shared__ float s_part[];  // [blocks][32]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  let_next_start();
+  wait_for_previous();
+  if (i <= kParams) {
+#pragma unroll 16
+    for (int r = warp; r < blocks; r += kReduceThreads / 32)
+      s_part[r * 32 + lane] = gpart[(size_t)r * kGradStride + i];
+  }
+  __syncthreads();
+  if (warp != 0 || i > kParams) return;
+  float g = 0.f;
+#pragma unroll 16
+  for (int r = 0; r < blocks; ++r) g += s_part[r * 32 + lane];
+  if (i == kParams) {
+    *loss += g;
+    return;
+  }
+  if (!params) {
+    grad[i] = g;
+    return;
+  }
   const float mi = 0.9f * m[i] + 0.1f * g;
   const float vi = 0.999f * v[i] + 0.001f * g * g;
   m[i] = mi;
@@ -971,8 +1063,11 @@ int aco_b200_prior_set_dataset(aco_b200_prior *p, const aco_b200_prior_dataset *
 
 // Gradient of the mean loss over `count` examples listed at order: the
 // tensor-core kernel writes one partial row per block, k_prior_reduce sums
-// them into d_grad in block order and adds the loss to *d_loss.
-static int run_gradient(aco_b200_prior *p, const int *order, int count, cudaStream_t s) {
+// them and adds the loss to *d_loss; step > 0: Adam's step number `step` on
+// the parameters, else the gradient into d_grad.  first: the launch follows
+// copies (the examples' order), which it must not overtake.
+static int run_gradient(aco_b200_prior *p, const int *order, int count, int step, float lr,
+                        bool first, cudaStream_t s) {
   MlpArgs a = {};
   a.params = p->d_params;
   a.feat = p->d_feat;
@@ -984,13 +1079,19 @@ static int run_gradient(aco_b200_prior *p, const int *order, int count, cudaStre
   a.gpart = p->d_gpart;
   a.error = p->d_error;
   a.tiles = (count + 3) / 4;
-  // Two training blocks per SM (256 tensor-memory columns and 94 KB of shared
+  // Two training blocks per SM (256 tensor-memory columns and 95 KB of shared
   // memory each): one block's MMA runs while the other's epilogue does.
   const int grid = std::max(1, std::min(a.tiles, p->num_sms * 2));
-  k_prior_mlp<true><<<grid, 128, kSmemTrain, s>>>(a);
-  PTRY(cudaGetLastError());
-  k_prior_reduce<<<(kParams + 1 + 255) / 256, 256, 0, s>>>(p->d_gpart, grid, p->d_grad, p->d_loss);
-  PTRY(cudaGetLastError());
+  if (first) {
+    k_prior_mlp<true><<<grid, 128, kSmemTrain, s>>>(a);
+    PTRY(cudaGetLastError());
+  } else {
+    PTRY(launch_after(k_prior_mlp<true>, grid, 128, kSmemTrain, s, a));
+  }
+  const float bc1 = 1.0f - powf(0.9f, (float)step), bc2 = 1.0f - powf(0.999f, (float)step);
+  PTRY(launch_after(k_prior_reduce, (kParams + 1 + 31) / 32, kReduceThreads,
+                    (size_t)grid * 32 * sizeof(float), s, (const float *)p->d_gpart, grid, p->d_grad, p->d_loss,
+                    step > 0 ? p->d_params : nullptr, p->d_m, p->d_v, lr, bc1, bc2));
   return ACO_OK;
 }
 
@@ -1014,7 +1115,7 @@ int aco_b200_prior_gradient(aco_b200_prior *p, const int *examples, int count, f
   cudaStream_t s = p->stream;
   PTRY(cudaMemcpyAsync(p->d_order, examples, count * sizeof(int), cudaMemcpyHostToDevice, s));
   PTRY(cudaMemsetAsync(p->d_loss, 0, sizeof(float), s));
-  int rc = run_gradient(p, p->d_order, count, s);
+  int rc = run_gradient(p, p->d_order, count, 0, 0.f, true, s);
   if (rc) return rc;
   PTRY(cudaStreamSynchronize(s));
   rc = check_error(p);
@@ -1044,14 +1145,9 @@ int aco_b200_prior_train(aco_b200_prior *p, int epochs, int batch, float lr, uns
     int steps = 0;
     for (long long b0 = 0; b0 < N; b0 += batch, ++steps) {
       const int cnt = (int)std::min<long long>(batch, N - b0);
-      int rc = run_gradient(p, p->d_order + b0, cnt, s);
-      if (rc) return rc;
       p->adam_step += 1;
-      const float bc1 = 1.0f - powf(0.9f, (float)p->adam_step);
-      const float bc2 = 1.0f - powf(0.999f, (float)p->adam_step);
-      k_prior_adam<<<(kParams + 255) / 256, 256, 0, s>>>(p->d_params, p->d_m, p->d_v, p->d_grad,
-                                                         kParams, lr, bc1, bc2);
-      PTRY(cudaGetLastError());
+      int rc = run_gradient(p, p->d_order + b0, cnt, p->adam_step, lr, b0 == 0, s);
+      if (rc) return rc;
     }
     float l = 0.f;
     PTRY(cudaMemcpyAsync(&l, p->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s));
