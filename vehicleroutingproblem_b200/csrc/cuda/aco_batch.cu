@@ -1218,8 +1218,7 @@ int aco_b200_batch_setup(aco_b200_batch *b, const aco_b200_batch_problem *p) {
   BTRY(cudaMemcpyAsync(d_soff, seg_off.data(), sizeof(long long) * count, cudaMemcpyHostToDevice, s));
   BTRY(cudaMemcpyAsync(d_sn, seg_n.data(), sizeof(int) * count, cudaMemcpyHostToDevice, s));
   BTRY(launch_knn_levels_multi(d_coords, d_soff, d_sn, count, node, k, d_thr, kThresholds, d_cand,
-                               d_lvl, s));
-  BTRY(launch_knn_tier_multi(d_coords, d_soff, d_sn, count, node, k, d_tier, s));
+                               d_lvl, d_tier, s));
   b->d_seg_off = d_soff;
   b->d_seg_n = d_sn;
   b->rows = node;
@@ -1375,9 +1374,8 @@ int aco_b200_batch_set_cand_k(aco_b200_batch *b, int k) {
   BatchArgs &a = b->args;
   BTRY(launch_knn_levels_multi(a.coords, b->d_seg_off, b->d_seg_n, b->count, b->rows, k,
                                b->d_thr, kThresholds, const_cast<uint16_t *>(a.cand),
-                               const_cast<uint16_t *>(a.lvl), b->stream));
-  BTRY(launch_knn_tier_multi(a.coords, b->d_seg_off, b->d_seg_n, b->count, b->rows, k,
-                             const_cast<uint16_t *>(a.tier), b->stream));
+                               const_cast<uint16_t *>(a.lvl), const_cast<uint16_t *>(a.tier),
+                               b->stream));
   b->k = k;
   a.k = k;
   // The launch shape must hold the new list: keep it when it does, else the
@@ -1544,16 +1542,14 @@ extern "C" int aco_b200_batch_apply_prior(aco_b200_batch *b, aco_b200_prior *pri
   const BatchArgs &a = b->args;
   uint16_t *lvl = const_cast<uint16_t *>(a.lvl);
   if (prior && gamma > 0.f) {
-    for (int i = 0; i < b->count; ++i) {
-      const BatchInst &I = b->inst[i];
-      int rc = acob200::prior::learned_levels(prior, a.coords + I.node_off, a.demand + I.node_off,
-                                              I.cap, I.n, b->k, a.cand + I.node_off * b->k,
-                                              lvl + I.node_off * b->k, gamma, 0, s);
-      if (rc) return rc;
-    }
+    const int rc = acob200::prior::learned_levels_multi(
+        prior, a.coords, a.demand, &a.inst->cap, (int)(sizeof(BatchInst) / sizeof(int)),
+        b->d_seg_off, b->d_seg_n, b->count, b->rows, b->k, a.cand, lvl, gamma, s);
+    if (rc) return rc;
   } else {
     BTRY(launch_knn_levels_multi(a.coords, b->d_seg_off, b->d_seg_n, b->count, b->rows, b->k,
-                                 b->d_thr, kThresholds, const_cast<uint16_t *>(a.cand), lvl, s));
+                                 b->d_thr, kThresholds, const_cast<uint16_t *>(a.cand), lvl,
+                                 nullptr, s));
   }
   BTRY(cudaStreamSynchronize(s));
   return ACO_OK;

@@ -106,11 +106,12 @@ ACO_API __global__ void kernel_evaporate_tau(uint8_t *d_tau, uint64_t total_elem
 
 ACO_API __global__ void kernel_build_candidate_lists(const float2 *d_coords, int *d_candidate_idx,
                                              float *d_eta_beta, CudaParams params) {
+  __shared__ unsigned long long s_buf[32][64];  // any block size the caller launches
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   const int k = params.cand_k;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i <= params.n; i += warps) {
-    const unsigned long long key = warp_knn(d_coords, params.n, k, i, lane);
+    const unsigned long long key = warp_knn(d_coords, params.n, k, i, lane, s_buf[threadIdx.x >> 5]);
     if (lane < k) {
       const int node = (key == ~0ull) ? 0 : (int)(key & 0xffffffffu);
       d_candidate_idx[i * k + lane] = node;

@@ -188,20 +188,18 @@ struct PheromoneView {
 // ---------------------------------------------------------------------------
 // Launch wrappers (aco_kernels.cu).
 // ---------------------------------------------------------------------------
+// Candidate lists and eta levels; tier, tier2: the fallback's lists too (null:
+// not).
 cudaError_t launch_knn_levels(const float2 *coords, int n, int k,
                               const float *thr, int J, uint16_t *cand,
-                              uint16_t *lvl, cudaStream_t s);
-cudaError_t launch_knn_tier(const float2 *coords, int n, int k, uint16_t *tier, uint16_t *tier2,
-                            cudaStream_t s);
-cudaError_t launch_knn_tier_multi(const float2 *coords, const long long *seg_off,
-                                  const int *seg_n, int count, long long rows, int k,
-                                  uint16_t *tier, cudaStream_t s);
+                              uint16_t *lvl, uint16_t *tier, uint16_t *tier2, cudaStream_t s);
 // Candidate lists of `count` instances packed one after another: instance s
-// has seg_n[s] customers and starts at row seg_off[s] (device arrays).
+// has seg_n[s] customers and starts at row seg_off[s] (device arrays).  tier:
+// the fallback's lists too (null: not).
 cudaError_t launch_knn_levels_multi(const float2 *coords, const long long *seg_off,
                                     const int *seg_n, int count, long long rows, int k,
                                     const float *thr, int J, uint16_t *cand, uint16_t *lvl,
-                                    cudaStream_t s);
+                                    uint16_t *tier, cudaStream_t s);
 cudaError_t launch_fill_u8(uint8_t *p, unsigned long long count, uint8_t v,
                            cudaStream_t s);
 cudaError_t launch_weights(const InstanceView &iv, const PheromoneView &pv,
@@ -373,43 +371,94 @@ __device__ __forceinline__ void st_cg_u8(uint8_t *p, uint8_t v) {
   asm volatile("st.global.cg.u8 [%0], %1;" ::"l"(p), "h"(w) : "memory");
 }
 
-// Warp-wide k-nearest selection for node i: the k smallest keys
-// (d^2 bits << 32 | j) over j in 1..n, j != i.  Lane t < k ends holding the
-// t-th smallest (~0 when fewer than k exist).  Keys are unique, so the order
-// is total: ascending d^2, ties to the lower j, as the reference's insertion
-// with a strict '<' (aco_cuda_kernels.cu:187-201).
-// With `after` given (not ~0), the k smallest keys greater than it: the
-// next ranks of the same order.
-__device__ inline unsigned long long warp_knn(const float2 *coords, int n, int k,
-                                       int i, int lane,
-                                       unsigned long long after = ~0ull) {
+// Keys of 32 lanes in ascending (up) or descending order (bitonic network).
+__device__ __forceinline__ unsigned long long warp_sort_step(unsigned long long x, int o,
+                                                             bool low_here) {
+  const unsigned long long y = __shfl_xor_sync(kFull, x, o);
+  return (x < y) == low_here ? x : y;
+}
+__device__ __forceinline__ unsigned long long warp_sort_descending(unsigned long long x, int lane) {
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+    for (int o = size >> 1; o > 0; o >>= 1)
+      x = warp_sort_step(x, o, ((lane & o) == 0) == ((lane & size) != 0 && size < 32));
+  return x;
+}
+
+// The k <= 32 smallest of the keys key_at(g) gives in groups 0 .. groups - 1
+// (one key per lane and group, ~0: none; unique otherwise): lane t < k ends
+// holding the t-th smallest.  Keys below the list's k-th wait in buf (64
+// words of the warp's shared memory) until 32 of them are sorted and merged
+// into the list at once; one insertion at a time was a chain of 8 shuffles
+// for every key (n=1000, three lists per node: 97 us, now 28).
+template <class KeyAt>
+__device__ __forceinline__ unsigned long long warp_smallest(KeyAt key_at, int groups, int k,
+                                                            int lane, unsigned long long *buf) {
   const unsigned long long kNone = ~0ull;
   unsigned long long list = kNone;
   unsigned long long kth = kNone;
-  const float2 pi = coords[i];
-  for (int base = 1; base <= n; base += 32) {
-    int j = base + lane;
-    unsigned long long key = kNone;
-    if (j <= n && j != i) {
-      float d2 = dist2f(pi, __ldg(coords + j));
-      key = ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)j;
-      if (after != kNone && key <= after) key = kNone;
-    }
-    unsigned m = __ballot_sync(kFull, key < kth);
-    while (m) {
-      int b = __ffs(m) - 1;
-      m &= m - 1;
-      unsigned long long x = __shfl_sync(kFull, key, b);
-      if (x < kth) {
-        int pos = __popc(__ballot_sync(kFull, lane < k && list < x));
-        unsigned long long up = __shfl_up_sync(kFull, list, 1);
-        if (lane > pos) list = up;
-        else if (lane == pos) list = x;
-        kth = __shfl_sync(kFull, list, k - 1);
+  int held = 0;
+  auto merge = [&](unsigned long long x) {
+    x = warp_sort_descending(x, lane);
+    list = x < list ? x : list;  // the 32 smallest of both, a bitonic sequence
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) list = warp_sort_step(list, o, (lane & o) == 0);
+    kth = __shfl_sync(kFull, list, k - 1);
+  };
+  constexpr int kAhead = 4;
+  for (int g = 0; g < groups; g += kAhead) {
+    unsigned long long keys[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) keys[u] = key_at(g + u);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const unsigned long long key = keys[u];
+      const unsigned m = __ballot_sync(kFull, key < kth);
+      if (m == 0u) continue;
+      if (key < kth) buf[held + __popc(m & ((1u << lane) - 1u))] = key;
+      held += __popc(m);
+      if (held >= 32) {
+        __syncwarp();
+        const unsigned long long x = buf[lane], rest = buf[32 + lane];
+        __syncwarp();
+        held -= 32;
+        if (lane < held) buf[lane] = rest;
+        merge(x);
+        __syncwarp();
       }
     }
   }
+  __syncwarp();
+  if (held > 0) merge(lane < held ? buf[lane] : kNone);
+  __syncwarp();
   return list;
+}
+
+// Key of node j seen from node i at pi: squared distance, then index; ~0 for
+// j = i and beyond n.  Keys are unique, so the order is total: ascending d^2,
+// ties to the lower j, as the reference's insertion with a strict '<'
+// (aco_cuda_kernels.cu:187-201).
+__device__ __forceinline__ unsigned long long node_key(const float2 *coords, int n, int i,
+                                                       float2 pi, int j) {
+  const float2 p = __ldg(coords + (j <= n ? j : i));
+  const unsigned long long key =
+      ((unsigned long long)__float_as_uint(dist2f(pi, p)) << 32) | (unsigned)j;
+  return j > n || j == i ? ~0ull : key;
+}
+
+// The k nearest nodes of node i (keys as node_key), of those with a key
+// greater than `after` if that is not ~0: the next ranks of the same order.
+__device__ inline unsigned long long warp_knn(const float2 *coords, int n, int k, int i, int lane,
+                                              unsigned long long *buf,
+                                              unsigned long long after = ~0ull) {
+  const float2 pi = coords[i];
+  return warp_smallest(
+      [&](int g) {
+        const unsigned long long key = node_key(coords, n, i, pi, 1 + 32 * g + lane);
+        return after != ~0ull && key <= after ? ~0ull : key;
+      },
+      (n + 31) / 32, k, lane, buf);
 }
 
 // What an ant still has to serve: one element per node in shared memory,

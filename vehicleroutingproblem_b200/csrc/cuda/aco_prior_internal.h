@@ -18,5 +18,14 @@ int learned_levels(aco_b200_prior *p, const float2 *coords, const int *demand, l
                    int n, int k, const uint16_t *cand, uint16_t *lvl, float gamma,
                    int residual, cudaStream_t s);
 
+// The same (residual = 0) for `count` instances packed one after another:
+// instance i owns seg_n[i] + 1 of the `rows` rows from seg_off[i] on and has
+// capacity cap[i cap_step] (device arrays; the rows of cand and lvl are all
+// rows').
+int learned_levels_multi(aco_b200_prior *p, const float2 *coords, const int *demand,
+                         const int *cap, int cap_step, const long long *seg_off, const int *seg_n,
+                         int count, long long rows, int k, const uint16_t *cand, uint16_t *lvl,
+                         float gamma, cudaStream_t s);
+
 }  // namespace prior
 }  // namespace acob200

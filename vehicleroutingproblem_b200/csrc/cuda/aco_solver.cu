@@ -503,8 +503,8 @@ int aco_b200_setup(aco_b200_ctx *ctx, const aco_b200_problem *p) {
   ctx->plan = plan_construct(iv, -1, ctx->num_sms, ctx->max_smem);
   ctx->evap_grid = evap_grid_for(tau_total, ctx->num_sms);
 
-  TRY(launch_knn_levels(ctx->d_coords, n, k, ctx->d_thr, kThresholds, ctx->d_cand, ctx->d_lvl, s));
-  TRY(launch_knn_tier(ctx->d_coords, n, k, ctx->d_tier, iv.tier2 ? ctx->d_tier2 : nullptr, s));
+  TRY(launch_knn_levels(ctx->d_coords, n, k, ctx->d_thr, kThresholds, ctx->d_cand, ctx->d_lvl,
+                        ctx->d_tier, iv.tier2 ? ctx->d_tier2 : nullptr, s));
   TRY(launch_fill_u8(ctx->d_tau, tau_total, ctx->q_tau0, s));
   if (ctx->d_lvl0) TRY(launch_depot_levels(ctx->d_coords, n, ctx->d_thr, kThresholds, ctx->d_lvl0, s));
 
@@ -667,14 +667,21 @@ int aco_b200_apply_prior_mode(aco_b200_ctx *ctx, aco_b200_prior *prior, float ga
   if (!ctx || !ctx->ready || mode < 0 || mode > 1) return ACO_ERR_INVALID_INPUT;
   cudaSetDevice(ctx->device);
   cudaStream_t s = ctx->stream;
-  // Plain levels first: they are the result without a prior and the base of
-  // the residual mode.
-  TRY(launch_knn_levels(ctx->d_coords, ctx->n, ctx->k, ctx->d_thr, kThresholds, ctx->d_cand,
-                        ctx->d_lvl, s));
-  if (prior && gamma > 0.f) {
+  const bool learned = prior && gamma > 0.f;
+  auto plain_levels = [&]() {
+    return launch_knn_levels(ctx->d_coords, ctx->n, ctx->k, ctx->d_thr, kThresholds, ctx->d_cand,
+                             ctx->d_lvl, nullptr, nullptr, s);
+  };
+  // Plain levels: the result without a prior and the base of the residual
+  // mode (mode 0 writes every level).
+  if (!learned || mode == 1) TRY(plain_levels());
+  if (learned) {
     int rc = acob200::prior::learned_levels(prior, ctx->d_coords, ctx->d_demand, ctx->cap, ctx->n,
                                             ctx->k, ctx->d_cand, ctx->d_lvl, gamma, mode, s);
-    if (rc) return rc;
+    if (rc) {
+      TRY(plain_levels());
+      return rc;
+    }
   }
   TRY(cudaStreamSynchronize(s));
   return ACO_OK;
