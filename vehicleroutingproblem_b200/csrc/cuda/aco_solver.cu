@@ -12,12 +12,14 @@ extern "C" {
 #include "solution.h"
 }
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <ctime>
+#include <type_traits>
 #include <vector>
 
 namespace acob200 {
@@ -37,15 +39,10 @@ using namespace acob200;
 namespace {
 
 constexpr int kChunkEpochs = 16;
-
-template <typename T>
-cudaError_t dalloc(T **p, size_t count) {
-  size_t bytes = (count * sizeof(T) + 15) & ~size_t(15);
-  if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMalloc((void **)p, bytes);
-  if (e == cudaSuccess) e = cudaMemset(*p, 0, bytes);
-  return e;
-}
+// Epochs per recorded graph, largest first; a run takes what fits.
+constexpr int kGraphEpochs[] = {kChunkEpochs, 4, 1};
+constexpr int kGraphs = 3;
+constexpr int kMaxAhead = 8 * kChunkEpochs;  // epochs in flight of one run
 
 }  // namespace
 
@@ -95,8 +92,22 @@ struct aco_b200_ctx {
   uint16_t *d_lvl0 = nullptr; // depot rule 1: eta level of d(i,0)^2
   unsigned int *d_counter = nullptr;
 
-  // host mirrors
-  DevState *h_state = nullptr;  // pinned
+  // Every device buffer is a 256-byte aligned slice of one allocation, kept
+  // while set-ups fit it.  The solution and the state are neighbours, and so
+  // are the state and all that a set-up uploads: one copy each.
+  unsigned char *arena = nullptr;
+  size_t arena_cap = 0;
+  size_t res_off = 0, res_lens = 0;          // best nodes, lengths, then the state
+  size_t up_off = 0, up_end = 0;             // the state and the other uploads
+  std::vector<unsigned char> stage;          // host side of those copies
+
+  // host mirrors.  Not pinned: a pinned allocation per context took longer
+  // (1.2 ms, and 0.4 ms to free) than it saves over a context's copies.
+  DevState h_state = {};
+  // h_state is what the device holds.  Not after launches that run() does not
+  // wait for; never between split-colony calls and the next set-up (a caller
+  // may replay those from a graph of its own).
+  bool state_known = false, split = false;
   int log_read = 0;
 
   InstanceView iv = {};
@@ -105,8 +116,8 @@ struct aco_b200_ctx {
   SmemPlan plan = {};
   int evap_grid = 1;
 
-  cudaGraphExec_t graph_chunk = nullptr;
-  cudaGraphExec_t graph_one = nullptr;
+  cudaGraphExec_t graphs[kGraphs] = {};  // of kGraphEpochs epochs, made when first needed
+  double table_key[3] = {};              // alpha, beta, level step of A and thr
   int graph_gen = 1;  // changes whenever the captured launch arguments may have
   bool run_limit_off = false;  // device run limit known to be disabled
   int depot_rule = 0;
@@ -117,6 +128,7 @@ struct aco_b200_ctx {
                           sizeof(AntBuffers) + sizeof(SmemPlan) + 8 * sizeof(void *)] = {};
   void make_graph_key(unsigned char *key) const;
 
+  void drop_graphs();
   void free_buffers();
   ~aco_b200_ctx();
 };
@@ -139,33 +151,25 @@ void aco_b200_ctx::make_graph_key(unsigned char *key) const {
   put(ptrs, sizeof(ptrs));
 }
 
+void aco_b200_ctx::drop_graphs() {
+  for (cudaGraphExec_t &g : graphs) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+}
+
 void aco_b200_ctx::free_buffers() {
-  if (graph_chunk) cudaGraphExecDestroy(graph_chunk);
-  if (graph_one) cudaGraphExecDestroy(graph_one);
-  graph_chunk = graph_one = nullptr;
+  drop_graphs();
   ++graph_gen;
-  void *ptrs[] = {d_coords, d_demand, d_cand, d_lvl, d_thr, d_A, d_lut, d_tau, d_tau2,
-                  d_w, d_rel, ab.routes, ab.lens, ab.cost, ab.feasible, ab.steps,
-                  ab.draws, ab.loads, ab.rep, ab.repc, d_state, d_log,
-                  d_gbest_nodes, d_gbest_lens, d_tmp_nodes, d_tmp_lens, d_iter_nodes,
-                  d_iter_lens, d_counter, d_rdep, d_lvl0, d_tier, d_tier2};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
-  d_coords = nullptr; d_demand = nullptr; d_cand = d_lvl = nullptr; d_thr = nullptr;
-  d_A = nullptr; d_lut = nullptr; d_tau = nullptr; d_tau2 = nullptr; d_w = nullptr;
-  d_rel = nullptr;
-  ab = AntBuffers{};
-  d_state = nullptr; d_log = nullptr; d_gbest_nodes = d_gbest_lens = nullptr;
-  d_tmp_nodes = d_tmp_lens = nullptr; d_iter_nodes = d_iter_lens = nullptr;
-  d_rdep = nullptr; d_lvl0 = nullptr; d_tier = nullptr; d_tier2 = nullptr;
-  d_counter = nullptr;
+  if (arena) cudaFree(arena);
+  arena = nullptr;
+  arena_cap = 0;
   ready = false;
 }
 
 aco_b200_ctx::~aco_b200_ctx() {
   cudaSetDevice(device);
   free_buffers();
-  if (h_state) cudaFreeHost(h_state);
   if (own_stream && stream) cudaStreamDestroy(stream);
   if (side) cudaStreamDestroy(side);
   if (ev_fork) cudaEventDestroy(ev_fork);
@@ -179,20 +183,6 @@ aco_b200_ctx::~aco_b200_ctx() {
       fprintf(stderr, "aco_b200: CUDA error %s at %s:%d\n",              \
               cudaGetErrorString(err__), __FILE__, __LINE__);            \
       return ACO_ERR_BACKEND;                                            \
-    }                                                                    \
-  } while (0)
-
-#define TRY_ALLOC(call)                                                  \
-  do {                                                                   \
-    cudaError_t err__ = (ctx->inject_alloc > 0 && --ctx->inject_alloc == 0) \
-                            ? cudaErrorMemoryAllocation                  \
-                            : (call);                                    \
-    if (err__ != cudaSuccess) {                                          \
-      fprintf(stderr, "aco_b200: device allocation failed: %s\n",       \
-              cudaGetErrorString(err__));                                \
-      ctx->free_buffers();                                               \
-      return err__ == cudaErrorMemoryAllocation ? ACO_ERR_ALLOCATION     \
-                                                : ACO_ERR_BACKEND;       \
     }                                                                    \
   } while (0)
 
@@ -304,8 +294,7 @@ int aco_b200_create(aco_b200_ctx **out, int device) {
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess ||
-      cudaMallocHost((void **)&ctx->h_state, sizeof(DevState)) != cudaSuccess) {
+      cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess) {
     delete ctx;
     return ACO_ERR_BACKEND;
   }
@@ -322,9 +311,7 @@ int aco_b200_destroy(aco_b200_ctx *ctx) {
 int aco_b200_set_stream(aco_b200_ctx *ctx, void *cuda_stream) {
   if (!ctx) return ACO_ERR_INVALID_INPUT;
   cudaSetDevice(ctx->device);
-  if (ctx->graph_chunk) cudaGraphExecDestroy(ctx->graph_chunk);
-  if (ctx->graph_one) cudaGraphExecDestroy(ctx->graph_one);
-  ctx->graph_chunk = ctx->graph_one = nullptr;
+  ctx->drop_graphs();
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   if (cuda_stream) {
     ctx->stream = (cudaStream_t)cuda_stream;
@@ -379,9 +366,9 @@ int aco_b200_setup(aco_b200_ctx *ctx, const aco_b200_problem *p) {
   cudaSetDevice(ctx->device);
   // Same sizes as the last set-up: the device buffers are reused (no
   // allocation), and the graphs too when their captured arguments match.
+  ctx->state_known = false;
   const bool reuse = ctx->ready && ctx->n == n && ctx->K == p->K && ctx->k == k &&
                      ctx->m == m && ctx->depot_rule == p->depot_rule;
-  if (!reuse) ctx->free_buffers();
   ctx->ready = false;
   ctx->depot_rule = p->depot_rule;
   ctx->n = n;
@@ -394,66 +381,127 @@ int aco_b200_setup(aco_b200_ctx *ctx, const aco_b200_problem *p) {
   ctx->seed = p->seed;
   derive_params(p->rho, p->tau0, &ctx->log_min, &ctx->log_step, &ctx->delta, &ctx->q_tau0);
   ctx->Qs = (float)p->Q * 100.0f;
-  build_tables(p->alpha, p->beta, ctx->log_step, ctx->A, ctx->lut, ctx->thr);
+  const double table_key[3] = {p->alpha, p->beta, (double)ctx->log_step};
+  if (ctx->thr.empty() || memcmp(table_key, ctx->table_key, sizeof(table_key)) != 0) {
+    build_tables(p->alpha, p->beta, ctx->log_step, ctx->A, ctx->lut, ctx->thr);
+    memcpy(ctx->table_key, table_key, sizeof(table_key));
+  }
 
   const size_t rows = (size_t)n + 1;
   const int R = n + 2 * p->K;
   const unsigned long long tau_total = (unsigned long long)rows * rows;
   const size_t dem_words = (rows + 3) & ~size_t(3);  // the ants' elements follow, 16-byte aligned
+  const int eb = demand_bytes(max_demand);
+  cudaStream_t s = ctx->stream;
   if (!reuse) {
-    TRY_ALLOC(dalloc(&ctx->d_coords, rows));
-    TRY_ALLOC(dalloc(&ctx->d_demand, dem_words + unserved_bytes(n, 4) / 4));
-    TRY_ALLOC(dalloc(&ctx->d_cand, rows * k));
-    TRY_ALLOC(dalloc(&ctx->d_lvl, rows * k));
-    TRY_ALLOC(dalloc(&ctx->d_tier, rows * kTierLen));
-    if (n >= kTier2MinCustomers) TRY_ALLOC(dalloc(&ctx->d_tier2, rows * kTier2Len));
-    TRY_ALLOC(dalloc(&ctx->d_thr, (size_t)kThresholds));
-    TRY_ALLOC(dalloc(&ctx->d_A, 256));
-    TRY_ALLOC(dalloc(&ctx->d_lut, 256));
-    TRY_ALLOC(dalloc(&ctx->d_tau, (size_t)tau_total));
-    TRY_ALLOC(dalloc(&ctx->d_tau2, (size_t)tau_total));
-    TRY_ALLOC(dalloc(&ctx->d_w, rows * k));
-    TRY_ALLOC(dalloc(&ctx->d_rel, rows * k));
-    TRY_ALLOC(dalloc(&ctx->ab.routes, (size_t)m * R));
-    TRY_ALLOC(dalloc(&ctx->ab.lens, (size_t)m * p->K));
-    TRY_ALLOC(dalloc(&ctx->ab.cost, (size_t)m));
-    TRY_ALLOC(dalloc(&ctx->ab.feasible, (size_t)m));
-    TRY_ALLOC(dalloc(&ctx->ab.steps, (size_t)m));
-    TRY_ALLOC(dalloc(&ctx->ab.draws, (size_t)m));
-    TRY_ALLOC(dalloc(&ctx->ab.loads, (size_t)m * p->K));
-    TRY_ALLOC(dalloc(&ctx->ab.rep, (size_t)m * n));
-    TRY_ALLOC(dalloc(&ctx->ab.repc, (size_t)m * p->K));
-    TRY_ALLOC(dalloc(&ctx->d_state, 1));
-    TRY_ALLOC(dalloc(&ctx->d_log, (size_t)kLogCap));
-    TRY_ALLOC(dalloc(&ctx->d_gbest_nodes, (size_t)R));
-    TRY_ALLOC(dalloc(&ctx->d_gbest_lens, (size_t)p->K));
-    TRY_ALLOC(dalloc(&ctx->d_tmp_nodes, (size_t)R));
-    TRY_ALLOC(dalloc(&ctx->d_tmp_lens, (size_t)p->K));
-    TRY_ALLOC(dalloc(&ctx->d_iter_nodes, (size_t)R));
-    TRY_ALLOC(dalloc(&ctx->d_iter_lens, (size_t)p->K));
-    if (p->depot_rule == kDepotRuleCudaRef) {
-      TRY_ALLOC(dalloc(&ctx->d_rdep, rows));
-      TRY_ALLOC(dalloc(&ctx->d_lvl0, rows));
+    const bool cref = p->depot_rule == kDepotRuleCudaRef;
+    const size_t mm = (size_t)m;
+    unsigned char *base = nullptr;
+    size_t off = 0;
+    bool failed = false;  // the injected failure (aco_b200_debug_inject)
+    auto carve = [&](auto **ptr, size_t count, bool want = true) {
+      using T = std::remove_reference_t<decltype(**ptr)>;
+      *ptr = want ? reinterpret_cast<T *>(base + off) : nullptr;
+      if (!want) return;
+      if (!base && ctx->inject_alloc > 0 && --ctx->inject_alloc == 0) failed = true;
+      off += (count * sizeof(T) + 255) & ~size_t(255);
+    };
+    auto layout = [&]() {
+      off = 0;
+      ctx->res_off = off;
+      carve(&ctx->d_gbest_nodes, (size_t)R);
+      ctx->res_lens = off;
+      carve(&ctx->d_gbest_lens, (size_t)p->K);
+      ctx->up_off = off;
+      carve(&ctx->d_state, 1);
+      carve(&ctx->d_counter, 1);
+      carve(&ctx->d_A, 256);
+      carve(&ctx->d_lut, 256);
+      carve(&ctx->d_thr, (size_t)kThresholds);
+      carve(&ctx->d_coords, rows);
+      carve(&ctx->d_demand, dem_words + unserved_bytes(n, 4) / 4);
+      ctx->up_end = off;
+      carve(&ctx->d_cand, rows * k);
+      carve(&ctx->d_lvl, rows * k);
+      carve(&ctx->d_tier, rows * kTierLen);
+      carve(&ctx->d_tier2, rows * kTier2Len, n >= kTier2MinCustomers);
+      carve(&ctx->d_tau, (size_t)tau_total);
+      carve(&ctx->d_tau2, (size_t)tau_total);
+      carve(&ctx->d_w, rows * k);
+      carve(&ctx->d_rel, rows * k);
+      carve(&ctx->ab.routes, mm * R);
+      carve(&ctx->ab.lens, mm * p->K);
+      carve(&ctx->ab.cost, mm);
+      carve(&ctx->ab.feasible, mm);
+      carve(&ctx->ab.steps, mm);
+      carve(&ctx->ab.draws, mm);
+      carve(&ctx->ab.loads, mm * p->K);
+      carve(&ctx->ab.rep, mm * n);
+      carve(&ctx->ab.repc, mm * p->K);
+      carve(&ctx->d_log, (size_t)kLogCap);
+      carve(&ctx->d_tmp_nodes, (size_t)R);
+      carve(&ctx->d_tmp_lens, (size_t)p->K);
+      carve(&ctx->d_iter_nodes, (size_t)R);
+      carve(&ctx->d_iter_lens, (size_t)p->K);
+      carve(&ctx->d_rdep, rows, cref);
+      carve(&ctx->d_lvl0, rows, cref);
+    };
+    layout();
+    cudaError_t err = failed ? cudaErrorMemoryAllocation : cudaSuccess;
+    // What is there stays if it is large enough and not far too large (other
+    // streams may still read it); else one new allocation.
+    if (err == cudaSuccess && ctx->arena && off <= ctx->arena_cap &&
+        ctx->arena_cap <= 4 * off + (size_t(16) << 20)) {
+      err = cudaDeviceSynchronize();
+    } else {
+      ctx->free_buffers();
+      if (err == cudaSuccess) err = cudaMalloc((void **)&ctx->arena, off);
+      if (err == cudaSuccess) ctx->arena_cap = off;
     }
-    TRY_ALLOC(dalloc(&ctx->d_counter, 1));
+    if (err == cudaSuccess) err = cudaMemsetAsync(ctx->arena, 0, off, s);
+    if (err != cudaSuccess) {
+      fprintf(stderr, "aco_b200: device allocation failed: %s\n", cudaGetErrorString(err));
+      ctx->free_buffers();
+      return err == cudaErrorMemoryAllocation ? ACO_ERR_ALLOCATION : ACO_ERR_BACKEND;
+    }
+    base = ctx->arena;
+    layout();
   }
 
-  std::vector<float2> xy(rows);
-  const int eb = demand_bytes(max_demand);
-  std::vector<int> dem(dem_words + unserved_bytes(n, eb) / 4, -1);
-  for (size_t i = 0; i < rows; ++i) dem[i] = i ? 1 : 0;
+  // The uploads, laid out as on the device: state, tables, coordinates,
+  // demands with the ants' elements behind them.
+  const size_t up = ctx->up_off;
+  ctx->stage.assign(ctx->up_end - up, 0);
+  auto staged = [&](const void *dev) {
+    return ctx->stage.data() + (reinterpret_cast<const unsigned char *>(dev) - ctx->arena - up);
+  };
+  memcpy(staged(ctx->d_A), ctx->A, sizeof(ctx->A));
+  memcpy(staged(ctx->d_lut), ctx->lut, sizeof(ctx->lut));
+  memcpy(staged(ctx->d_thr), ctx->thr.data(), kThresholds * sizeof(float));
+  float2 *xy = reinterpret_cast<float2 *>(staged(ctx->d_coords));
   for (size_t i = 0; i < rows; ++i) xy[i] = make_float2(p->x[i], p->y[i]);
-  if (p->demand) for (size_t i = 0; i < rows; ++i) dem[i] = p->demand[i];
-  uint8_t *elems = reinterpret_cast<uint8_t *>(dem.data() + dem_words);
+  int *dem = reinterpret_cast<int *>(staged(ctx->d_demand));
+  for (size_t i = 1; i < rows; ++i) dem[i] = p->demand ? p->demand[i] : 1;
+  uint8_t *elems = reinterpret_cast<uint8_t *>(dem + dem_words);
+  memset(elems, 0xff, unserved_bytes(n, eb));
   for (int j = 1; j <= n; ++j)  // little-endian: the low bytes are the demand
     memcpy(elems + (size_t)j * eb, &dem[j], (size_t)eb);
-  cudaStream_t s = ctx->stream;
-  if (reuse) TRY(cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned int), s));
-  TRY(cudaMemcpyAsync(ctx->d_coords, xy.data(), rows * sizeof(float2), cudaMemcpyHostToDevice, s));
-  TRY(cudaMemcpyAsync(ctx->d_demand, dem.data(), dem.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-  TRY(cudaMemcpyAsync(ctx->d_thr, ctx->thr.data(), kThresholds * sizeof(float), cudaMemcpyHostToDevice, s));
-  TRY(cudaMemcpyAsync(ctx->d_A, ctx->A, sizeof(ctx->A), cudaMemcpyHostToDevice, s));
-  TRY(cudaMemcpyAsync(ctx->d_lut, ctx->lut, sizeof(ctx->lut), cudaMemcpyHostToDevice, s));
+  DevState st = {};
+  st.global_best = DBL_MAX;
+  st.iter_best = DBL_MAX;
+  st.best_ant = -1;
+  st.stagnation = p->stagnation_epochs > 0 ? p->stagnation_epochs : 0;
+  st.fixed_epochs = p->fixed_epochs > 0 ? p->fixed_epochs : 0;
+  st.min_rel = p->min_rel_improvement > 0.0 ? p->min_rel_improvement : 1e-3;
+  st.timeout_ns = p->timeout_seconds > 0.0
+                      ? (unsigned long long)(p->timeout_seconds * 1e9)
+                      : 0ull;
+  st.Qs = ctx->Qs;
+  st.seed = ctx->seed;
+  ctx->h_state = st;
+  memcpy(staged(ctx->d_state), &st, sizeof(st));
+  TRY(cudaMemcpyAsync(ctx->d_state, ctx->stage.data(), ctx->stage.size(), cudaMemcpyHostToDevice,
+                      s));
 
   InstanceView &iv = ctx->iv;
   iv.n = n;
@@ -508,30 +556,16 @@ int aco_b200_setup(aco_b200_ctx *ctx, const aco_b200_problem *p) {
   TRY(launch_fill_u8(ctx->d_tau, tau_total, ctx->q_tau0, s));
   if (ctx->d_lvl0) TRY(launch_depot_levels(ctx->d_coords, n, ctx->d_thr, kThresholds, ctx->d_lvl0, s));
 
-  DevState st = {};
-  st.global_best = DBL_MAX;
-  st.iter_best = DBL_MAX;
-  st.best_ant = -1;
-  st.stagnation = p->stagnation_epochs > 0 ? p->stagnation_epochs : 0;
-  st.fixed_epochs = p->fixed_epochs > 0 ? p->fixed_epochs : 0;
-  st.min_rel = p->min_rel_improvement > 0.0 ? p->min_rel_improvement : 1e-3;
-  st.timeout_ns = p->timeout_seconds > 0.0
-                      ? (unsigned long long)(p->timeout_seconds * 1e9)
-                      : 0ull;
-  st.Qs = ctx->Qs;
-  st.seed = ctx->seed;
-  *ctx->h_state = st;
-  TRY(cudaMemcpyAsync(ctx->d_state, ctx->h_state, sizeof(DevState), cudaMemcpyHostToDevice, s));
   TRY(cudaStreamSynchronize(s));
   ctx->log_read = 0;
+  ctx->state_known = true;
+  ctx->split = false;
   ctx->run_limit_off = true;  // fresh state: run_limit = 0
   unsigned char key[sizeof(ctx->graph_key)];
   memset(key, 0, sizeof(key));
   ctx->make_graph_key(key);
   if (memcmp(key, ctx->graph_key, sizeof(key)) != 0) {
-    if (ctx->graph_chunk) cudaGraphExecDestroy(ctx->graph_chunk);
-    if (ctx->graph_one) cudaGraphExecDestroy(ctx->graph_one);
-    ctx->graph_chunk = ctx->graph_one = nullptr;
+    ctx->drop_graphs();
     memcpy(ctx->graph_key, key, sizeof(key));
     ++ctx->graph_gen;
   }
@@ -539,14 +573,17 @@ int aco_b200_setup(aco_b200_ctx *ctx, const aco_b200_problem *p) {
   return ACO_OK;
 }
 
-static int ensure_graphs(aco_b200_ctx *ctx) {
-  if (!ctx->graph_one) {
-    int rc = build_graph(ctx, 1, &ctx->graph_one);
-    if (rc) return rc;
-  }
-  if (!ctx->graph_chunk) {
-    int rc = build_graph(ctx, kChunkEpochs, &ctx->graph_chunk);
-    if (rc) return rc;
+// Enqueues `epochs` epochs as graphs of kGraphEpochs, recorded when first
+// needed.
+static int launch_epochs(aco_b200_ctx *ctx, int epochs) {
+  for (int g = 0; g < kGraphs; ++g) {
+    for (; epochs >= kGraphEpochs[g]; epochs -= kGraphEpochs[g]) {
+      if (!ctx->graphs[g]) {
+        const int rc = build_graph(ctx, kGraphEpochs[g], &ctx->graphs[g]);
+        if (rc) return rc;
+      }
+      TRY(cudaGraphLaunch(ctx->graphs[g], ctx->stream));
+    }
   }
   return ACO_OK;
 }
@@ -556,23 +593,31 @@ int aco_b200_run(aco_b200_ctx *ctx, int max_epochs, aco_b200_state *state,
                  int *n_records) {
   if (!ctx || !ctx->ready || max_epochs < 0) return ACO_ERR_INVALID_INPUT;
   cudaSetDevice(ctx->device);
-  int rc = ensure_graphs(ctx);
-  if (rc) return rc;
   cudaStream_t s = ctx->stream;
-  TRY(cudaMemcpyAsync(ctx->h_state, ctx->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, s));
-  TRY(cudaStreamSynchronize(s));
-  const int limit = ctx->h_state->epoch + max_epochs;
+  if (!ctx->state_known) {
+    TRY(cudaMemcpyAsync(&ctx->h_state, ctx->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, s));
+    TRY(cudaStreamSynchronize(s));
+  }
+  ctx->state_known = false;
+  const int limit = ctx->h_state.epoch + max_epochs;
   TRY(launch_set_run_limit(ctx->d_state, limit, s));
   ctx->run_limit_off = false;
+  // What k_set_run_limit makes of the state just read.
+  ctx->h_state.stop_flags &= ~kStopRunLimit;
+  if (limit > 0 && ctx->h_state.epoch >= limit) ctx->h_state.stop_flags |= kStopRunLimit;
+  bool known = true;
   int nrec = 0;
   std::vector<EpochRec> recs;
   // Every pass either stops or advances the device epoch; the guard only
   // bounds the loop should a device-side rule misbehave.
   long long guard = (long long)max_epochs + 8;
   while (guard-- > 0) {
-    TRY(cudaMemcpyAsync(ctx->h_state, ctx->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, s));
-    TRY(cudaStreamSynchronize(s));
-    const DevState &hs = *ctx->h_state;
+    if (!known) {
+      TRY(cudaMemcpyAsync(&ctx->h_state, ctx->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, s));
+      TRY(cudaStreamSynchronize(s));
+    }
+    known = false;
+    const DevState &hs = ctx->h_state;
     // Epoch records written since the last read.
     int avail = hs.log_count - ctx->log_read;
     if (avail > kLogCap) {
@@ -601,14 +646,16 @@ int aco_b200_run(aco_b200_ctx *ctx, int max_epochs, aco_b200_state *state,
       return ACO_ERR_BACKEND;
     }
     if (hs.stop_flags || hs.epoch >= limit) break;
-    const int left = limit - hs.epoch;
-    if (left >= kChunkEpochs) {
-      TRY(cudaGraphLaunch(ctx->graph_chunk, s));
-    } else {
-      for (int i = 0; i < left; ++i) TRY(cudaGraphLaunch(ctx->graph_one, s));
-    }
+    int left = limit - hs.epoch;
+    if (hs.fixed_epochs > 0) left = std::min(left, hs.fixed_epochs - hs.epoch);
+    // A rule that may stop the run early is looked at after every chunk; with
+    // none, up to kMaxAhead epochs are enqueued at a time.
+    if (hs.stagnation > 0 || hs.timeout_ns > 0ull) left = std::min(left, kChunkEpochs);
+    const int rc = launch_epochs(ctx, std::min(left, kMaxAhead));
+    if (rc) return rc;
   }
-  if (state) fill_state(state, *ctx->h_state);
+  ctx->state_known = !ctx->split;
+  if (state) fill_state(state, ctx->h_state);
   if (n_records) *n_records = nrec;
   return ACO_OK;
 }
@@ -616,20 +663,13 @@ int aco_b200_run(aco_b200_ctx *ctx, int max_epochs, aco_b200_state *state,
 int aco_b200_enqueue_epochs(aco_b200_ctx *ctx, int epochs) {
   if (!ctx || !ctx->ready || epochs < 0) return ACO_ERR_INVALID_INPUT;
   cudaSetDevice(ctx->device);
-  int rc = ensure_graphs(ctx);
-  if (rc) return rc;
   cudaStream_t s = ctx->stream;
   if (!ctx->run_limit_off) {
     TRY(launch_set_run_limit(ctx->d_state, 0, s));
     ctx->run_limit_off = true;
   }
-  int left = epochs;
-  while (left >= kChunkEpochs) {
-    TRY(cudaGraphLaunch(ctx->graph_chunk, s));
-    left -= kChunkEpochs;
-  }
-  for (int i = 0; i < left; ++i) TRY(cudaGraphLaunch(ctx->graph_one, s));
-  return ACO_OK;
+  ctx->state_known = false;
+  return launch_epochs(ctx, epochs);
 }
 
 int aco_b200_debug_inject(aco_b200_ctx *ctx, int what, int value) {
@@ -641,9 +681,7 @@ int aco_b200_debug_inject(aco_b200_ctx *ctx, int what, int value) {
   if (what == 2) {
     cudaSetDevice(ctx->device);
     ctx->iv.stage_extra_tx = value ? 16 : 0;
-    if (ctx->graph_chunk) cudaGraphExecDestroy(ctx->graph_chunk);
-    if (ctx->graph_one) cudaGraphExecDestroy(ctx->graph_one);
-    ctx->graph_chunk = ctx->graph_one = nullptr;
+    ctx->drop_graphs();
     memset(ctx->graph_key, 0, sizeof(ctx->graph_key));
     ++ctx->graph_gen;
     return ACO_OK;
@@ -704,6 +742,8 @@ int aco_b200_shard_packet_ints(aco_b200_ctx *ctx) {
 int aco_b200_shard_construct(aco_b200_ctx *ctx, int32_t *d_send) {
   if (!ctx || !ctx->ready || !d_send) return ACO_ERR_INVALID_INPUT;
   cudaSetDevice(ctx->device);
+  ctx->state_known = false;
+  ctx->split = true;
   cudaStream_t s = ctx->stream;
   if (!ctx->run_limit_off) {
     TRY(launch_set_run_limit(ctx->d_state, 0, s));
@@ -725,6 +765,8 @@ int aco_b200_shard_construct(aco_b200_ctx *ctx, int32_t *d_send) {
 int aco_b200_shard_update(aco_b200_ctx *ctx, const int32_t *d_recv, int world) {
   if (!ctx || !ctx->ready || !d_recv || world < 1) return ACO_ERR_INVALID_INPUT;
   cudaSetDevice(ctx->device);
+  ctx->state_known = false;
+  ctx->split = true;
   cudaStream_t s = ctx->stream;
   TRY(launch_shard_select(ctx->iv, ctx->d_state, d_recv, world, ctx->d_iter_nodes,
                           ctx->d_iter_lens, ctx->d_gbest_nodes, ctx->d_gbest_lens, ctx->d_log,
@@ -734,6 +776,7 @@ int aco_b200_shard_update(aco_b200_ctx *ctx, const int32_t *d_recv, int world) {
 
 int aco_b200_profile_epochs(aco_b200_ctx *ctx, int epochs, float *kernel_ms) {
   if (!ctx || !ctx->ready || epochs < 0 || !kernel_ms) return ACO_ERR_INVALID_INPUT;
+  ctx->state_known = false;
   cudaSetDevice(ctx->device);
   cudaStream_t s = ctx->stream;
   cudaEvent_t ev[5];
@@ -772,6 +815,7 @@ int aco_b200_profile_epochs(aco_b200_ctx *ctx, int epochs, float *kernel_ms) {
 
 int aco_b200_profile_update(aco_b200_ctx *ctx, int launches, float *ms_per_launch) {
   if (!ctx || !ctx->ready || launches < 1 || !ms_per_launch) return ACO_ERR_INVALID_INPUT;
+  ctx->state_known = false;
   cudaSetDevice(ctx->device);
   cudaStream_t s = ctx->stream;
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -813,9 +857,9 @@ int aco_b200_synchronize(aco_b200_ctx *ctx) {
 int aco_b200_get_state(aco_b200_ctx *ctx, aco_b200_state *state) {
   if (!ctx || !ctx->ready || !state) return ACO_ERR_INVALID_INPUT;
   cudaSetDevice(ctx->device);
-  TRY(cudaMemcpyAsync(ctx->h_state, ctx->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
+  TRY(cudaMemcpyAsync(&ctx->h_state, ctx->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
   TRY(cudaStreamSynchronize(ctx->stream));
-  fill_state(state, *ctx->h_state);
+  fill_state(state, ctx->h_state);
   return ACO_OK;
 }
 
@@ -841,22 +885,26 @@ int aco_b200_get_best(aco_b200_ctx *ctx, int *nodes, int *lens, double *cost) {
   if (!ctx || !ctx->ready) return ACO_ERR_INVALID_INPUT;
   cudaSetDevice(ctx->device);
   cudaStream_t s = ctx->stream;
-  TRY(cudaMemcpyAsync(ctx->h_state, ctx->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, s));
-  if (lens) TRY(cudaMemcpyAsync(lens, ctx->d_gbest_lens, sizeof(int) * ctx->K, cudaMemcpyDeviceToHost, s));
-  if (nodes)
-    TRY(cudaMemcpyAsync(nodes, ctx->d_gbest_nodes, sizeof(int) * (ctx->n + 2 * ctx->K),
-                        cudaMemcpyDeviceToHost, s));
+  // Nodes, lengths and state lie one after another: one copy.
+  const size_t bytes = ctx->up_off + sizeof(DevState) - ctx->res_off;
+  ctx->stage.resize(std::max(ctx->stage.size(), bytes));
+  const unsigned char *h = ctx->stage.data();
+  TRY(cudaMemcpyAsync(ctx->stage.data(), ctx->arena + ctx->res_off, bytes, cudaMemcpyDeviceToHost,
+                      s));
   TRY(cudaStreamSynchronize(s));
-  if (cost) *cost = ctx->h_state->global_best;
-  return ctx->h_state->global_best < DBL_MAX ? ACO_OK : ACO_ERR_NO_SOLUTION;
+  memcpy(&ctx->h_state, h + (ctx->up_off - ctx->res_off), sizeof(DevState));
+  if (lens) memcpy(lens, h + (ctx->res_lens - ctx->res_off), sizeof(int) * ctx->K);
+  if (nodes) memcpy(nodes, h, sizeof(int) * (ctx->n + 2 * ctx->K));
+  if (cost) *cost = ctx->h_state.global_best;
+  return ctx->h_state.global_best < DBL_MAX ? ACO_OK : ACO_ERR_NO_SOLUTION;
 }
 
 // The context's current pheromone buffer (read from the device state).
 static int current_tau(aco_b200_ctx *ctx, uint8_t **out) {
-  TRY(cudaMemcpyAsync(ctx->h_state, ctx->d_state, sizeof(DevState), cudaMemcpyDeviceToHost,
+  TRY(cudaMemcpyAsync(&ctx->h_state, ctx->d_state, sizeof(DevState), cudaMemcpyDeviceToHost,
                       ctx->stream));
   TRY(cudaStreamSynchronize(ctx->stream));
-  *out = ctx->h_state->tau_sel ? ctx->d_tau2 : ctx->d_tau;
+  *out = ctx->h_state.tau_sel ? ctx->d_tau2 : ctx->d_tau;
   return ACO_OK;
 }
 
