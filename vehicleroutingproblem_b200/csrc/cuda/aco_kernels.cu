@@ -540,8 +540,7 @@ __device__ __forceinline__ int clamp_int(long long v) {
 // What bounds it: the latency of the step's dependent chain (row load, the
 // candidates' elements, sums, choice, next row's address) at one or two
 // warps per scheduler, about 200 cycles of a step's 270 at n=1000.  Candidate t sits in lane
-// 31 - t, so that "the first candidate" is the highest set bit of a ballot
-// (one find-leading-one).
+// 31 - t, so that "the first candidate" is the highest lane.
 template <int L, int E, bool CREF>
 __device__ __forceinline__ void build_ant(const ConstructArgs &a, const Tables<L> &tb,
                                           Unserved<E> &us, uint32_t *dbuf, int *route_s, int ant,
@@ -608,14 +607,29 @@ __device__ __forceinline__ void build_ant(const ConstructArgs &a, const Tables<L
     int c = tb.candidate(0u);
     uint32_t w = tb.weight(0u);
     uint32_t e = us.get(c);
-    auto take_step = [&](int nx, uint32_t base, uint32_t dnx) {
+    auto take_step = [&](int nx, uint32_t dnx, bool draw) {
+      const uint32_t base = (uint32_t)nx * (uint32_t)k;
       c = tb.candidate(base);
-      w = tb.weight(base);
+      // From shared memory the candidates' elements, which wait for the row's
+      // candidates, come before its weights, which do not; a row on its way
+      // from L2 is asked for as a whole first (clustered n=2000 483 -> 464 us,
+      // n=3000 997 -> 991 us).
+      if (L == kLayoutGlobal) w = tb.weight(base);
       us.mark(nx);
+      if (L != kLayoutGlobal) {
+        e = us.get(c);
+        w = tb.weight(base);
+      }
+      // A draw is consumed only by a roulette selection.
+      if (draw) {
+        --left;
+        next_draw();
+      }
       route[pos] = nx;  // every lane stores the same value
       ++pos;
       room -= (int)dnx;
       cur = nx;
+      if (L == kLayoutGlobal) e = us.get(c);
     };
     while (open && room > floor_room) {
       // The step loop proper.  Its one loop test is a vote, so that the
@@ -625,9 +639,12 @@ __device__ __forceinline__ void build_ant(const ConstructArgs &a, const Tables<L
 #pragma unroll 1
       while (__any_sync(kFull, room > floor_room && left > 0)) {
         const uint32_t lim = us.limit(room);
-        // This lane's candidate's row offset, off the chain, so that the
-        // selected lane's reaches the next row's loads by one shuffle.
-        const uint32_t cb = (uint32_t)c * (uint32_t)k;
+        // Lane and candidate (and, where it fits, the candidate's demand) in
+        // one word: the largest such word of the lanes past the threshold is
+        // the first one's, so one reduction (20 cycles) chooses the customer,
+        // where ballot, find-leading-one and shuffle took 60.
+        const uint32_t word = E == 1 ? (uint32_t)c | (e << 16) | ((uint32_t)(lane + 1) << 24)
+                                     : (uint32_t)c | ((uint32_t)(lane + 1) << 16);
         const uint32_t wv = e <= lim ? w : 0u;
         const uint32_t denom = __reduce_add_sync(kFull, wv);
         // cum 2^24 >= r denom  <=>  cum >= ceil(r denom / 2^24)  <=>
@@ -638,25 +655,23 @@ __device__ __forceinline__ void build_ant(const ConstructArgs &a, const Tables<L
         // (lanes 24..31: the inclusive prefix, where most draws land) from 7
         // independent shuffles and an add tree: one shuffle latency on the
         // chain instead of the scan's three.  The windows beyond are added
-        // only if needed.
+        // only if needed (always: n=1000 195 -> 202 us).
         uint32_t u[8];
         u[0] = wv * own;
 #pragma unroll
         for (int o = 1; o < 8; ++o) u[o] = __shfl_down_sync(kFull, wv, o);
         uint32_t cum = ((u[1] + u[2]) + (u[3] + u[4])) + ((u[5] + u[6]) + (u[7] + u[0]));
-        unsigned msk = __ballot_sync(kFull, first8 && cum > thr);
-        if (msk == 0u) {
+        uint32_t first = __reduce_max_sync(kFull, first8 && cum > thr ? word : 0u);
+        if (first == 0u) {
           const uint32_t t8 = __shfl_down_sync(kFull, cum, 8);
           const uint32_t t16 = __shfl_down_sync(kFull, cum, 16);
           const uint32_t t24 = __shfl_down_sync(kFull, cum, 24);
           cum += (lane < 24 ? t8 : 0u) + (lane < 16 ? t16 : 0u) + (lane < 8 ? t24 : 0u);
-          msk = __ballot_sync(kFull, cum > thr);
-          if (msk == 0u) break;  // no eligible candidate has a weight
+          first = __reduce_max_sync(kFull, cum > thr ? word : 0u);
+          if (first == 0u) break;  // no eligible candidate has a weight
         }
-        const int src = 31 - __clz((int)msk);
-        const uint32_t nbase = __shfl_sync(kFull, cb, src);
-        const int next = __shfl_sync(kFull, c, src);
-        const uint32_t dn = __shfl_sync(kFull, e, src);
+        const int next = (int)(first & 0xffffu);
+        const uint32_t dn = E == 1 ? (first >> 16) & 0xffu : us.get(next);
         if (CREF && room <= close_room) {
           // The roulette draw is spent, and a second one decides.
           if (--left == 0) refill(d0 + 128u); else next_draw();
@@ -670,11 +685,8 @@ __device__ __forceinline__ void build_ant(const ConstructArgs &a, const Tables<L
             break;
           }
         }
-        take_step(next, nbase, dn);
-        // A draw is consumed only by a roulette selection.
-        --left;
-        next_draw();
-        e = us.get(c);
+        if (E != 1) __syncwarp();  // every lane has read the element that the step marks
+        take_step(next, dn, true);
       }
       if (!open || room <= floor_room) break;
       if (left == 0) {
@@ -691,8 +703,7 @@ __device__ __forceinline__ void build_ant(const ConstructArgs &a, const Tables<L
       if (nx <= 0) break;
       const uint32_t dnx = us.get(nx);
       __syncwarp();  // every lane has read the element that the step marks
-      take_step(nx, (uint32_t)nx * (uint32_t)k, dnx);
-      e = us.get(c);
+      take_step(nx, dnx, false);
     }
     rem_dem -= cap - room;
     if (lane == 0) {
