@@ -58,6 +58,13 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
          ((uint32_t)(M >> 4) << 24);
 }
 
+// The same tile read as its transpose (MN-major): bits 15 and 16 of the
+// instruction descriptor.  The core matrix is the same (8 rows of 16 bytes);
+// rows now run along K, so the descriptor's leading offset is the distance of
+// core matrices along the rows (128 bytes), its stride offset the one along
+// the columns, and a K step of 16 is two core matrices along the rows.
+constexpr uint32_t kTransposeA = 1u << 15, kTransposeB = 1u << 16;
+
 // D[tmem] (+)= A * B^T, issued by one thread.
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                          uint32_t idesc, uint32_t accumulate) {
