@@ -57,13 +57,14 @@ constexpr uint32_t kPolls = 1u << 24;
 // the weights): the products that need its transpose read it MN-major.  H1 and
 // the inputs are neighbours, and so are dZ2 and dZ1: each pair is one operand
 // of the weight-gradient product.  Transposed copies of H1, the inputs, dZ2,
-// dZ1 and W2 took 200 two-byte stores per edge and 30 KB more: 3.07 ms for 96
-// full-batch steps over 112,633 examples, 2.82 ms without them.
+// dZ1 and W2 took 200 two-byte stores per edge and 30 KB more: 3.07 ms for 56
+// steps of 4096 examples, 2.82 ms without them.
 constexpr uint32_t kSB1 = 0;                         // W1|b1   64 x 16
 constexpr uint32_t kSB2 = kSB1 + 64 * 16 * 2;         // W2      64 x 64 [o][j]
 constexpr uint32_t kSA2 = kSB2 + 64 * 64 * 2;         // H1      128 x 64
 constexpr uint32_t kSA1 = kSA2 + 128 * 64 * 2;        // X       128 x 16
-constexpr uint32_t kSdZ2 = kSA1 + 128 * 16 * 2;       // dZ2     128 x 64
+constexpr uint32_t kSHX = 128 * (64 + 16) * 2;         // H1 and X, of alternate tiles
+constexpr uint32_t kSdZ2 = kSA2 + 2 * kSHX;           // dZ2     128 x 64
 constexpr uint32_t kSdZ1 = kSdZ2 + 128 * 64 * 2;      // dZ1     128 x 64
 constexpr uint32_t kSF32 = kSdZ1 + 128 * 64 * 2;      // b2[64], w3[64]
 constexpr uint32_t kSRed = kSF32 + 128 * 4;           // 4 warps x 65 partial sums
@@ -296,11 +297,29 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
          ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi)) << 16);
 }
 
+// Four values of a table in shared memory, read where they are used: kept in
+// registers over the tiles, b2 and w3 alone would take 128 of them.
+__device__ __forceinline__ float4 lds4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr));
+  return v;
+}
+
+// The same value, as one that is not known to stay the same: what is computed
+// from it is computed where it is used, by the thread that issues the MMAs,
+// instead of in registers of every thread over the tiles.
+__device__ __forceinline__ uint32_t fresh(uint32_t v) {
+  asm volatile("" : "+r"(v));
+  return v;
+}
+
 template <bool TRAIN>
 __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char *sB1 = smem + kSB1, *sB2 = smem + kSB2;
-  unsigned char *sA1 = smem + kSA1, *sA2 = smem + kSA2, *sdZ2 = smem + kSdZ2, *sdZ1 = smem + kSdZ1;
+  unsigned char *sdZ2 = smem + kSdZ2, *sdZ1 = smem + kSdZ1;
   float *s_b2 = reinterpret_cast<float *>(smem + kSF32);
   float *s_w3 = s_b2 + 64;
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem + kSBar);
@@ -318,37 +337,60 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
     fence_mbar_init();
   }
   // Constant input 8 = 1 (layer-1 bias), inputs 9-15 = 0, for every edge.
-  *reinterpret_cast<uint4 *>(sA1 + umma::kmajor_offset(tid, 8, 128)) =
-      make_uint4(0x3F80u, 0u, 0u, 0u);
+#pragma unroll
+  for (int b = 0; b < 2; ++b)
+    *reinterpret_cast<uint4 *>(smem + kSA1 + b * kSHX + umma::kmajor_offset(tid, 8, 128)) =
+        make_uint4(0x3F80u, 0u, 0u, 0u);
   // The first tile's rows: features and examples are fixed, so they are on
   // their way before this launch waits for the parameters' update.
   int tile = blockIdx.x;
-  RowRef now = row_ref<TRAIN>(a, tile, warp), next = row_ref<TRAIN>(a, tile + gridDim.x, warp);
-  int kvr = now.live ? (int)a.kv[now.row] : 0;
-  uint4 fv = a.feat[now.row * kSlots + lane];
+  // now: the tile worked on; next: the one whose inputs are in fv (n_slots of
+  // them); after: where the rows of the one behind it are.
+  RowRef now = row_ref<TRAIN>(a, tile, warp), next = now;
+  RowRef after = row_ref<TRAIN>(a, tile + gridDim.x, warp);
+  int slots = 0, n_slots = next.live ? (int)a.kv[next.row] : 0;
+  uint4 fv = a.feat[next.row * kSlots + lane];
+  // The inputs of `next` into buffer b, and the request for those behind them.
+  auto take_inputs = [&](uint32_t b) {
+    *reinterpret_cast<uint4 *>(smem + kSA1 + b * kSHX + umma::kmajor_offset(tid, 0, 128)) =
+        next.live && lane < n_slots ? fv : make_uint4(0u, 0u, 0u, 0u);
+    now = next;
+    slots = n_slots;
+    next = after;
+    n_slots = next.live ? (int)a.kv[next.row] : 0;
+    fv = a.feat[next.row * kSlots + lane];
+  };
   wait_for_previous();
   // Weights into their operand layouts (BF16), 8 along K at a time (16-byte
-  // stores); biases of layers 2-3 in FP32.
+  // stores); biases of layers 2-3 in FP32.  All of them are asked for before
+  // the first store, which the loads behind it could not be moved ahead of.
   const float *P = a.params;
-  for (int e = tid; e < 64 * 16; e += 128) {
-    const int o = e >> 4, f = e & 15;
-    const float w = f < 8 ? P[kW1 + o * 8 + f] : (f == 8 ? P[kB1 + o] : 0.f);
-    st_bf16(sB1, umma::kmajor_offset(o, f, 64), w);
+  float w1[8];
+  float4 w2[4][2];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int o = (tid + 128 * i) >> 4, f = tid & 15;
+    w1[i] = f < 8 ? P[kW1 + o * 8 + f] : (f == 8 ? P[kB1 + o] : 0.f);
   }
 #pragma unroll
-  for (int e = tid; e < 64 * 8; e += 128) {
-    const int o = e >> 3, j = (e & 7) * 8;
-    const float4 lo = *reinterpret_cast<const float4 *>(P + kW2 + o * 64 + j);
-    const float4 hi = *reinterpret_cast<const float4 *>(P + kW2 + o * 64 + j + 4);
+  for (int i = 0; i < 4; ++i) {
+    const float4 *p = reinterpret_cast<const float4 *>(P + kW2) + 2 * (tid + 128 * i);
+    w2[i][0] = p[0];
+    w2[i][1] = p[1];
+  }
+  const float b2w3 = tid < 64 ? P[kB2 + tid] : P[kW3 + tid - 64], b3 = P[kB3];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    st_bf16(sB1, umma::kmajor_offset((tid + 128 * i) >> 4, tid & 15, 64), w1[i]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int o = (tid + 128 * i) >> 3, j = (tid & 7) * 8;
+    const float4 lo = w2[i][0], hi = w2[i][1];
     *reinterpret_cast<uint4 *>(sB2 + umma::kmajor_offset(o, j, 64)) =
         make_uint4(bf16_pair(lo.x, lo.y), bf16_pair(lo.z, lo.w), bf16_pair(hi.x, hi.y),
                    bf16_pair(hi.z, hi.w));
   }
-  if (tid < 64) {
-    s_b2[tid] = P[kB2 + tid];
-    s_w3[tid] = P[kW3 + tid];
-  }
-  const float b3 = P[kB3];
+  s_b2[tid] = b2w3;  // b2, then w3
   umma::fence_async_smem();
   umma::fence_before_sync();
   __syncthreads();
@@ -363,9 +405,10 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
   const uint32_t idesc64t = idesc64 | umma::kTransposeB;
   const uint32_t idesc80t =
       umma::idesc_bf16_f32(128, 80) | umma::kTransposeA | umma::kTransposeB;
-  const uint32_t aA1 = umma::smem_u32(sA1), aA2 = umma::smem_u32(sA2),
+  const uint32_t aA1 = umma::smem_u32(smem + kSA1), aA2 = umma::smem_u32(smem + kSA2),
                  adZ2 = umma::smem_u32(sdZ2), aB1 = umma::smem_u32(sB1),
-                 aB2 = umma::smem_u32(sB2);
+                 aB2 = umma::smem_u32(sB2), ab2 = umma::smem_u32(s_b2),
+                 aw3 = umma::smem_u32(s_w3);
 
   float acc_w3[64];
 #pragma unroll
@@ -375,73 +418,111 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
   bool ok = true;
   int done = 0;
 
-  for (; tile < a.tiles; tile += gridDim.x) {
-    const bool live = now.live, valid = live && lane < kvr;
-    const long long row = now.row;
-    const int tgt = now.tgt;
-    if (!valid) fv = make_uint4(0u, 0u, 0u, 0u);
-    *reinterpret_cast<uint4 *>(sA1 + umma::kmajor_offset(tid, 0, 128)) = fv;
-    // The next tile's rows while this one is worked on, and where the rows
-    // after those are.
-    now = next;
-    kvr = now.live ? (int)a.kv[now.row] : 0;
-    fv = a.feat[now.row * kSlots + lane];
-    next = row_ref<TRAIN>(a, tile + 2 * gridDim.x, warp);
+  // Z1 = X W1^T (+ b1 through the constant input)
+  auto issue_z1 = [&](uint32_t b) {
+    umma::mma_bf16(tm + kColZ1, umma::smem_desc(fresh(aA1 + b * kSHX), lbo128, 128),
+                   umma::smem_desc(fresh(aB1), lbo64, 128), idesc64, 0u);
+  };
+  // Every thread waits for the group committed last; a wait that gives up is
+  // noticed at the next barrier, which every thread still reaches.
+  auto wait_group = [&]() {
+    ok = mbar_wait_bounded(bar, phase, kPolls) && ok;
+    phase ^= 1u;
+    __syncwarp();
+    umma::fence_after_sync();
+  };
+  auto operands_ready = [&]() {
     umma::fence_async_smem();
     umma::fence_before_sync();
-    __syncthreads();
-    // Z1 = X W1^T (+ b1 through the constant input)
+    ok = __syncthreads_and(ok);
+    return ok;
+  };
+
+  // The tensor cores' work of a tile hides behind its neighbours': a commit
+  // covers every MMA that the thread issued before it.  Inference issues the next tile's Z1 with
+  // this tile's Z2 (one wait per tile); training issues it with dH1, and does
+  // not wait for dW, which ends before the next tile's Z2 (two waits per tile).
+  // A stage reads its accumulator in one go: sixteen loads of 16 columns with a
+  // wait behind each were most of a tile's latency (with four waits per tile
+  // 25.7 us for 4096 examples, now 22.8: 8 us in all for the launch, the
+  // weights and the partial sums, then 3.7 us for two tiles per SM, twice
+  // what their instructions take to issue).  Two threads per edge, each with
+  // half the units, took 26 us.
+  if (tile < a.tiles) {
+    take_inputs(0u);
+    after = row_ref<TRAIN>(a, tile + 2 * gridDim.x, warp);
+    operands_ready();
     if (tid == 0) {
       umma::fence_after_sync();
-      umma::mma_bf16(tm + kColZ1, umma::smem_desc(aA1, lbo128, 128),
-                     umma::smem_desc(aB1, lbo64, 128), idesc64, 0u);
+      issue_z1(0u);
       umma::commit(bar);
     }
-    ok = __syncthreads_and(mbar_wait_bounded(bar, phase, kPolls));
-    phase ^= 1u;
-    if (!ok) break;
-    umma::fence_after_sync();
+    wait_group();
+  }
+  for (; tile < a.tiles; tile += gridDim.x) {
+    const uint32_t buf = (uint32_t)done & 1u;
+    unsigned char *sA2 = smem + kSA2 + buf * kSHX;
+    const bool more = tile + (int)gridDim.x < a.tiles;
+    const bool live = now.live, valid = live && lane < slots;
+    const long long row = now.row;
+    const int tgt = now.tgt;
+    uint32_t pos_z1[2] = {0u, 0u};  // TRAIN: units with Z1 > 0
+    if (!TRAIN) {
+      take_inputs(buf ^ 1u);
+      after = row_ref<TRAIN>(a, tile + 3 * gridDim.x, warp);
+    }
     // H1 = relu(Z1) -> BF16 operand
+    float z[64];
+    umma::tmem_ld64(tl + kColZ1, z);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      float z[16];
-      umma::tmem_ld16(tl + kColZ1 + 16 * q, z);
-      umma::tmem_wait_ld();
       uint32_t w[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        w[i] = bf16_pair(fmaxf(z[2 * i], 0.f), fmaxf(z[2 * i + 1], 0.f));
+        const float lo = z[16 * q + 2 * i], hi = z[16 * q + 2 * i + 1];
+        w[i] = bf16_pair(fmaxf(lo, 0.f), fmaxf(hi, 0.f));
+        if (TRAIN) {
+          const int at = 16 * (q & 1) + 2 * i;
+          pos_z1[q >> 1] |= (lo > 0.f ? 1u << at : 0u) | (hi > 0.f ? 2u << at : 0u);
+        }
       }
       *reinterpret_cast<uint4 *>(sA2 + umma::kmajor_offset(tid, 16 * q, 128)) =
           make_uint4(w[0], w[1], w[2], w[3]);
       *reinterpret_cast<uint4 *>(sA2 + umma::kmajor_offset(tid, 16 * q + 8, 128)) =
           make_uint4(w[4], w[5], w[6], w[7]);
     }
-    umma::fence_async_smem();
-    umma::fence_before_sync();
-    __syncthreads();
+    if (!operands_ready()) break;
     // Z2 = H1 W2^T
     if (tid == 0) {
       umma::fence_after_sync();
+      const uint64_t da = umma::smem_desc(fresh(aA2 + buf * kSHX), lbo128, 128);
+      const uint64_t db = umma::smem_desc(fresh(aB2), lbo64, 128);
 #pragma unroll
       for (int s = 0; s < 4; ++s)
-        umma::mma_bf16(tm + kColZ2, umma::smem_desc(aA2 + 2 * s * lbo128, lbo128, 128),
-                       umma::smem_desc(aB2 + 2 * s * lbo64, lbo64, 128), idesc64, s > 0 ? 1u : 0u);
+        umma::mma_bf16(tm + kColZ2, da + 2 * s * (lbo128 >> 4), db + 2 * s * (lbo64 >> 4), idesc64,
+                       s > 0 ? 1u : 0u);
+      if (!TRAIN && more) issue_z1(buf ^ 1u);
       umma::commit(bar);
     }
-    ok = __syncthreads_and(mbar_wait_bounded(bar, phase, kPolls));
-    phase ^= 1u;
-    if (!ok) break;
-    umma::fence_after_sync();
+    wait_group();
+    if (TRAIN) {
+      take_inputs(buf ^ 1u);
+      after = row_ref<TRAIN>(a, tile + 3 * gridDim.x, warp);
+    }
     // s = b3 + w3 . relu(Z2 + b2)
     float sc = b3;
+    umma::tmem_ld64(tl + kColZ2, z);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float z[16];
-      umma::tmem_ld16(tl + kColZ2 + 16 * q, z);
-      umma::tmem_wait_ld();
-#pragma unroll
-      for (int i = 0; i < 16; ++i) sc += s_w3[16 * q + i] * fmaxf(z[i] + s_b2[16 * q + i], 0.f);
+    for (int j = 0; j < 64; j += 4) {
+      const float4 b2 = lds4(ab2 + 4 * j), w3 = lds4(aw3 + 4 * j);
+      z[j] = fmaxf(z[j] + b2.x, 0.f);
+      z[j + 1] = fmaxf(z[j + 1] + b2.y, 0.f);
+      z[j + 2] = fmaxf(z[j + 2] + b2.z, 0.f);
+      z[j + 3] = fmaxf(z[j + 3] + b2.w, 0.f);
+      sc += w3.x * z[j];
+      sc += w3.y * z[j + 1];
+      sc += w3.z * z[j + 2];
+      sc += w3.w * z[j + 3];
     }
     if (!TRAIN) {
       if (live) a.scores[row * kSlots + lane] = sc;
@@ -458,88 +539,79 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
       // dZ2 = g w3 relu'(Z2 + b2): operand of dH1 and of dW.
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        float z[16];
-        umma::tmem_ld16(tl + kColZ2 + 16 * q, z);
-        umma::tmem_wait_ld();
         uint32_t w[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float d2[2];
+        for (int i = 0; i < 8; i += 2) {
+          const int j = 16 * q + 2 * i;
+          const float4 w3 = lds4(aw3 + 4 * j);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int j = 16 * q + 2 * i + h;
-            const float h2 = z[2 * i + h] + s_b2[j];
-            acc_w3[j] += g * fmaxf(h2, 0.f);
-            d2[h] = h2 > 0.f ? g * s_w3[j] : 0.f;
-          }
-          w[i] = bf16_pair(d2[0], d2[1]);
+          for (int h = 0; h < 4; ++h) acc_w3[j + h] += g * z[j + h];
+          w[i] = bf16_pair(z[j] > 0.f ? g * w3.x : 0.f, z[j + 1] > 0.f ? g * w3.y : 0.f);
+          w[i + 1] = bf16_pair(z[j + 2] > 0.f ? g * w3.z : 0.f, z[j + 3] > 0.f ? g * w3.w : 0.f);
         }
         *reinterpret_cast<uint4 *>(sdZ2 + umma::kmajor_offset(tid, 16 * q, 128)) =
             make_uint4(w[0], w[1], w[2], w[3]);
         *reinterpret_cast<uint4 *>(sdZ2 + umma::kmajor_offset(tid, 16 * q + 8, 128)) =
             make_uint4(w[4], w[5], w[6], w[7]);
       }
-      umma::fence_async_smem();
-      umma::fence_before_sync();
-      __syncthreads();
+      if (!operands_ready()) break;
       // dH1 = dZ2 W2
       if (tid == 0) {
         umma::fence_after_sync();
+        const uint64_t da = umma::smem_desc(fresh(adZ2), lbo128, 128);
+        const uint64_t db = umma::smem_desc(fresh(aB2), 128, lbo64);
 #pragma unroll
         for (int s = 0; s < 4; ++s)
-          umma::mma_bf16(tm + kColDH1, umma::smem_desc(adZ2 + 2 * s * lbo128, lbo128, 128),
-                         umma::smem_desc(aB2 + 2 * s * 128, 128, lbo64), idesc64t,
-                         s > 0 ? 1u : 0u);
+          umma::mma_bf16(tm + kColDH1, da + 2 * s * (lbo128 >> 4), db + 2 * s * (128 >> 4),
+                         idesc64t, s > 0 ? 1u : 0u);
+        if (more) issue_z1(buf ^ 1u);
         umma::commit(bar);
       }
-      ok = __syncthreads_and(mbar_wait_bounded(bar, phase, kPolls));
-      phase ^= 1u;
-      if (!ok) break;
-      umma::fence_after_sync();
+      wait_group();
       // dZ1 = dH1 relu'(Z1)
+      umma::tmem_ld64(tl + kColDH1, z);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        float dh[16], z[16];
-        umma::tmem_ld16(tl + kColDH1 + 16 * q, dh);
-        umma::tmem_ld16(tl + kColZ1 + 16 * q, z);
-        umma::tmem_wait_ld();
         uint32_t w[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-          w[i] = bf16_pair(z[2 * i] > 0.f ? dh[2 * i] : 0.f,
-                           z[2 * i + 1] > 0.f ? dh[2 * i + 1] : 0.f);
+        for (int i = 0; i < 8; ++i) {
+          const uint32_t m = pos_z1[q >> 1] >> (16 * (q & 1) + 2 * i);
+          w[i] = bf16_pair(m & 1u ? z[16 * q + 2 * i] : 0.f,
+                           m & 2u ? z[16 * q + 2 * i + 1] : 0.f);
+        }
         *reinterpret_cast<uint4 *>(sdZ1 + umma::kmajor_offset(tid, 16 * q, 128)) =
             make_uint4(w[0], w[1], w[2], w[3]);
         *reinterpret_cast<uint4 *>(sdZ1 + umma::kmajor_offset(tid, 16 * q + 8, 128)) =
             make_uint4(w[4], w[5], w[6], w[7]);
       }
-      umma::fence_async_smem();
-      umma::fence_before_sync();
-      __syncthreads();
+      if (!operands_ready()) break;
       // dW += [dZ2 dZ1]^T [H1 X], accumulated over this block's tiles
       if (tid == 0) {
         umma::fence_after_sync();
+        const uint64_t da = umma::smem_desc(fresh(adZ2), 128, lbo128);
+        const uint64_t db = umma::smem_desc(fresh(aA2 + buf * kSHX), 128, lbo128);
 #pragma unroll
         for (int s = 0; s < 8; ++s)
-          umma::mma_bf16(tm + kColDW, umma::smem_desc(adZ2 + 2 * s * 128, 128, lbo128),
-                         umma::smem_desc(aA2 + 2 * s * 128, 128, lbo128), idesc80t,
+          umma::mma_bf16(tm + kColDW, da + 2 * s * (128 >> 4), db + 2 * s * (128 >> 4), idesc80t,
                          (done > 0 || s > 0) ? 1u : 0u);
-        umma::commit(bar);
       }
-      ok = __syncthreads_and(mbar_wait_bounded(bar, phase, kPolls));
-      phase ^= 1u;
-      if (!ok) break;
-      umma::fence_after_sync();
     }
     ++done;
-    umma::fence_before_sync();
-    __syncthreads();
   }
+  if (TRAIN && ok && done > 0) {
+    if (tid == 0) umma::commit(bar);
+    wait_group();
+  }
+  umma::fence_before_sync();
+  ok = __syncthreads_and(ok);
+  umma::fence_after_sync();
 
   if (!ok) {
-    // A wait gave up: wait (bounded) for the group still in flight before
-    // the tensor memory is released.
+    // A wait gave up: wait (bounded) for the group still in flight, and for
+    // what was issued behind it, before the tensor memory is released.
     mbar_wait_bounded(bar, phase ^ 1u, kPolls);
+    if (tid == 0) umma::commit(bar);
+    mbar_wait_bounded(bar, phase, kPolls);
     if (tid == 0) atomicOr(a.error, kErrStageTimeout);
   } else if (TRAIN && done > 0) {
     // This block's partial gradient, row blockIdx.x of gpart (summed in a
@@ -607,27 +679,38 @@ __global__ void __launch_bounds__(128, 2) k_prior_mlp(MlpArgs a) {
 
 // Sum of the blocks' partial gradients in block order, into grad or (params
 // given) taken as Adam's step; the loss goes to *loss.  A block takes 32
-// parameters: all its threads bring the rows' values to shared memory at once,
-// one warp adds them in order, so that training stays bit-reproducible.  (One
-// thread per parameter loading row after row, and the step in a launch of its
-// own, took 15 + 4 us behind every 48 us of gradients.)
+// parameters: all its threads bring the rows' values to shared memory at once
+// by asynchronous copies, one warp adds them in order, so that training stays
+// bit-reproducible.  It is bound by the latency of those copies and of the
+// 296 dependent adds: 5.8 us (9.4 with 16 loads in flight per thread and the
+// moments asked for behind the sum; one thread per parameter loading row after
+// row, and the step in a launch of its own, took 15 + 4 us).
 constexpr int kReduceThreads = 256;
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 __global__ void __launch_bounds__(kReduceThreads)
     k_prior_reduce(const float *gpart, int blocks, float *grad, float *loss, float *params,
                    float *m, float *v, float lr, float bc1, float bc2) {
-  extern __shared__ float s_part[];  // [blocks][32]
+  extern __shared__ __align__(16) float s_part[];  // [blocks][32]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
   let_next_start();
   wait_for_previous();
-  if (i <= kParams) {
-#pragma unroll 16
-    for (int r = warp; r < blocks; r += kReduceThreads / 32)
-      s_part[r * 32 + lane] = gpart[(size_t)r * kGradStride + i];
+  for (int e = threadIdx.x; e < blocks * 8; e += kReduceThreads) {
+    const int r = e >> 3, col = blockIdx.x * 32 + 4 * (e & 7);
+    if (col < kGradStride)
+      cp_async16(smem_addr(s_part + r * 32 + 4 * (e & 7)), gpart + (size_t)r * kGradStride + col);
   }
+  const bool mine = warp == 0 && i <= kParams;
+  const bool step = mine && i < kParams && params;
+  const float m0 = step ? m[i] : 0.f, v0 = step ? v[i] : 0.f, p0 = step ? params[i] : 0.f;
+  cp_async_wait();
   __syncthreads();
-  if (warp != 0 || i > kParams) return;
+  if (!mine) return;
   float g = 0.f;
 #pragma unroll 16
   for (int r = 0; r < blocks; ++r) g += s_part[r * 32 + lane];
@@ -639,11 +722,11 @@ __global__ void __launch_bounds__(kReduceThreads)
     grad[i] = g;
     return;
   }
-  const float mi = 0.9f * m[i] + 0.1f * g;
-  const float vi = 0.999f * v[i] + 0.001f * g * g;
+  const float mi = 0.9f * m0 + 0.1f * g;
+  const float vi = 0.999f * v0 + 0.001f * g * g;
   m[i] = mi;
   v[i] = vi;
-  params[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + 1e-8f);
+  params[i] = p0 - lr * (mi / bc1) / (sqrtf(vi / bc2) + 1e-8f);
 }
 
 // Levels from scores: warp per row, L = min(4095, round(scale (s_max - s))).
@@ -1149,7 +1232,7 @@ static int run_gradient(aco_b200_prior *p, const int *order, int count, int step
   a.gpart = p->d_gpart;
   a.error = p->d_error;
   a.tiles = (count + 3) / 4;
-  // Two training blocks per SM (256 tensor-memory columns and 64 KB of shared
+  // Two training blocks per SM (256 tensor-memory columns and 84 KB of shared
   // memory each): one block's MMA runs while the other's epilogue does.
   const int grid = std::max(1, std::min(a.tiles, p->num_sms * 2));
   if (first) {
