@@ -105,9 +105,11 @@ struct aco_b200_ctx {
   // (1.2 ms, and 0.4 ms to free) than it saves over a context's copies.
   DevState h_state = {};
   // h_state is what the device holds.  Not after launches that run() does not
-  // wait for; never between split-colony calls and the next set-up (a caller
-  // may replay those from a graph of its own).
-  bool state_known = false, split = false;
+  // wait for, and never while recordings of split-colony calls may be about: a
+  // caller replays those without a call of this library, after a set-up too,
+  // until the generation they were made in is over (split_gen: the last one).
+  bool state_known = false;
+  int split_gen = 0;
   int log_read = 0;
 
   InstanceView iv = {};
@@ -119,6 +121,7 @@ struct aco_b200_ctx {
   cudaGraphExec_t graphs[kGraphs] = {};  // of kGraphEpochs epochs, made when first needed
   double table_key[3] = {};              // alpha, beta, level step of A and thr
   int graph_gen = 1;  // changes whenever the captured launch arguments may have
+  bool may_be_replayed() const { return split_gen == graph_gen; }
   bool run_limit_off = false;  // device run limit known to be disabled
   int depot_rule = 0;
   int inject_alloc = 0;  // test hook: the n-th device allocation of a set-up fails
@@ -558,8 +561,6 @@ int aco_b200_setup(aco_b200_ctx *ctx, const aco_b200_problem *p) {
 
   TRY(cudaStreamSynchronize(s));
   ctx->log_read = 0;
-  ctx->state_known = true;
-  ctx->split = false;
   ctx->run_limit_off = true;  // fresh state: run_limit = 0
   unsigned char key[sizeof(ctx->graph_key)];
   memset(key, 0, sizeof(key));
@@ -569,6 +570,7 @@ int aco_b200_setup(aco_b200_ctx *ctx, const aco_b200_problem *p) {
     memcpy(ctx->graph_key, key, sizeof(key));
     ++ctx->graph_gen;
   }
+  ctx->state_known = !ctx->may_be_replayed();
   ctx->ready = true;
   return ACO_OK;
 }
@@ -654,7 +656,7 @@ int aco_b200_run(aco_b200_ctx *ctx, int max_epochs, aco_b200_state *state,
     const int rc = launch_epochs(ctx, std::min(left, kMaxAhead));
     if (rc) return rc;
   }
-  ctx->state_known = !ctx->split;
+  ctx->state_known = !ctx->may_be_replayed();
   if (state) fill_state(state, ctx->h_state);
   if (n_records) *n_records = nrec;
   return ACO_OK;
@@ -743,7 +745,7 @@ int aco_b200_shard_construct(aco_b200_ctx *ctx, int32_t *d_send) {
   if (!ctx || !ctx->ready || !d_send) return ACO_ERR_INVALID_INPUT;
   cudaSetDevice(ctx->device);
   ctx->state_known = false;
-  ctx->split = true;
+  ctx->split_gen = ctx->graph_gen;
   cudaStream_t s = ctx->stream;
   if (!ctx->run_limit_off) {
     TRY(launch_set_run_limit(ctx->d_state, 0, s));
@@ -766,7 +768,7 @@ int aco_b200_shard_update(aco_b200_ctx *ctx, const int32_t *d_recv, int world) {
   if (!ctx || !ctx->ready || !d_recv || world < 1) return ACO_ERR_INVALID_INPUT;
   cudaSetDevice(ctx->device);
   ctx->state_known = false;
-  ctx->split = true;
+  ctx->split_gen = ctx->graph_gen;
   cudaStream_t s = ctx->stream;
   TRY(launch_shard_select(ctx->iv, ctx->d_state, d_recv, world, ctx->d_iter_nodes,
                           ctx->d_iter_lens, ctx->d_gbest_nodes, ctx->d_gbest_lens, ctx->d_log,
