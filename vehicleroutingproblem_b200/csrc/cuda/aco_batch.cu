@@ -469,7 +469,10 @@ __device__ __forceinline__ void build_ants(const BatchArgs &a, const BatchShape 
       // The nearest eligible customer (the rule of nearest_eligible in
       // aco_kernels.cu), one ant after another by the whole warp.  An
       // eligible candidate whose weight is 0 would come before the tier row:
-      // an ant that has one is left to the scan.
+      // an ant that has one is left to the scan.  The other ants' lanes read
+      // elements that this ant's lanes marked in earlier steps, and neither
+      // shuffles nor ballots order memory.
+      __syncwarp();
       const unsigned zero = __ballot_sync(
           kFull, e[0] <= lim || e[1] <= lim || e[2] <= lim || e[3] <= lim);
       do {
@@ -514,10 +517,10 @@ __device__ __forceinline__ void build_ants(const BatchArgs &a, const BatchShape 
   }
 
   if (valid && l < (pos & (LPA - 1))) route[(pos & ~(LPA - 1)) + l] = held;
+  __syncwarp();  // routes, lengths and elements before other lanes read them
   int left = valid ? n - (pos - 2 * K) : 0;
   unsigned rm = __ballot_sync(kFull, left > 0 && l == 0);
   if (rm) {
-    __syncwarp();
     int *scratch = reinterpret_cast<int *>(smem + sh.off_red) + 32 * warp;
     do {
       const int b = __ffs(rm) - 1;
