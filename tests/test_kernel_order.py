@@ -39,3 +39,15 @@ def test_batch_cost_reads_routes_after_a_warp_barrier():
     unconditional = stores_to_loads.split("if (rm)")[0]
     assert "__syncwarp()" in unconditional
     assert "__syncwarp()" in _between(stores_to_loads, "left -= added;", "} while (rm);")
+
+
+def test_construction_reads_the_epochs_weights_coherently():
+    """The construction's blocks start while k_weights still writes the
+    epoch's tables; the read-only path (__ldg) is for what no epoch writes."""
+    with open(os.path.join(CUDA, "aco_kernels.cu")) as f:
+        text = "".join(line.split("//")[0] for line in f)
+    weight = _between(text, "uint32_t weight(uint32_t nb) const {", "}")
+    assert "w[nb * step]" in weight and "__ldg" not in weight
+    build = _function("aco_kernels.cu", "build_ant") + _function("aco_kernels.cu", "k_construct")
+    for written in ("et.w", "et.rel", "et.rdep"):
+        assert written in build and f"__ldg(a.{written}" not in build

@@ -337,7 +337,8 @@ struct Tables {
   }
   __device__ __forceinline__ uint32_t weight(uint32_t nb) const {
     if (L == kLayoutSmemPacked) return lut[rel[nb * step]];
-    if (L == kLayoutGlobal) return __ldg(w + nb * step);
+    // Not the read-only path: k_weights writes them while blocks of this
+    // launch are there already.
     return w[nb * step];
   }
   __device__ __forceinline__ float2 coord(int node) const {
