@@ -294,16 +294,17 @@ extern "C" ACO_API int aco_b200_seq_pheromone_update(
   unsigned long long g = (pairs + per_block - 1) / per_block;
   if (g < 1) g = 1;
   // The arc kernels: one arc per thread (a solution has n + K arcs at most).
-  // Both solutions' offsets fit the default 48 KB of shared memory up to 6143
-  // routes.
   const int one = (n + K + kArcThreads - 1) / kArcThreads, two = 2 * one;
+  // Both solutions' offsets fit the default 48 KB of shared memory up to 6143
+  // routes.  Beyond, the kernels' limit is always raised to the same value: it
+  // is the function's, not the launch's, and threads with fewer routes must not
+  // lower it for the others.
   cudaError_t e = cudaSuccess;
   if (2 * smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(k_seq_mark, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(2 * smem));
+    constexpr int kMost = 2 * (int)sizeof(int) * (kSeqMaxRoutes + 1);
+    e = cudaFuncSetAttribute(k_seq_mark, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_seq_clamp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(2 * smem));
+      e = cudaFuncSetAttribute(k_seq_clamp, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
   }
   if (e == cudaSuccess) {
     k_seq_mark<<<two, kArcThreads, 2 * smem, s>>>(a);
