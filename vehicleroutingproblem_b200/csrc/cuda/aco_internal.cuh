@@ -100,7 +100,7 @@ struct SmemPlan {
   uint32_t bytes_cand, bytes_w, bytes_coords;
   uint32_t total;
   uint32_t vis_bytes;      // one ant's elements (see Unserved)
-  int elem;                // bytes per element; 0: one bit, demands in global memory
+  int elem;                // bytes per element, kElemBits or kElemUnitBits
   int wpb;                 // warps (ants) per block
   int layout;
   uint32_t off_route;      // route_smem: each ant's route (route_stride ints) in shared memory
@@ -139,10 +139,15 @@ struct InstanceView {
 inline int demand_bytes(int max_demand) {
   return max_demand < 0xff ? 1 : (max_demand < 0xffff ? 2 : 4);
 }
-// Bytes of one ant's elements (elem = 0: its bitmap), whole 16-byte pieces.
+// In place of a size: one bit per node, demands in global memory or all 1.
+constexpr int kElemBits = 0, kElemUnitBits = 3;
+__host__ __device__ constexpr bool elem_is_bits(int elem) {
+  return elem == kElemBits || elem == kElemUnitBits;
+}
+// Bytes of one ant's elements or bitmap, whole 16-byte pieces.
 inline uint32_t unserved_bytes(int n, int elem) {
   const uint32_t rows = (uint32_t)n + 1u;
-  const uint32_t b = elem ? rows * (uint32_t)elem : (rows + 31u) / 32u * 4u;
+  const uint32_t b = elem_is_bits(elem) ? (rows + 31u) / 32u * 4u : rows * (uint32_t)elem;
   return (b + 15u) & ~15u;
 }
 
@@ -467,9 +472,10 @@ __device__ inline unsigned long long warp_knn(const float2 *coords, int n, int k
 // load and one compare against the room left answer "unvisited and fits",
 // one store marks a visit, and the loaded element is the demand the step
 // needs.  E = 1, 2 or 4 bytes, the smallest that holds every demand below
-// that largest value; E = 0: a bitmap (word wi holding nodes 32 wi .. 32 wi
-// + 31) with the demands in global memory, for instances whose elements do
-// not fit beside the other ants of the block.
+// that largest value; E = kElemBits: a bitmap (word wi holding nodes 32 wi ..
+// 32 wi + 31) with the demands in global memory, for instances whose elements
+// do not fit beside the other ants of the block; E = kElemUnitBits: the same
+// where every demand is 1 and none is read.
 //
 // The elements replace a bitmap in registers read by a shuffle: that took a
 // shuffle, the bit's forming and testing, a second load for the demand and a
@@ -479,7 +485,7 @@ struct Unserved {
   static constexpr uint32_t kVisited = E == 1 ? 0xffu : (E == 2 ? 0xffffu : 0xffffffffu);
   uint32_t base;     // shared address of this ant's elements
   uint32_t chunks;   // 16-byte pieces
-  const int *dem;    // E = 0
+  const int *dem;    // E = kElemBits
 
   // The accesses are volatile so that they keep their order: a visit's store
   // comes before the next step's loads.
@@ -492,7 +498,7 @@ struct Unserved {
     } else if (E == 4) {
       asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(base + 4u * (uint32_t)node));
     } else {
-      const uint32_t d = (uint32_t)__ldg(dem + node);
+      const uint32_t d = E == kElemBits ? (uint32_t)__ldg(dem + node) : 1u;
       asm volatile("ld.shared.u32 %0, [%1];"
                    : "=r"(v) : "r"(base + 4u * ((uint32_t)node >> 5)));
       v = (__funnelshift_r(v, v, node) & 1u) ? kVisited : d;
@@ -517,7 +523,7 @@ struct Unserved {
     } else {
       uint32_t v;
       asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(base + 4u * ((uint32_t)q >> 4)));
-      const int2 d = __ldg(reinterpret_cast<const int2 *>(dem) + q);
+      const int2 d = E == kElemBits ? __ldg(reinterpret_cast<const int2 *>(dem) + q) : make_int2(1, 1);
       v >>= (2 * q) & 31;
       e0 = (v & 1u) ? kVisited : (uint32_t)d.x;
       e1 = (v & 2u) ? kVisited : (uint32_t)d.y;
@@ -542,8 +548,8 @@ struct Unserved {
   __device__ __forceinline__ uint32_t limit(int room) const {
     return (E == 1 || E == 2) ? min((uint32_t)room, kVisited - 1u) : (uint32_t)room;
   }
-  // E = 0: the bitmap of an unserved instance (by one warp); the elements
-  // are copied from iv.elems.
+  // The bitmap of an unserved instance (by one warp); elements are copied from
+  // iv.elems.
   __device__ __forceinline__ void init_bits(int n, int lane) {
     for (uint32_t wi = (uint32_t)lane; wi < 4u * chunks; wi += 32u) {
       const int lo = (int)wi << 5, valid = n + 1 - lo;  // nodes lo..n in this word

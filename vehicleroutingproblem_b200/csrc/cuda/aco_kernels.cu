@@ -855,7 +855,8 @@ __global__ void __launch_bounds__(512, 1) k_construct(const __grid_constant__ Co
   // Staging by bulk copies: the tables that no epoch changes and every ant's
   // elements on the first barrier, before this launch waits for the kernel
   // that makes the weights; the weights on the second one.
-  constexpr bool kFixed = L != kLayoutGlobal || E > 0, kWeights = L != kLayoutGlobal;
+  constexpr bool kElems = !elem_is_bits(E);
+  constexpr bool kFixed = L != kLayoutGlobal || kElems, kWeights = L != kLayoutGlobal;
   const uint32_t kChunk = 32768u;
   auto issue = [&](unsigned char *dst, const void *src, uint32_t bytes, uint64_t *on) {
     const unsigned char *sp = reinterpret_cast<const unsigned char *>(src);
@@ -871,9 +872,9 @@ __global__ void __launch_bounds__(512, 1) k_construct(const __grid_constant__ Co
     reinterpret_cast<uint32_t *>(smem)[4] = 0u;
     reinterpret_cast<uint32_t *>(smem)[5] = kRelMax;  // packed levels: weight 0
     const uint32_t ants = blockDim.x >> 5;
-    mbar_arrive_expect_tx(bar, pl.bytes_cand + pl.bytes_coords + (E > 0 ? ants * pl.vis_bytes : 0u) +
+    mbar_arrive_expect_tx(bar, pl.bytes_cand + pl.bytes_coords + (kElems ? ants * pl.vis_bytes : 0u) +
                                    (uint32_t)iv.stage_extra_tx);
-    if (E > 0)
+    if (kElems)
       for (uint32_t i = 0; i < ants; ++i)
         issue(smem + pl.off_vis + i * pl.vis_bytes, iv.elems, pl.vis_bytes, bar);
     if (L != kLayoutGlobal) {
@@ -887,7 +888,7 @@ __global__ void __launch_bounds__(512, 1) k_construct(const __grid_constant__ Co
   us.base = smem_addr(smem + pl.off_vis + (size_t)warp * pl.vis_bytes);
   us.chunks = pl.vis_bytes / 16u;
   us.dem = iv.demand;
-  if (E == 0) us.init_bits(iv.n, lane);
+  if (!kElems) us.init_bits(iv.n, lane);
 
   wait_for_previous();
   // Graph replays read the epoch number and the seed from the device state,
@@ -965,7 +966,7 @@ SmemPlan plan_construct(const InstanceView &iv, int layout, int num_sms,
   int wpb = (iv.m + num_sms - 1) / num_sms;
   if (wpb < 1) wpb = 1;
   if (wpb > 16) wpb = 16;
-  const int elem = demand_bytes(iv.max_demand);
+  const int elem = demand_bytes(iv.max_demand), bit = iv.unit ? kElemUnitBits : kElemBits;
   auto finish = [&](int lay, int el, int ants) {
     p.layout = lay;
     p.elem = el;
@@ -1004,17 +1005,36 @@ SmemPlan plan_construct(const InstanceView &iv, int layout, int num_sms,
     }
     return (int)p.total <= max_smem;
   };
-  // Rows from global memory with more ants per block than their elements
-  // leave room for: the bitmaps (1/8 byte per node) instead.
-  auto finish_global = [&]() { return finish(kLayoutGlobal, elem, wpb) || finish(kLayoutGlobal, 0, wpb); };
+  // With more ants per block than their elements leave room for, bitmaps (1/8
+  // byte per node) instead.
+  auto fits = [&](int lay, int ants) { return finish(lay, elem, ants) || finish(lay, bit, ants); };
+  // Packed levels with bitmaps come before rows from global memory with
+  // elements where the demands, then read through what is left of L1 (24 KB),
+  // fit there, and up to 12 ants per block: beyond, the bitmaps' bits cost more
+  // to form than the rows' way takes (construction, packed | global: n=2000
+  // demands to 1000, 7 ants 625 | 723 us, 11 693 | 721, 16 787 | 774; n=5000
+  // k=12, 4 ants 1695 | 1845; n=7000 k=8 2443 | 2414).  Unit demands are not
+  // read: n=2000, 16 ants 579 | 651, n=6900 k=8, 4 ants 1494 | 2278.
+  const bool bits = iv.unit || (wpb <= 12 && rows <= 6144);
+  auto packed_or_global = [&]() {
+    if (!finish(kLayoutSmemPacked, elem, wpb) && !(bits && finish(kLayoutSmemPacked, bit, wpb)))
+      fits(kLayoutGlobal, wpb);
+  };
   if (layout == kLayoutGlobal) {
-    finish_global();
+    fits(kLayoutGlobal, wpb);
   } else if (layout >= 0) {
-    // An explicit layout: fewer ants per block where all of them do not fit.
+    // A forced layout: fewer ants per block where not all of them fit.  A
+    // unit-demand instance whose tables and draws fit while the one ant's
+    // bitmap is up to 300 bytes too much is built with the next layout (the
+    // routes are the same) rather than refused.
     int ants = wpb;
-    while (!finish(layout, elem, ants) && ants > 1) --ants;
-  } else if (!finish(kLayoutSmemWeights, elem, wpb) && !finish(kLayoutSmemPacked, elem, wpb)) {
-    finish_global();
+    while (!fits(layout, ants) && ants > 1) --ants;
+    const size_t words = rows > 2048 ? (rows + 31) / 32 : 0;
+    if ((int)p.total > max_smem && wpb == 1 && iv.unit &&
+        p.off_draw + 512u - 16u + 4u * words <= (size_t)max_smem)
+      packed_or_global();
+  } else if (!finish(kLayoutSmemWeights, elem, wpb)) {
+    packed_or_global();
   }
   return p;
 }
@@ -1035,6 +1055,8 @@ static cudaError_t configure_l() {
   cudaError_t e = configure_t<L, 1>();
   if (e == cudaSuccess) e = configure_t<L, 2>();
   if (e == cudaSuccess) e = configure_t<L, 4>();
+  if (e == cudaSuccess) e = configure_t<L, kElemBits>();
+  if (e == cudaSuccess) e = configure_t<L, kElemUnitBits>();
   return e;
 }
 
@@ -1044,7 +1066,6 @@ cudaError_t prepare_construct_kernels() {
   cudaError_t e = configure_l<kLayoutSmemWeights>();
   if (e == cudaSuccess) e = configure_l<kLayoutSmemPacked>();
   if (e == cudaSuccess) e = configure_l<kLayoutGlobal>();
-  if (e == cudaSuccess) e = configure_t<kLayoutGlobal, 0>();
   return e;
 }
 
@@ -1065,6 +1086,8 @@ static cudaError_t launch_construct_l(const ConstructArgs &a, cudaStream_t s) {
     case 1: return launch_construct_le<L, 1>(a, s);
     case 2: return launch_construct_le<L, 2>(a, s);
     case 4: return launch_construct_le<L, 4>(a, s);
+    case kElemBits: return launch_construct_le<L, kElemBits>(a, s);
+    case kElemUnitBits: return launch_construct_le<L, kElemUnitBits>(a, s);
   }
   return cudaErrorInvalidValue;
 }
@@ -1091,9 +1114,7 @@ cudaError_t launch_construct(const InstanceView &iv, const EpochTables &et,
   switch (plan.layout) {
     case kLayoutSmemWeights: return launch_construct_l<kLayoutSmemWeights>(a, s);
     case kLayoutSmemPacked: return launch_construct_l<kLayoutSmemPacked>(a, s);
-    case kLayoutGlobal:
-      return plan.elem ? launch_construct_l<kLayoutGlobal>(a, s)
-                       : launch_construct_le<kLayoutGlobal, 0>(a, s);
+    case kLayoutGlobal: return launch_construct_l<kLayoutGlobal>(a, s);
   }
   return cudaErrorInvalidValue;
 }
