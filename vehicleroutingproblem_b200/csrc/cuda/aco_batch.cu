@@ -89,7 +89,8 @@ struct BatchShape {
   int lpa, S, elem, threads, round;
   int tau_smem;              // levels in shared memory (else BatchArgs::tau)
   uint32_t off_lut, off_cand, off_w, off_coords, off_tau, off_el0, off_el, off_draw, off_red;
-  uint32_t el_bytes;         // one ant's elements
+  uint32_t el_bytes;         // one ant's elements or bitmap
+  uint32_t el0_bytes;        // the elements of an unserved instance; with bitmaps, the demands
   uint32_t total;
 };
 
@@ -103,6 +104,7 @@ BatchShape batch_shape(int max_rows, int max_n, int k, int m, int elem, int roun
   if (s.threads < 128) s.threads = 128;
   s.tau_smem = tau_smem ? 1 : 0;
   s.el_bytes = unserved_bytes(max_n, elem);
+  s.el0_bytes = elem_is_bits(elem) ? unserved_bytes(max_n, 4) : s.el_bytes;
   const uint32_t r = (uint32_t)max_rows, S = (uint32_t)s.S;
   uint32_t o = 16;  // zeros, for lanes without candidates
   o += 1024;        // tau levels
@@ -111,7 +113,7 @@ BatchShape batch_shape(int max_rows, int max_n, int k, int m, int elem, int roun
   s.off_w = o; o += r * S * 4;
   s.off_coords = o; o += pad16u(r * 8);
   s.off_tau = o; o += tau_smem ? pad16u(r * S * 2) : 0u;
-  s.off_el0 = o; o += s.el_bytes;
+  s.off_el0 = o; o += s.el0_bytes;
   s.off_el = o; o += (uint32_t)round * s.el_bytes;
   s.off_draw = o; o += (uint32_t)round * 32u * (uint32_t)s.lpa;
   // per warp: 32 words of scratch; then the reductions
@@ -140,12 +142,8 @@ constexpr int kBatchTierMinCustomers = 128;
 // Nearest eligible customer of one ant by the scan of every node, made by the
 // whole warp (all arguments but lane are the warp's).  0 if none.
 template <int E>
-__device__ __noinline__ int coop_scan(const float2 *coords, uint32_t el_base, int n, int cur,
+__device__ __noinline__ int coop_scan(const float2 *coords, Unserved<E> us, int n, int cur,
                                       uint32_t lim, int lane) {
-  Unserved<E> us;
-  us.base = el_base;
-  us.chunks = 0;
-  us.dem = nullptr;
   uint32_t best_h;
   const float2 pc = coords[cur];
   const uint32_t best_n = scan_pairs<false, E, 2>(coords, us, n, pc, lim, lane, &best_h);
@@ -158,11 +156,7 @@ __device__ __noinline__ int coop_scan(const float2 *coords, uint32_t el_base, in
 // when the row lists every remaining customer and none is eligible, -1 when
 // it is full and none is.
 template <int E>
-__device__ __forceinline__ int coop_tier(uint32_t two, uint32_t el_base, uint32_t lim) {
-  Unserved<E> us;
-  us.base = el_base;
-  us.chunks = 0;
-  us.dem = nullptr;
+__device__ __forceinline__ int coop_tier(uint32_t two, const Unserved<E> &us, uint32_t lim) {
   const int n0 = (int)(two & 0xffffu), n1 = (int)(two >> 16);
   const bool ok0 = us.get(n0) <= lim, ok1 = us.get(n1) <= lim;
   const unsigned m = __ballot_sync(kFull, ok0 || ok1);
@@ -178,14 +172,10 @@ __device__ __forceinline__ int coop_tier(uint32_t two, uint32_t el_base, uint32_
 // added.  With at most 32 of them each lane holds one (ascending), and no
 // search looks at another node.
 template <int E>
-__device__ __noinline__ int coop_repair(const float2 *coords, uint32_t el_base, int n, int K,
+__device__ __noinline__ int coop_repair(const float2 *coords, Unserved<E> us, int n, int K,
                                         int cap, int pos, int left, int *route, int *lens,
                                         const int *loads, const int *last, int *rep,
                                         int *scratch, int lane) {
-  Unserved<E> us;
-  us.base = el_base;
-  us.chunks = 0;
-  us.dem = nullptr;
   const bool few = left <= 32;
   int mine = 0;
   uint32_t mdem = Unserved<E>::kVisited;
@@ -233,7 +223,7 @@ __device__ __noinline__ int coop_repair(const float2 *coords, uint32_t el_base, 
           dn = __shfl_sync(kFull, mdem, src);
           if (lane == src) mdem = Unserved<E>::kVisited;
         } else {
-          next = coop_scan<E>(coords, el_base, n, cur, lim, lane);
+          next = coop_scan<E>(coords, us, n, cur, lim, lane);
           if (next <= 0) break;
           dn = us.get(next);
           __syncwarp();
@@ -344,13 +334,16 @@ __device__ __forceinline__ void build_ants(const BatchArgs &a, const BatchShape 
   int *last = a.last + I.lens_off + (long long)use * K;
   Unserved<E> us;
   us.base = smem_addr(smem + sh.off_el) + (uint32_t)(valid ? slot : 0) * sh.el_bytes;
-  us.chunks = 0;
+  us.chunks = sh.el_bytes / 16u;
   us.dem = nullptr;
+  us.dem_s = smem_addr(smem + sh.off_el0);
+  constexpr bool kBits = elem_is_bits(E);
   const uint32_t ring = smem_addr(smem + sh.off_draw) + (uint32_t)(valid ? slot : 0) * 32u * LPA;
   // The elements from the instance's, and the first draws.
   if (valid) {
     const uint32_t src = smem_addr(smem + sh.off_el0);
-    for (uint32_t o = 16u * (uint32_t)l; o < sh.el_bytes; o += 16u * LPA) {
+    if (kBits) us.init_bits(n, l, LPA);
+    for (uint32_t o = 16u * (uint32_t)l; !kBits && o < sh.el_bytes; o += 16u * LPA) {
       uint32_t x[4];
       asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                    : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(src + o));
@@ -454,7 +447,7 @@ __device__ __forceinline__ void build_ants(const BatchArgs &a, const BatchShape 
     const int src = 31 - __clz((int)msk);
     int next;
     uint32_t dn;
-    if (E == 4) {
+    if (E == 4 || kBits) {
       next = (int)__shfl_sync(kFull, cs, src);
       dn = __shfl_sync(kFull, es, src);
     } else {
@@ -479,14 +472,16 @@ __device__ __forceinline__ void build_ants(const BatchArgs &a, const BatchShape 
         const int b = __ffs(none) - 1;
         none &= none - 1u;
         const int fc = __shfl_sync(kFull, cur, b);
-        const uint32_t fl = __shfl_sync(kFull, lim, b), fb = __shfl_sync(kFull, us.base, b);
+        const uint32_t fl = __shfl_sync(kFull, lim, b);
+        Unserved<E> its = us;
+        its.base = __shfl_sync(kFull, us.base, b);
         int nx = -1;
         if (tb.tier && ((zero >> b) & (LPA == 4 ? 0xfu : 0xffu)) == 0u) {
           const uint32_t two =
               __ldg(reinterpret_cast<const uint32_t *>(tb.tier + (size_t)fc * kTierLen) + lane);
-          nx = coop_tier<E>(two, fb, fl);
+          nx = coop_tier<E>(two, its, fl);
         }
-        if (nx < 0) nx = coop_scan<E>(tb.coords, fb, n, fc, fl, lane);
+        if (nx < 0) nx = coop_scan<E>(tb.coords, its, n, fc, fl, lane);
         if ((lane & ~(LPA - 1)) == b) {
           next = nx;
           take = nx > 0;
@@ -497,8 +492,10 @@ __device__ __forceinline__ void build_ants(const BatchArgs &a, const BatchShape 
       __syncwarp();  // the elements are read before they are marked
     }
     // The step, without a branch: an ant that takes none marks the depot,
-    // which is marked from the start.
-    us.mark(take ? next : 0);
+    // which is marked from the start (not in a bitmap: lanes without an ant
+    // would write back the first ant's word as it was).
+    if (!kBits) us.mark(take ? next : 0);
+    else if (take) us.mark(next);
     held = take && l == (pos & (LPA - 1)) ? next : held;
     pos += take ? 1 : 0;
     if (take && (pos & (LPA - 1)) == 0) route[pos - LPA + l] = held;
@@ -527,8 +524,10 @@ __device__ __forceinline__ void build_ants(const BatchArgs &a, const BatchShape 
       rm &= rm - 1u;
       const int who = ant0 + warp * kApw + b / LPA;
       const long long lo = I.lens_off + (long long)who * K;
+      Unserved<E> its = us;
+      its.base = __shfl_sync(kFull, us.base, b);
       const int added = coop_repair<E>(
-          tb.coords, __shfl_sync(kFull, us.base, b), n, K, cap, __shfl_sync(kFull, pos, b),
+          tb.coords, its, n, K, cap, __shfl_sync(kFull, pos, b),
           __shfl_sync(kFull, left, b), a.routes + I.route_off + (long long)who * R, a.lens + lo,
           a.loads + lo, a.last + lo, a.rep + I.rep_off + (long long)who * n, scratch, lane);
       if ((lane & ~(LPA - 1)) == b) {
@@ -757,7 +756,8 @@ __global__ void __launch_bounds__(kBatchThreads)
       s_cand[e] = t < k ? a.cand[(I.node_off + r) * k + t] : (uint16_t)0;
     }
     for (int e = tid; e < rows; e += nthr) s_coords[e] = a.coords[I.node_off + e];
-    for (uint32_t e = tid; e < sh.el_bytes / E; e += nthr) {
+    constexpr uint32_t kSize = elem_is_bits(E) ? 4u : (uint32_t)E;
+    for (uint32_t e = tid; e < sh.el0_bytes / kSize; e += nthr) {
       const uint32_t x = e >= 1 && e <= (uint32_t)n ? (uint32_t)a.demand[I.node_off + e]
                                                     : Unserved<E>::kVisited;
       if (E == 1) smem[sh.off_el0 + e] = (unsigned char)x;
@@ -875,18 +875,25 @@ __global__ void __launch_bounds__(kBatchThreads)
 
 using BatchKernel = void (*)(BatchArgs, BatchShape);
 
-BatchKernel batch_kernel(int lpa, int elem) {
-  if (lpa == 4) {
-    return elem == 1 ? k_batch_solve<4, 1> : (elem == 2 ? k_batch_solve<4, 2> : k_batch_solve<4, 4>);
+template <int LPA>
+BatchKernel batch_kernel_of(int elem) {
+  switch (elem) {
+    case 1: return k_batch_solve<LPA, 1>;
+    case 2: return k_batch_solve<LPA, 2>;
+    case 4: return k_batch_solve<LPA, 4>;
   }
-  return elem == 1 ? k_batch_solve<8, 1> : (elem == 2 ? k_batch_solve<8, 2> : k_batch_solve<8, 4>);
+  return k_batch_solve<LPA, kElemStagedBits>;
+}
+
+BatchKernel batch_kernel(int lpa, int elem) {
+  return lpa == 4 ? batch_kernel_of<4>(elem) : batch_kernel_of<8>(elem);
 }
 
 // Opts the kernels into the largest dynamic shared memory their static
 // shared variables leave free.
 cudaError_t configure_batch() {
   for (int lpa : {4, 8})
-    for (int elem : {1, 2, 4}) {
+    for (int elem : {1, 2, 4, kElemStagedBits}) {
       cudaFuncAttributes fa;
       const void *f = reinterpret_cast<const void *>(batch_kernel(lpa, elem));
       cudaError_t e = cudaFuncGetAttributes(&fa, f);
@@ -967,31 +974,35 @@ static int batch_v_for(int lanes, int max_rows) {
 }
 
 // The launch for the batch: every ant of a colony at a time where a block's
-// threads and shared memory allow; of the ways to do that, the one with the
-// most blocks resident at once that the instances can use, and then with the
+// threads and shared memory allow, with bitmaps in place of the ants' elements
+// where those leave no room; of the ways to do that, the one with the most
+// blocks resident at once that the instances can use, and then with the
 // pheromone levels in shared memory.
 static bool choose_shape(const aco_b200_batch *b, BatchShape *out, int *grid) {
-  const int elem = demand_bytes(b->max_demand), lpa = b->k <= 16 ? 4 : 8;
+  const int lpa = b->k <= 16 ? 4 : 8;
   const int most = kBatchThreads / lpa;
   const int rounds = (b->m + most - 1) / most;
   const int useful = (b->count + b->num_sms - 1) / b->num_sms;  // blocks per SM with work
   int best = 0;
   for (int round = (b->m + rounds - 1) / rounds; round >= 1 && best == 0;
        round = round > 8 ? round * 3 / 4 : round - 1) {
-    for (int tau_smem = 1; tau_smem >= 0; --tau_smem) {
-      const BatchShape sh =
-          batch_shape(b->max_rows, b->max_n, b->k, b->m, elem, round, tau_smem != 0);
-      if ((int)sh.total + 64 > construct_max_smem()) continue;
-      int per_sm = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-              &per_sm, reinterpret_cast<const void *>(batch_kernel(sh.lpa, elem)), sh.threads,
-              sh.total) != cudaSuccess)
-        return false;
-      per_sm = std::min(per_sm, useful);
-      if (per_sm > best) {
-        best = per_sm;
-        *out = sh;
+    for (int elem : {demand_bytes(b->max_demand), kElemStagedBits}) {
+      for (int tau_smem = 1; tau_smem >= 0; --tau_smem) {
+        const BatchShape sh =
+            batch_shape(b->max_rows, b->max_n, b->k, b->m, elem, round, tau_smem != 0);
+        if ((int)sh.total + 64 > construct_max_smem()) continue;
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                &per_sm, reinterpret_cast<const void *>(batch_kernel(sh.lpa, elem)), sh.threads,
+                sh.total) != cudaSuccess)
+          return false;
+        per_sm = std::min(per_sm, useful);
+        if (per_sm > best) {
+          best = per_sm;
+          *out = sh;
+        }
       }
+      if (best > 0) break;
     }
   }
   *grid = std::min(best * b->num_sms, b->count);

@@ -139,10 +139,11 @@ struct InstanceView {
 inline int demand_bytes(int max_demand) {
   return max_demand < 0xff ? 1 : (max_demand < 0xffff ? 2 : 4);
 }
-// In place of a size: one bit per node, demands in global memory or all 1.
-constexpr int kElemBits = 0, kElemUnitBits = 3;
+// In place of a size: one bit per node, demands in global memory, all 1, or in
+// shared memory once for all ants of the block.
+constexpr int kElemBits = 0, kElemUnitBits = 3, kElemStagedBits = 5;
 __host__ __device__ constexpr bool elem_is_bits(int elem) {
-  return elem == kElemBits || elem == kElemUnitBits;
+  return elem == kElemBits || elem == kElemUnitBits || elem == kElemStagedBits;
 }
 // Bytes of one ant's elements or bitmap, whole 16-byte pieces.
 inline uint32_t unserved_bytes(int n, int elem) {
@@ -475,7 +476,8 @@ __device__ inline unsigned long long warp_knn(const float2 *coords, int n, int k
 // that largest value; E = kElemBits: a bitmap (word wi holding nodes 32 wi ..
 // 32 wi + 31) with the demands in global memory, for instances whose elements
 // do not fit beside the other ants of the block; E = kElemUnitBits: the same
-// where every demand is 1 and none is read.
+// where every demand is 1 and none is read; E = kElemStagedBits: the same with
+// the demands in shared memory, 4 bytes each (batched solver).
 //
 // The elements replace a bitmap in registers read by a shuffle: that took a
 // shuffle, the bit's forming and testing, a second load for the demand and a
@@ -486,6 +488,7 @@ struct Unserved {
   uint32_t base;     // shared address of this ant's elements
   uint32_t chunks;   // 16-byte pieces
   const int *dem;    // E = kElemBits
+  uint32_t dem_s;    // E = kElemStagedBits: the demands' shared address
 
   // The accesses are volatile so that they keep their order: a visit's store
   // comes before the next step's loads.
@@ -498,7 +501,10 @@ struct Unserved {
     } else if (E == 4) {
       asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(base + 4u * (uint32_t)node));
     } else {
-      const uint32_t d = E == kElemBits ? (uint32_t)__ldg(dem + node) : 1u;
+      uint32_t d = 1u;
+      if (E == kElemBits) d = (uint32_t)__ldg(dem + node);
+      if (E == kElemStagedBits)
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(d) : "r"(dem_s + 4u * (uint32_t)node));
       asm volatile("ld.shared.u32 %0, [%1];"
                    : "=r"(v) : "r"(base + 4u * ((uint32_t)node >> 5)));
       v = (__funnelshift_r(v, v, node) & 1u) ? kVisited : d;
@@ -523,7 +529,11 @@ struct Unserved {
     } else {
       uint32_t v;
       asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(base + 4u * ((uint32_t)q >> 4)));
-      const int2 d = E == kElemBits ? __ldg(reinterpret_cast<const int2 *>(dem) + q) : make_int2(1, 1);
+      int2 d = make_int2(1, 1);
+      if (E == kElemBits) d = __ldg(reinterpret_cast<const int2 *>(dem) + q);
+      if (E == kElemStagedBits)
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];"
+                     : "=r"(d.x), "=r"(d.y) : "r"(dem_s + 8u * (uint32_t)q));
       v >>= (2 * q) & 31;
       e0 = (v & 1u) ? kVisited : (uint32_t)d.x;
       e1 = (v & 2u) ? kVisited : (uint32_t)d.y;
@@ -548,16 +558,15 @@ struct Unserved {
   __device__ __forceinline__ uint32_t limit(int room) const {
     return (E == 1 || E == 2) ? min((uint32_t)room, kVisited - 1u) : (uint32_t)room;
   }
-  // The bitmap of an unserved instance (by one warp); elements are copied from
-  // iv.elems.
-  __device__ __forceinline__ void init_bits(int n, int lane) {
-    for (uint32_t wi = (uint32_t)lane; wi < 4u * chunks; wi += 32u) {
+  // The bitmap of an unserved instance, by `lanes` lanes of a warp; elements are
+  // copied from the instance's.
+  __device__ __forceinline__ void init_bits(int n, int lane, int lanes = 32) {
+    for (uint32_t wi = (uint32_t)lane; wi < 4u * chunks; wi += (uint32_t)lanes) {
       const int lo = (int)wi << 5, valid = n + 1 - lo;  // nodes lo..n in this word
       uint32_t v = lo == 0 ? 1u : 0u;
       if (valid < 32) v |= valid <= 0 ? 0xffffffffu : (0xffffffffu << valid);
       asm volatile("st.shared.u32 [%0], %1;" ::"r"(base + 4u * wi), "r"(v));
     }
-    __syncwarp();
   }
 };
 

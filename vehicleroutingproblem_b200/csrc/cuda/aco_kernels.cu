@@ -908,7 +908,10 @@ __global__ void __launch_bounds__(512, 1) k_construct(const __grid_constant__ Co
   us.base = smem_addr(smem + pl.off_vis + (size_t)warp * pl.vis_bytes);
   us.chunks = pl.vis_bytes / 16u;
   us.dem = iv.demand;
-  if (!kElems) us.init_bits(iv.n, lane);
+  if (!kElems) {
+    us.init_bits(iv.n, lane);
+    __syncwarp();
+  }
 
   wait_for_previous();
   // Graph replays read the epoch number and the seed from the device state,
