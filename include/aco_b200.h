@@ -392,7 +392,8 @@ ACO_API int aco_b200_batch_apply_prior(aco_b200_batch *batch, aco_b200_prior *pr
  * the evaporation step as in the reference (src/cuda/aco_cuda.cu:214-215).
  * Same result as aco_b200_evaporate_deposit.
  *
- * Three launches (the sweep, one per deposit; no scratch in device memory).
+ * One launch for a small matrix with few routes, else three (the sweep, one
+ * per deposit); no scratch in device memory.
  * The route offsets are kept in shared memory, so K may be at most 4096
  * routes; larger K is rejected with ACO_ERR_INVALID_INPUT and a message on
  * stderr.  Calls on different matrices are independent; calls on one matrix

@@ -15,6 +15,8 @@ extern "C" {
 #include "aco_b200.h"
 }
 
+#include <cooperative_groups.h>
+
 #include <cmath>
 #include <cstdio>
 
@@ -49,6 +51,31 @@ __global__ void __launch_bounds__(kDepositThreads)
   wait_for_previous();
   deposit_solution(pv, (size_t)n + 1, CompactNodes{nodes}, lens, K, dep, s_off,
                    (int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(gridDim.x * blockDim.x));
+}
+
+// Small matrices with few routes: the sweep and both deposits in one launch, a
+// cluster of blocks with its barrier in between.  Three launches cost the host
+// 12.6 us, this one 8.4 (one kernel whose last block deposits, with its scratch
+// cleared by a memset, took 9.6): n=100 K=5 8.4 us per call, 12.8 with three
+// launches; n=500 K=1 10.8 and 12.8.  Beyond, eight SMs sweep and deposit too
+// slowly (n=1000 K=1 14.9 and 12.7, n=512 K=16 14.5 and 12.7, n=50 K=50 39.0
+// and 37.0).
+constexpr int kSmallCluster = 8;
+constexpr int kSmallThreads = 512;
+inline bool small_update(int n, int K) { return K <= 16 && n <= 640 - 16 * K; }
+
+__global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kSmallThreads)
+    k_noalloc_small(PheromoneView pv, int n, int K, const int *it_nodes, const int *it_lens,
+                    float dep_it, const int *gb_nodes, const int *gb_lens, float dep_gb) {
+  extern __shared__ int s_off[];
+  const auto cluster = cooperative_groups::this_cluster();
+  const int gt = (int)(blockIdx.x * blockDim.x + threadIdx.x), gn = kSmallCluster * kSmallThreads;
+  evap_sweep<kSweepUnroll>(pv.tau, pv.tau, pv.total, pv.q_min, pv.delta);
+  cluster.sync();
+  deposit_solution(pv, (size_t)n + 1, CompactNodes{it_nodes}, it_lens, K, dep_it, s_off, gt, gn);
+  if (!gb_nodes) return;
+  cluster.sync();
+  deposit_solution(pv, (size_t)n + 1, CompactNodes{gb_nodes}, gb_lens, K, dep_gb, s_off, gt, gn);
 }
 
 }  // namespace
@@ -88,12 +115,22 @@ extern "C" ACO_API int aco_b200_evaporate_deposit_noalloc(
   pv.delta = (uint8_t)fmaxf(1.0f, roundf(-log_rho / step));
   pv.pad = 0;
   cudaStream_t s = (cudaStream_t)stream;
+  const size_t smem = sizeof(int) * (size_t)(K + 1);
+  if (small_update(n, K)) {
+    k_noalloc_small<<<kSmallCluster, kSmallThreads, smem, s>>>(
+        pv, n, K, d_iter_nodes, d_iter_lens, dep_iter, d_gbest_nodes, d_gbest_lens, dep_global);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+      fprintf(stderr, "aco_b200_evaporate_deposit_noalloc: launch: %s\n", cudaGetErrorString(e));
+      return ACO_ERR_BACKEND;
+    }
+    return ACO_OK;
+  }
   const unsigned long long tile = (unsigned long long)kSweepUnroll * kSweepThreads;
   const unsigned long long tiles = (pv.total / 16 + tile - 1) / tile;
   k_noalloc_sweep<<<(unsigned)(tiles < 1 ? 1 : tiles), kSweepThreads, 0, s>>>(pv);
   cudaError_t e = cudaGetLastError();
   const int grid = (n + 2 * K + kDepositThreads - 1) / kDepositThreads;
-  const size_t smem = sizeof(int) * (size_t)(K + 1);
   if (e == cudaSuccess)
     e = launch_after(k_noalloc_deposit, grid, kDepositThreads, smem, s, pv, n, K, d_iter_nodes,
                      d_iter_lens, dep_iter);
