@@ -311,10 +311,11 @@ typedef struct {
   double min_rel_improvement;
 } aco_b200_batch_problem;
 
-/* Launch shape: candidate slots per ant (16: needs cand_k <= 16; 32), at four
- * slots per lane; ants a block must be able to hold (a block builds all ants
- * of an instance at a time where its threads and shared memory allow); queue
- * order (0: as given, 1: largest first).  Results do not depend on it. */
+/* Launch shape: lanes per ant (16: needs cand_k <= 16; 32) and ants per block,
+ * checked against the batch's sizes but otherwise without effect: the launch
+ * takes a lane per four candidates and builds all ants of an instance at a time
+ * where a block's threads and shared memory allow; queue order (0: as given, 1:
+ * largest first).  Results do not depend on it. */
 typedef struct {
   int lanes_per_ant;
   int ants_per_block;
@@ -328,8 +329,10 @@ ACO_API int aco_b200_batch_set_stream(aco_b200_batch *batch, void *cuda_stream);
 ACO_API int aco_b200_batch_setup(aco_b200_batch *batch, const aco_b200_batch_problem *problem);
 ACO_API int aco_b200_batch_set_tuning(aco_b200_batch *batch, const aco_b200_batch_tuning *tuning);
 ACO_API int aco_b200_batch_get_tuning(aco_b200_batch *batch, aco_b200_batch_tuning *tuning);
-/* Times every candidate launch shape on `trial_epochs` epochs of the whole
- * batch and keeps the fastest; per-trial ms through trial_ms. */
+/* Times the two queue orders on `trial_epochs` epochs of the whole batch and
+ * keeps the faster one beside the shape that is set (the other fields of a
+ * shape do not change the launch).  trial_ms gets the time of every candidate
+ * shape the batch accepts, which is its order's. */
 ACO_API int aco_b200_batch_autotune(aco_b200_batch *batch, int trial_epochs,
                                     aco_b200_batch_tuning *chosen, float *trial_ms,
                                     int max_trials, int *n_trials);
@@ -340,7 +343,7 @@ ACO_API int aco_b200_batch_autotune(aco_b200_batch *batch, int trial_epochs,
  * {32, 16, 1}.  Learned levels applied before are replaced. */
 ACO_API int aco_b200_batch_set_cand_k(aco_b200_batch *batch, int k);
 ACO_API int aco_b200_batch_get_cand_k(aco_b200_batch *batch, int *k);
-/* Chooses the candidate-list length, then the launch shape.  Stage 1 solves
+/* Chooses the candidate-list length, then the queue order.  Stage 1 solves
  * the whole batch once per length ks[0..nks) (nks <= 16) on the default
  * shape and records its device time (k_solve_ms), the mean final cost over
  * the instances every length solved (k_mean_cost) and the instances solved
