@@ -16,7 +16,7 @@ large16000 / large32000: n=16000, K=16 / n=32000, K=32, uniform, 256 ants,
 batched: 512 instances (n~U[50,500], K=ceil(n/60), seeds 30000-30511), 64
 ants, 300 epochs each, all in one persistent launch; the autotuner chooses
 the candidate-list length (16, 20 or 32: the fastest within 0.5 % of the
-best mean final cost) and the launch shape; a step is one solve of the
+best mean final cost) and the queue order; a step is one solve of the
 whole batch and the metric is instances/s.
 learned: the learned prior's time-to-cost against plain eta on 256 held-out
 n=1000 instances (training set, training and evaluation inside the run).
@@ -817,7 +817,7 @@ def run_sharded(args, rank, world, local, torch, dist, _native):
 def batched_measure(torch, local, _native, insts, seed0, steps, warmup, e2e_steps,
                     looped_sample, dist=None, world=1):
     """The batched solver on `insts` (instance i solved with seed seed0 + i):
-    autotuned candidate length and shape, `steps` solves timed with CUDA
+    autotuned candidate length and queue order, `steps` solves timed with CUDA
     events on one stream (L2 flushed between them), the end-to-end rate
     through the C ABI with host buffers on one reused batch object, and the
     single-instance solver looped over a sample of the same instances
@@ -829,7 +829,7 @@ def batched_measure(torch, local, _native, insts, seed0, steps, warmup, e2e_step
     b.setup(insts, ants=BATCHED["ants"], cand_k=BATCHED["cand_k"], seed=seed0,
             epochs=BATCHED["epochs"])
     # The autotuner picks the candidate-list length (fastest within 0.5 % of
-    # the best mean final cost), then the launch shape.
+    # the best mean final cost), then the queue order.
     k, chosen, per_k, trials = b.autotune_k(ks=(16, 20, 32), quality_tol=0.005, trial_epochs=3)
     for _ in range(warmup):
         b.enqueue()
@@ -895,12 +895,12 @@ def batched_measure(torch, local, _native, insts, seed0, steps, warmup, e2e_step
 
 def batched_h2d_d2h(insts):
     """Bytes copied per end-to-end batched step: coordinates (8 B) and
-    demands (4 B) per node, a 72-byte descriptor, row offset and size
+    demands (4 B) per node, a 64-byte descriptor, row offset and size
     (12 B) and two queue orders (8 B) per instance, the level and weight
     tables (256 + 256 ints) and the 4095 eta thresholds up; every best route
     slot (n + 2K ints), the route lengths (K ints) and the costs (8 B) down."""
     nodes = sum(x.n + 1 for x in insts)
-    h2d = nodes * 12 + len(insts) * (72 + 12 + 8) + 2048 + 4095 * 4
+    h2d = nodes * 12 + len(insts) * (64 + 12 + 8) + 2048 + 4095 * 4
     d2h = sum((x.n + 2 * x.vehicles) * 4 + x.vehicles * 4 + 8 for x in insts)
     return h2d, d2h
 

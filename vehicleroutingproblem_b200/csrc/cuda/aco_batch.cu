@@ -31,8 +31,7 @@ using namespace acob200;
 namespace {
 
 struct BatchInst {
-  int n, K, cap, total_demand, max_demand;
-  int pad;
+  int n, K, cap, total_demand;
   long long node_off;   // coords / demand / rows (cand, lvl at node_off * k)
   long long route_off;  // m * (n + 2K) ints
   long long lens_off;   // m * K ints
@@ -781,7 +780,7 @@ __global__ void __launch_bounds__(kBatchThreads)
       for (int a0 = 0; a0 < a.m; a0 += sh.round)
         build_ants<LPA, E>(a, sh, I, tb, smem, seed, (uint32_t)epoch, a0, ii);
       __syncthreads();
-      // Iteration best: first minimum among feasible ants (k_best).
+      // Iteration best: first minimum among feasible ants (k_best_cluster).
       {
         double bc = DBL_MAX;
         int ba = INT_MAX;
@@ -1102,7 +1101,6 @@ int aco_b200_batch_setup(aco_b200_batch *b, const aco_b200_batch_problem *p) {
     }
     if (tot > 0x7fffffffLL) return ACO_ERR_INVALID_INPUT;
     I.total_demand = (int)tot;
-    I.max_demand = mx;
     max_demand = std::max(max_demand, mx);
     I.node_off = node;
     seg_off[i] = node;

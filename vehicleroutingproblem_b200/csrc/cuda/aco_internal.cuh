@@ -216,14 +216,6 @@ cudaError_t launch_construct(const InstanceView &iv, const EpochTables &et,
                              uint32_t stream_id, int use_state_epoch,
                              cudaStream_t s, const uint32_t *draw_src = nullptr,
                              uint32_t draw_per_ant = 0);
-cudaError_t launch_best(const InstanceView &iv, const AntBuffers &ab,
-                        DevState *st, int *gbest_nodes, int *gbest_lens,
-                        EpochRec *log, cudaStream_t s);
-cudaError_t launch_evap_deposit(const InstanceView &iv, const PheromoneView &pv,
-                                const AntBuffers &ab, DevState *st,
-                                const int *gbest_nodes, const int *gbest_lens,
-                                unsigned int *counter, int grid, uint8_t *tau_alt,
-                                cudaStream_t s);
 cudaError_t launch_set_run_limit(DevState *st, int limit, cudaStream_t s);
 int evap_grid_for(unsigned long long total, int num_sms);
 cudaError_t launch_evaporate_to(const PheromoneView &pv, uint8_t *tau_alt, DevState *st,

@@ -12,10 +12,9 @@
 //                     engine (reference kernel: aco_cuda_kernels.cu:447-562)
 //   k_best_cluster    iteration best, global best, stop rules and both
 //                     deposits of the pipelined epoch over a cluster of 8
-//                     blocks; k_best the same without the deposits, on the
-//                     device (src/cuda/aco_cuda.cu:83-126, :331-399)
-//   k_evap_deposit    128-bit streaming evaporation, then the deposit of the
-//                     iteration best and global best by the last block
+//                     blocks (src/cuda/aco_cuda.cu:83-126, :331-399)
+//   k_evap_deposit    128-bit streaming evaporation, then the deposit of two
+//                     given solutions by the last block
 //                     (aco_cuda_kernels.cu:145-155, :569-668)
 #include "aco_internal.cuh"
 
@@ -1276,37 +1275,6 @@ __device__ __forceinline__ void block_iter_best(const AntBuffers &ab, int m, dou
   }
 }
 
-// Iteration best, bookkeeping and the global-best copy in one block, for the
-// epochs whose pheromone update is a separate k_evap_deposit launch.
-__global__ void __launch_bounds__(1024) k_best(InstanceView iv, AntBuffers ab,
-                                               DevState *st, int *gbest_nodes,
-                                               int *gbest_lens, EpochRec *log) {
-  if (*(volatile int *)&st->skip) return;
-  __shared__ double s_cost[32];
-  __shared__ int s_ant[32];
-  __shared__ unsigned long long s_steps[32];
-  __shared__ int s_improved, s_best;
-  double bc;
-  int ba;
-  unsigned long long steps;
-  block_iter_best(ab, iv.m, s_cost, s_ant, s_steps, bc, ba, steps);
-  if (threadIdx.x == 0) {
-    s_improved = epoch_bookkeeping(st, ba != INT_MAX, bc, ba, steps, log);
-    s_best = ba;
-  }
-  __syncthreads();
-  if (s_improved) {
-    // New global best: keep a copy (the reference copies it to the host and
-    // uploads a flat buffer, aco_cuda.cu:367-380).
-    const int *src = ab.routes + (size_t)s_best * iv.route_stride;
-    const int *sl = ab.lens + (size_t)s_best * iv.K;
-    int total = 0;
-    for (int v = 0; v < iv.K; ++v) total += sl[v];
-    for (int t = threadIdx.x; t < total; t += blockDim.x) gbest_nodes[t] = src[t];
-    for (int v = threadIdx.x; v < iv.K; v += blockDim.x) gbest_lens[v] = sl[v];
-  }
-}
-
 // The pipelined epoch's iteration best, bookkeeping and both deposits over a
 // cluster of kBestCluster blocks, so that the deposits' scattered pheromone
 // reads and writes are issued from as many SMs.  Every block finds the same
@@ -1440,13 +1408,6 @@ __global__ void __cluster_dims__(kBestCluster, 1, 1) __launch_bounds__(kBestThre
                    s_improved ? it_nodes : gbest_nodes, s_improved ? it_lens : gbest_lens);
 }
 
-cudaError_t launch_best(const InstanceView &iv, const AntBuffers &ab,
-                        DevState *st, int *gbest_nodes, int *gbest_lens,
-                        EpochRec *log, cudaStream_t s) {
-  k_best<<<1, 1024, 0, s>>>(iv, ab, st, gbest_nodes, gbest_lens, log);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_best_deposit(const InstanceView &iv, const AntBuffers &ab,
                                 const PheromoneView &pv, uint8_t *tau_alt, DevState *st,
                                 int *gbest_nodes, int *gbest_lens, EpochRec *log,
@@ -1517,21 +1478,15 @@ struct EvapArgs {
   InstanceView iv;
   PheromoneView pv;
   AntBuffers ab;
-  DevState *st;
   const int *gbest_nodes;
   const int *gbest_lens;
   unsigned int *counter;
-  int best_ant;          // used when st == nullptr
+  int best_ant;
   float dep_iter, dep_global;
-  uint8_t *tau_alt;      // second pheromone buffer of the context, or null
 };
 
 __global__ void __launch_bounds__(kEvapThreads) k_evap_deposit(EvapArgs a) {
-  if (a.st) {
-    if (*(volatile int *)&a.st->skip || !*(volatile int *)&a.st->found) return;
-  }
-  PheromoneView pv = a.pv;  // in place, on the current buffer
-  pv.tau = cur_tau(a.pv.tau, a.tau_alt, a.st);
+  const PheromoneView &pv = a.pv;
   evap_sweep<kEvapUnroll>(pv.tau, pv.tau, pv.total, pv.q_min, pv.delta);
   // The last block to finish the sweep deposits (threadfence reduction).
   __shared__ int s_last;
@@ -1545,9 +1500,8 @@ __global__ void __launch_bounds__(kEvapThreads) k_evap_deposit(EvapArgs a) {
   if (!s_last) return;
   __threadfence();
   const size_t stride_n = (size_t)a.iv.n + 1;
-  const int best = a.st ? a.st->best_ant : a.best_ant;
-  const float dep_i = a.st ? a.st->dep_iter : a.dep_iter;
-  const float dep_g = a.st ? a.st->dep_global : a.dep_global;
+  const int best = a.best_ant;
+  const float dep_i = a.dep_iter, dep_g = a.dep_global;
   extern __shared__ int s_off[];
   int *offs = (a.iv.K <= kDepositSmemRoutes) ? s_off : nullptr;
   deposit_solution(pv, stride_n, CompactNodes{a.ab.routes + (size_t)best * a.iv.route_stride},
@@ -1559,28 +1513,7 @@ __global__ void __launch_bounds__(kEvapThreads) k_evap_deposit(EvapArgs a) {
   if (threadIdx.x == 0) *a.counter = 0u;
 }
 
-cudaError_t launch_evap_deposit(const InstanceView &iv, const PheromoneView &pv,
-                                const AntBuffers &ab, DevState *st,
-                                const int *gbest_nodes, const int *gbest_lens,
-                                unsigned int *counter, int grid, uint8_t *tau_alt,
-                                cudaStream_t s) {
-  EvapArgs a;
-  a.iv = iv;
-  a.pv = pv;
-  a.ab = ab;
-  a.st = st;
-  a.gbest_nodes = gbest_nodes;
-  a.gbest_lens = gbest_lens;
-  a.counter = counter;
-  a.best_ant = 0;
-  a.dep_iter = a.dep_global = 0.0f;
-  a.tau_alt = tau_alt;
-  const size_t smem = iv.K <= kDepositSmemRoutes ? sizeof(int) * (iv.K + 1) : 0;
-  k_evap_deposit<<<grid, kEvapThreads, smem, s>>>(a);
-  return cudaGetLastError();
-}
-
-// Test-hook variant with explicit best ant and amounts (no device state).
+// In place, with the ant and the amounts given by the caller.
 cudaError_t launch_evap_deposit_explicit(const InstanceView &iv,
                                          const PheromoneView &pv,
                                          const AntBuffers &ab, int best_ant,
@@ -1594,14 +1527,12 @@ cudaError_t launch_evap_deposit_explicit(const InstanceView &iv,
   a.iv = iv;
   a.pv = pv;
   a.ab = ab;
-  a.st = nullptr;
   a.gbest_nodes = gbest_nodes;
   a.gbest_lens = gbest_lens;
   a.counter = counter;
   a.best_ant = best_ant;
   a.dep_iter = dep_iter;
   a.dep_global = dep_global;
-  a.tau_alt = nullptr;  // the caller passes the current buffer
   const size_t smem = iv.K <= kDepositSmemRoutes ? sizeof(int) * (iv.K + 1) : 0;
   k_evap_deposit<<<grid, kEvapThreads, smem, s>>>(a);
   return cudaGetLastError();
@@ -1653,7 +1584,7 @@ __global__ void __launch_bounds__(1024) k_shard_pack(InstanceView iv, AntBuffers
 
 // Winner over the gathered packets (lowest cost, then lowest global ant:
 // the first minimum a single device holding every ant would find), then the
-// same bookkeeping as k_best; its route goes to iter_nodes/iter_lens and,
+// same bookkeeping as k_best_cluster; its route goes to iter_nodes/iter_lens and,
 // on improvement, to the global best; then both deposits into the
 // evaporated pheromone buffer and the buffer switch.
 __global__ void __cluster_dims__(kBestCluster, 1, 1) __launch_bounds__(kBestThreads)
