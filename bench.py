@@ -626,8 +626,7 @@ def run_single(args, rank, world, local, torch, dist, _native):
     value = steps_all / (dev_ms_max / 1e3)
 
     e2e_vals = []
-    h2d = (n + 1) * (8 + 4) + 4095 * 4 + 2 * 256 * 4
-    d2h = (n + 2 * K) * 4 + K * 4
+    h2d, d2h = single_h2d_d2h(n, K)
     # One context serves every solve (as a solver service would keep it):
     # each step uploads the instance from host memory, builds the candidate
     # lists, runs the epochs and downloads the best routes; the context's
@@ -748,8 +747,7 @@ def run_sharded(args, rank, world, local, torch, dist, _native):
     col.close()
 
     e2e_vals = []
-    h2d = (n + 1) * (8 + 4) + 4095 * 4 + 2 * 256 * 4
-    d2h = (n + 2 * K) * 4 + K * 4
+    h2d, d2h = single_h2d_d2h(n, K)
     c2 = None
     for i in range(args.e2e_steps):
         dist.barrier()
@@ -891,6 +889,20 @@ def batched_measure(torch, local, _native, insts, seed0, steps, warmup, e2e_step
             "ant_steps": float(ant_steps.sum()),
             "mean_cost": float(np.mean(costs[costs < 1e300])) if np.any(costs < 1e300) else None,
             "e2e": statistics.median(e2e_vals) if e2e_vals else None, "looped": looped}
+
+
+def single_h2d_d2h(n, K):
+    """Bytes copied per end-to-end step of one context: one upload of 256-byte
+    aligned pieces (device state, a counter, the level and weight tables, the
+    4095 eta thresholds, coordinates, demands with room for 4 bytes per node of
+    the ants' elements behind them) and one download (the best route slots, the
+    route lengths, the 120-byte device state)."""
+    def up(b, to=256):
+        return -(-b // to) * to
+    demands = up(4 * (n + 1), 16)
+    h2d = 2 * 256 + 2 * 1024 + up(4095 * 4) + up(8 * (n + 1)) + up(2 * demands)
+    d2h = up(4 * (n + 2 * K)) + up(4 * K) + 120
+    return h2d, d2h
 
 
 def batched_h2d_d2h(insts):
