@@ -554,7 +554,7 @@ def seq_update_roofline(torch, ctx, n, K, launches, peak, peak_kind):
     nbytes = 16 * (n + 1) ** 2
     achieved = nbytes / (ms / 1e3) / 1e9
     del tau, scratch
-    return {"bound": "hbm", "kernel": "k_seq_sweep + k_seq_mark + k_seq_deposit",
+    return {"bound": "hbm", "kernel": "k_seq_mark + k_seq_sweep + k_seq_add + k_seq_clamp",
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "peak_kind": peak_kind, "n": n, "bytes_per_update": nbytes,
             "us_per_update": ms * 1e3, "launches": launches, "traffic": None,

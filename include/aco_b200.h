@@ -158,9 +158,10 @@ ACO_API int aco_b200_get_tables(aco_b200_ctx *ctx, int32_t *A, uint32_t *lut,
 /* Weights recomputed from the current pheromone ((n+1) k values). */
 ACO_API int aco_b200_get_weights(aco_b200_ctx *ctx, uint32_t *w);
 /* Fault-injection test hooks (host-made failures; no GPU fault):
- *   what 1: the value-th device allocation of the following set-up fails as
- *           out of memory (0 = off) -- set-up must return ACO_ERR_ALLOCATION
- *           and free what it allocated;
+ *   what 1: the device allocation of the following set-up that makes its
+ *           buffers anew fails as out of memory, if it has at least `value`
+ *           buffers (0 = off) -- set-up must return ACO_ERR_ALLOCATION and give
+ *           back what the context held;
  *   what 2: value 1 makes the construct kernel's bounded wait for its staged
  *           tables run out (the wait expects 16 bytes more than it copies):
  *           the kernel flags the error and returns, and aco_b200_run returns

@@ -644,7 +644,7 @@ class Batch:
         return k.value
 
     def autotune_k(self, ks=(16, 20, 32), quality_tol=0.005, trial_epochs=3):
-        """Candidate-list length, then launch shape (aco_b200_batch_autotune_k):
+        """Candidate-list length, then queue order (aco_b200_batch_autotune_k):
         returns (k, shape, per-length {k: (solve ms, mean cost, solved)},
         shape trial ms)."""
         kk = np.array(ks, np.int32)

@@ -1497,7 +1497,7 @@ int aco_b200_batch_autotune_k(aco_b200_batch *b, int trial_epochs, const int *ks
   int rc = aco_b200_batch_set_cand_k(b, ks[pick]);
   if (rc) return rc;
   if (chosen_k) *chosen_k = ks[pick];
-  // Stage 2: the launch shape for that length.
+  // Stage 2: the queue order for that length.
   return aco_b200_batch_autotune(b, trial_epochs, chosen, trial_ms, max_trials, n_trials);
 }
 

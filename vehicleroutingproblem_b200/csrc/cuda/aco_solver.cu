@@ -124,7 +124,7 @@ struct aco_b200_ctx {
   bool may_be_replayed() const { return split_gen == graph_gen; }
   bool run_limit_off = false;  // device run limit known to be disabled
   int depot_rule = 0;
-  int inject_alloc = 0;  // test hook: the n-th device allocation of a set-up fails
+  int inject_alloc = 0;  // test hook: a set-up's allocation fails, counted by its buffers
   // Kernel arguments the graphs were captured with: a set-up that leaves
   // them unchanged (same sizes, parameters and buffers) keeps the graphs.
   unsigned char graph_key[sizeof(InstanceView) + sizeof(PheromoneView) + sizeof(EpochTables) +
