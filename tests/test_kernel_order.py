@@ -33,6 +33,16 @@ def test_batch_fallback_reads_marked_elements_after_a_warp_barrier():
     assert "__syncwarp()" in _between(build, "} while (none);", "us.mark(")
 
 
+def test_bitmap_words_are_rewritten_after_a_warp_barrier():
+    """Every lane of an ant writes the word back: one step's writes must not
+    follow the next one's."""
+    build = _function("aco_batch.cu", "build_ants")
+    step = _between(build, "} while (none);", "us.mark(take ? next : 0)")
+    assert "if (kBits) __syncwarp();" in step
+    single = _function("aco_kernels.cu", "build_ant")
+    assert "if (E != 1) __syncwarp();" in _between(single, "if (first == 0u) break;", "take_step(next")
+
+
 def test_batch_cost_reads_routes_after_a_warp_barrier():
     build = _function("aco_batch.cu", "build_ants")
     stores_to_loads = _between(build, "route[(pos & ~(LPA - 1)) + l] = held;", "load_nodes(0)")

@@ -494,6 +494,9 @@ __device__ __forceinline__ void build_ants(const BatchArgs &a, const BatchShape 
     // The step, without a branch: an ant that takes none marks the depot,
     // which is marked from the start (not in a bitmap: lanes without an ant
     // would write back the first ant's word as it was).
+    // A bitmap's word is read, changed and written by each of the ant's lanes: the
+    // last step's writes come first.
+    if (kBits) __syncwarp();
     if (!kBits) us.mark(take ? next : 0);
     else if (take) us.mark(next);
     held = take && l == (pos & (LPA - 1)) ? next : held;
